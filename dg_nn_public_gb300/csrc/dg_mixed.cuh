@@ -1277,43 +1277,22 @@ int residual32(dg_ctx* c, const float* x, const float* b, float* r, float* x_out
                    : launch_residual32<2>(c, x, b, r, x_out, flags, st, ws);
 }
 
-// residual / smoothing with the BF16 block copies (FP32 vectors and sums)
-template <int D>
-int launch_residual16(dg_ctx* c, const float* x, const float* b, float* r, float* x_out, int flags,
-                      cudaStream_t st, const float* ws = nullptr) {
-  using E = Elem<D>;
-  Mixed& M = mixed_of(c);
-  unsigned g = nblk(c->B, E::EPB);
-  if (g)
-    residual_kernel<E::N, E::F, E::EPB, __nv_bfloat16, float, float><<<g, E::EPB * E::N, 0, st>>>(
-        M.blk16, M.W16, c->d_nbe, x, b, r, x_out, c->B, flags, c->T.P, M.r1, ws);
-  bump();
-  CKL(c);
-  return DG_OK;
-}
-
 // residual in the preconditioner: BF16 blocks when enabled, FP32 otherwise
 // *ws (device memory, so that captured graphs follow a rebuilt schedule;
 // nullptr = 1) scales the smoother's correction of this step,
 // x_out = x + ws W_e res: with W_e = w A_ee^-1 the step is damped by ws * w
 int residual_pc(dg_ctx* c, const float* x, const float* b, float* r, float* x_out, int flags, cudaStream_t st,
                 const float* ws = nullptr) {
-  if (c->precond_bf16) {
-    if (c->D == 3 && c->bf16_tma) {
-      Mixed& M = mixed_of(c);
-      return launch_bf16_tma(c, M, x, b, r, x_out, flags, st, ws);
-    }
-    if (c->D == 3) {
-      Mixed& M = mixed_of(c);
-      unsigned g = nblk(c->B, 8);
-      if (g)
-        residual_bf16c20_kernel<8><<<g, 8 * 20, 0, st>>>(M.blk16, M.W16, c->d_nbe, x, b, r, x_out, c->B, flags,
-                                                          c->d_P32, M.r1, ws);
-      bump();
-      CKL(c);
-      return DG_OK;
-    }
-    return launch_residual16<2>(c, x, b, r, x_out, flags, st, ws);
+  if (c->pc_bf16()) {
+    Mixed& M = mixed_of(c);
+    if (c->bf16_tma) return launch_bf16_tma(c, M, x, b, r, x_out, flags, st, ws);
+    unsigned g = nblk(c->B, 8);
+    if (g)
+      residual_bf16c20_kernel<8><<<g, 8 * 20, 0, st>>>(M.blk16, M.W16, c->d_nbe, x, b, r, x_out, c->B, flags,
+                                                        c->d_P32, M.r1, ws);
+    bump();
+    CKL(c);
+    return DG_OK;
   }
   return residual32(c, x, b, r, x_out, flags, st, ws);
 }
@@ -1812,11 +1791,13 @@ void cheb_factors(const dg_ctx* c, double lmax, int deg, double ratio, float* ou
 }
 
 // DG-level smoothing steps of the mixed preconditioner (pre and post each):
-// DG_MIXED_SWEEPS when set, else kMixedChebSteps with the damped block
-// inverse (a Chebyshev polynomial of that degree), else the configured V(s,s)
+// DG_MIXED_SWEEPS when set, else kMixedChebSteps (2D: kMixedChebSteps2D) with
+// the damped block inverse (a Chebyshev polynomial of that degree), else the
+// configured V(s,s)
 int mixed_steps(const dg_ctx* c) {
   if (c->mixed_sweeps >= 0) return c->mixed_sweeps;
-  return c->mixed_smoother == 1 ? kMixedChebSteps : c->cfg.pre_smooth_its;
+  if (c->mixed_smoother != 1) return c->cfg.pre_smooth_its;
+  return c->D == 3 ? kMixedChebSteps : kMixedChebSteps2D;
 }
 
 // one smoothing step of the preconditioner with x != 0: x_out = x + s W (b -
@@ -1898,12 +1879,6 @@ __global__ void convert_f64_f32_kernel(const ST* __restrict__ a, float* __restri
   if (k < n) b[k] = (float)a[k];
 }
 
-template <typename ST>
-__global__ void convert_f64_bf16_kernel(const ST* __restrict__ a, __nv_bfloat16* __restrict__ b, int64_t n) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) b[k] = __float2bfloat16_rn((float)a[k]);
-}
-
 // Deterministic start vector of the power iteration: a hash of the index
 // mapped to [-1, 1).
 __global__ void probe_init_kernel(float* __restrict__ v, int64_t n) {
@@ -1982,7 +1957,7 @@ int set_smoother_schedule(dg_ctx* c, cudaStream_t st) {
   CKL(c);
   const double lmax = lam / c->mixed_smooth_w;   // of A_ee^-1 A
   const int deg = std::min(kMaxSmoothSteps, std::max(2, mixed_steps(c)));
-  cheb_factors(c, lmax, deg, c->cheb_ratio, c->mixed_wscale);
+  cheb_factors(c, lmax, deg, c->cheb_ratio > 0.0 ? c->cheb_ratio : (c->D == 3 ? 64.0 : 32.0), c->mixed_wscale);
   c->smoother_lmax = lmax;
   if (c->verbose)
     std::fprintf(stderr, "[build_mixed] smoother: lambda_max(A_ee^-1 A) ~ %.4f, degree %d, damping %.4f .. %.4f\n",
@@ -2003,13 +1978,11 @@ int build_blk5(dg_ctx* c, cudaStream_t st) {
   else
     convert_f64_f32_kernel<<<nblk((int64_t)nb, 256), 256, 0, st>>>(c->d_blk, M.blk, (int64_t)nb);
   bump();
-  if (c->precond_bf16) {
+  if (c->pc_bf16()) {
     if (!M.blk16 && (rc = dalloc(c, &M.blk16, nb))) return rc;
-    if (c->D == 3)   // chunked layout read by residual_bf16c20_kernel
-      convert_f64_bf16_chunk20_kernel<<<nblk((int64_t)nb, 256), 256, 0, st>>>(c->d_blk, M.blk16,
-                                                                             (int64_t)c->B * (c->F + 1));
-    else
-      convert_f64_bf16_kernel<<<nblk((int64_t)nb, 256), 256, 0, st>>>(c->d_blk, M.blk16, (int64_t)nb);
+    // chunked layout read by residual_bf16c20_kernel
+    convert_f64_bf16_chunk20_kernel<<<nblk((int64_t)nb, 256), 256, 0, st>>>(c->d_blk, M.blk16,
+                                                                           (int64_t)c->B * (c->F + 1));
     bump();
   }
   CKL(c);
@@ -2087,13 +2060,10 @@ int build_mixed(dg_ctx* c, cudaStream_t st) {
     else
       convert_f64_f32_kernel<<<nblk((int64_t)nw, 256), 256, 0, st>>>(src, M.W, (int64_t)nw);
     bump();
-    if (c->precond_bf16) {
+    if (c->pc_bf16()) {
       int r2;
       if (!M.W16 && (r2 = dalloc(c, &M.W16, nw))) return r2;
-      if (c->D == 3)
-        convert_f64_bf16_chunk20_kernel<<<nblk((int64_t)nw, 256), 256, 0, st>>>(src, M.W16, (int64_t)c->B);
-      else
-        convert_f64_bf16_kernel<<<nblk((int64_t)nw, 256), 256, 0, st>>>(src, M.W16, (int64_t)nw);
+      convert_f64_bf16_chunk20_kernel<<<nblk((int64_t)nw, 256), 256, 0, st>>>(src, M.W16, (int64_t)c->B);
       bump();
     }
     return DG_OK;

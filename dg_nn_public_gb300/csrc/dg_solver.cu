@@ -62,6 +62,11 @@ constexpr int kMaxSmoothSteps = 8;
 // 14.0 / 13.8 / 14.1 / 15.3 ms at 78 / 54 / 38 / 33 / 30 / 27 inner steps;
 // c3: 2 / 4 / 5 / 6 steps 161 / 114 / 107 / 115 ms)
 constexpr int kMixedChebSteps = 5;
+// ... on triangles, with FP32 copies (dg_ctx::pc_bf16) and ratio 32.  Sum of
+// eight solves (4 meshes of 960 .. 28,600 triangles, kappa = 1 and
+// log-normal): degree / ratio 3/16 29.0 ms, 3/24 28.1, 4/32 27.8, 5/32 29.6,
+// 5/64 29.9, 6/64 32.1
+constexpr int kMixedChebSteps2D = 4;
 // ... and of the batched preconditioner, whose inner steps carry more fixed
 // work (per-RHS Gram-Schmidt, FP32 apply on CUDA cores, FP64 residuals):
 // c4 with 4 / 5 / 6 steps and ratio 32 / 64 / 128 took 213 / 196 / 166 ms
@@ -158,6 +163,15 @@ struct dg_ctx {
   int dense_n = 0;
   // mixed preconditioner reads BF16 copies of the blocks / smoother matrices
   bool precond_bf16 = true;
+  // BF16 copies are for tetrahedra, whose blocks stream from HBM.  On
+  // triangles the rounding of the blocks (2^-9 of their entries, while A
+  // times a smooth vector is smaller than the entries by the mesh size
+  // squared) made the smoother couple low modes into high ones: more or
+  // longer smoothing raised the inner steps, and a few flipped BF16 bits
+  // moved them by several.  FP32 copies of these small blocks cost little
+  // (most meshes stay in L2): 97 x 61 x 2 triangles 72 -> 25 inner steps,
+  // 8.4 -> 3.2 ms; 130 x 110 x 2 138 -> 29, 26.7 -> 5.4 ms.
+  bool pc_bf16() const { return precond_bf16 && D == 3; }
   // ... streamed by the persistent bulk-copy (TMA) kernel (3D)
   bool bf16_tma = true;
   // FP32 operator copy (3D) in the chunked layout, read by the bulk-copy kernel
@@ -196,14 +210,12 @@ struct dg_ctx {
   // -> 80 / 84 / 88 inner steps; c3: 94 / 94 / 106); a larger margin keeps
   // the polynomial below 1 further past an underestimated lambda_max
   double cheb_margin = 1.05;
-  // the Chebyshev interval is [beta / cheb_ratio, beta] (c2 / c3 with 5 steps:
-  // ratio 32 / 64 / 128 -> 37 / 34 / 33 and - / 36 / - inner steps; with 2
-  // steps the ratio 8 of the first schedule).  With host checks every 3
-  // steps, ratio 128 gave c2 12.88 ms (30 steps) and c3 99.3 ms (33) against
-  // 13.26 / 104.9 ms, but on a 2D case (64^2 x 2 triangles) the inner steps
-  // then moved from 64 to 81 with a rounding-level change of the coarse
-  // inverse; 64 keeps them within 2
-  double cheb_ratio = 64.0;
+  // the Chebyshev interval is [beta / ratio, beta]; 0 = the default, 64 (c2 /
+  // c3 with 5 steps: ratio 32 / 64 / 128 -> 37 / 34 / 33 and - / 36 / - inner
+  // steps; with 2 steps the ratio 8 of the first schedule; with host checks
+  // every 3 steps 64 / 128: c2 13.26 / 12.88 ms, c3 104.9 / 99.3 ms), 32 on
+  // triangles (kMixedChebSteps2D)
+  double cheb_ratio = 0.0;
   // the batched preconditioner's schedule: steps per leg (-1 = kBatchedChebSteps,
   // or DG_MIXED_SWEEPS when that is set) and Chebyshev interval ratio
   int batched_sweeps = -1;

@@ -247,7 +247,8 @@ int dg_smooth_scaled_batched(dg_ctx* ctx, const float* x, const float* cv, float
 /* Options of the mixed preconditioner, applied at the next mixed solve:
  * smoother 0 = three point-Jacobi sweeps per element block (as the
  * reference), 1 = damped exact block inverse smooth_w * A_ee^{-1};
- * precond_bf16 != 0 keeps the preconditioner's blocks in BF16; dense_max =
+ * precond_bf16 != 0 keeps the preconditioner's blocks in BF16 (tetrahedra;
+ * on triangles they are FP32 either way); dense_max =
  * size limit of the first SFC level solved exactly with a dense inverse
  * (0 = run the V-cycle down to the one-node level). */
 int dg_set_mixed_options(dg_ctx* ctx, int32_t smoother, double smooth_w, int32_t precond_bf16,
