@@ -488,6 +488,25 @@ __global__ void affine_check_kernel(const double* __restrict__ x, const double* 
   atomicMax(dev, (unsigned long long)__double_as_longlong(rel));
 }
 
+// Block diagonal out of the stored blocks: bdiag (B, N, N) row-major and, when
+// set, diag (B, N).  One CTA per element; the block is stored column-major,
+// so it is transposed through shared memory (one column of padding) and both
+// sides of the copy are contiguous.  Bound by HBM: 2 x 154 MB at 48,000
+// tetrahedra.  The transposition went through host memory before (33 ms at
+// that size: two pageable copies and a host loop).
+template <int N, int F>
+__global__ void __launch_bounds__(128) copy_bdiag_kernel(const double* __restrict__ blk, double* __restrict__ bdiag,
+                                                         double* __restrict__ diag) {
+  __shared__ double s[N][N + 1];
+  const int64_t e = blockIdx.x;
+  const double* A = blk + (size_t)e * (F + 1) * N * N;   // A(m, n) at [n * N + m]
+  for (int k = threadIdx.x; k < N * N; k += 128) s[k / N][k % N] = A[k];
+  __syncthreads();
+  double* out = bdiag + (size_t)e * N * N;
+  for (int k = threadIdx.x; k < N * N; k += 128) out[k] = s[k % N][k / N];
+  if (diag && threadIdx.x < N) diag[e * N + threadIdx.x] = s[threadIdx.x][threadIdx.x];
+}
+
 // ---------------------------------------------------------------------------
 // Smoother matrix.  The reference smooths with three point-Jacobi sweeps on
 // each element block, c <- c + w D^-1 (r - A_ee c) from c = 0, then

@@ -1582,23 +1582,14 @@ int dg_get_bdiag(dg_ctx* c, double* bdiag, double* diag, void* stream) {
   cudaStream_t st = S(stream);
   CK(c, cudaSetDevice(c->dev));
   const int N = c->N, F = c->F;
-  // blocks are stored column-major: transpose block 0 of every element
-  CK(c, cudaMemcpy2DAsync(bdiag, sizeof(double) * N * N, c->d_blk, sizeof(double) * N * N * (F + 1),
-                          sizeof(double) * N * N, c->B, cudaMemcpyDeviceToDevice, st));
-  // in-place transpose on the device copy (row-major output)
-  // (A_ee is symmetric up to roundoff; transpose keeps the exact entries)
-  std::vector<double> h((size_t)c->B * N * N);
-  CK(c, cudaMemcpyAsync(h.data(), bdiag, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, st));
-  CK(c, cudaStreamSynchronize(st));
-  std::vector<double> t(h.size()), dgv((size_t)c->B * N);
-  for (int64_t e = 0; e < c->B; ++e)
-    for (int m = 0; m < N; ++m) {
-      for (int n = 0; n < N; ++n) t[(e * N + m) * N + n] = h[(e * N + n) * N + m];
-      dgv[e * N + m] = h[(e * N + m) * N + m];
-    }
-  CK(c, cudaMemcpyAsync(bdiag, t.data(), sizeof(double) * t.size(), cudaMemcpyHostToDevice, st));
-  if (diag) CK(c, cudaMemcpyAsync(diag, dgv.data(), sizeof(double) * dgv.size(), cudaMemcpyHostToDevice, st));
-  CK(c, cudaStreamSynchronize(st));
+  if (c->B > 0) {
+    if (c->D == 3)
+      copy_bdiag_kernel<20, 4><<<(unsigned)c->B, 128, 0, st>>>(c->d_blk, bdiag, diag);
+    else
+      copy_bdiag_kernel<10, 3><<<(unsigned)c->B, 128, 0, st>>>(c->d_blk, bdiag, diag);
+    bump();
+  }
+  CKL(c);
   return DG_OK;
 }
 
