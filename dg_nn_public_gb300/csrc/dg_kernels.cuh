@@ -399,27 +399,30 @@ __global__ void __launch_bounds__(kBuildThreads, 3) build_blocks_kernel(BuildPar
 // n_f and area element sdet_f per face, every quadrature sum of the general
 // kernel factors into a geometric coefficient times a reference matrix that
 // is the same for all elements (ftab, formed once per context on the host):
-//   volume   det * sum_{jj,kk} (M^T M)[jj][kk] K[jj][kk]
-//   cs, sc   sdet_f * sum_jj c_f[jj] R[f][jj] (and its transpose),
-//            c_f = M^T n_f
-//   ss       sdet_f * Mf[f]
-//   cnb      sdet_f * sum_jj cn_f[jj] Q[f][fn][al][jj], cn_f = M_nb^T n_f
-//   snbv     sdet_f * sum_jj c_f[jj] P[f][fn][al][jj]
-//   ssnb     sdet_f * S[f][fn][al]
-// with al the face's alignment code and fn the neighbour's local face, so the
-// blocks equal the general kernel's to rounding (tested).  Table layout:
-// K (D*D), R (F*D), Mf (F), Q (F*F*D*D), P (F*F*D*D), S (F*F*D) matrices of
-// N*N doubles, entry (m, n) at [m * N + n].
+//   own block    det k_e sum_{i<=j} (M^T M)[i][j] V[ij]
+//                + k_f sdet_f (gamma_f Mf[f] - a sum_j c_f[j] R[f][j])
+//   face block   k_f sdet_f (-1/2 sum_j cn_f[j] Q[j] + 1/2 sum_j c_f[j] P[j]
+//                - gamma_f S)
+// with c_f = M^T n_f, cn_f = M_nb^T n_f, V and R symmetrised, and Q, P, S by
+// (f, neighbour's local face, alignment code), so the blocks equal the
+// general kernel's to rounding (tested).  Q and S have rows for the nodes on
+// the face only, P and S columns for those on the neighbour's face, so the
+// tables hold the entries of a face block class by class (both, row only,
+// column only, neither; FaceNodes) and those of the own block for m >= n.
+// GV, GM.. are the same tables projected on P1 (P^T T P): the Galerkin
+// products P^T A_b P come from them, without reading the blocks back.
 template <int D, int N, int F>
 struct FastTab {
-  static constexpr int NN = N * N;
-  static constexpr int K = 0;
-  static constexpr int R = K + D * D * NN;
-  static constexpr int Mf = R + F * D * NN;
-  static constexpr int Q = Mf + F * NN;
-  static constexpr int P = Q + F * F * D * D * NN;
-  static constexpr int S = P + F * F * D * D * NN;
-  static constexpr int Size = S + F * F * D * NN;
+  static constexpr int NN = N * N, NL = N * (N + 1) / 2, NC = D + 1, GG = NC * NC;
+  static constexpr int NV = D * (D + 1) / 2;        // V[ij], i <= j
+  static constexpr int ND = NV + F * (D + 1);       // + R[f][j], Mf[f] per face
+  static constexpr int NO = 2 * D + 1;              // Q[j], P[j], S
+  static constexpr int NCMB = F * F * D;
+  static constexpr int Diag = 0;                    // ND x NL
+  static constexpr int Off = Diag + ND * NL;        // NCMB x NO x NN
+  static constexpr int GDiag = Off + NCMB * NO * NN;   // ND x GG
+  static constexpr int GOff = GDiag + ND * GG;      // NCMB x NO x GG
+  static constexpr int Size = GOff + NCMB * NO * GG;
 };
 
 // Per-element geometry of the affine build, kappa-free and fixed for a
@@ -494,82 +497,126 @@ __global__ void __launch_bounds__(128) geom_affine_kernel(BuildParams p, double*
 }
 
 // Blocks of straight-sided elements from the geometry record and the
-// kappa-dependent face coefficients: one CTA per element, one thread per
-// block entry, no serial phase (the record is read into shared memory).
+// kappa-dependent face coefficients: one CTA per element.  Bound by the FP64
+// pipe: 22 products per entry of the own block's lower half, 7, 3, 3 or none
+// per entry of a face block by its class; 10,600 FMAs per tetrahedron with
+// the Galerkin products, 26,000 + 9,600 with full tables and the products
+// taken from the blocks.  131,712 tetrahedra: 9.64 -> 3.25 ms, the products taken from the
+// blocks 3.40 -> 0 ms.
+constexpr int kAffineThreads = 128;
 template <int D, int N, int F, int VG, int SG>
-__global__ void __launch_bounds__(N* N) build_blocks_affine_kernel(BuildParams p, const double* __restrict__ ftab,
-                                                                   const double* __restrict__ geom) {
+__global__ void __launch_bounds__(kAffineThreads) build_blocks_affine_kernel(
+    BuildParams p, const double* __restrict__ ftab, const double* __restrict__ geom,
+    const FaceNodes* __restrict__ fnp, double* __restrict__ Gout) {
   using TB = FastTab<D, N, F>;
   using G = GeomRec<D, F>;
-  constexpr int NN = N * N;
+  constexpr int NN = N * N, NT = kAffineThreads;
   __shared__ double rec[G::Size];
-  __shared__ double kf[F];
-  __shared__ int nbi[F], nbfc[F], aln[F], bct[F];
+  __shared__ double cd[TB::ND];      // coefficients of the own block's tables
+  __shared__ double co[F][TB::NO];   // ... of the face blocks' tables
+  __shared__ FaceNodes fn;
+  __shared__ int cmb[F], nbfc[F];
   const int64_t e = blockIdx.x;
   const int tid = threadIdx.x;
-  for (int k = tid; k < G::Size; k += NN) rec[k] = geom[e * G::Size + k];
+  for (int k = tid; k < G::Size; k += NT) rec[k] = geom[e * G::Size + k];
+  for (int k = tid; k < (int)(sizeof(FaceNodes) / 4); k += NT)
+    reinterpret_cast<int*>(&fn)[k] = reinterpret_cast<const int*>(fnp)[k];
+  __syncthreads();
+  const double ke = p.kappa[e];
   if (tid < F) {
-    const int64_t fi = e * F + tid;
     const int f = tid;
-    nbi[f] = p.nbe[fi];
-    nbfc[f] = p.nbface[fi];
-    aln[f] = p.aln[fi];
-    bct[f] = p.bct[fi];
-    const double ke = p.kappa[e];
-    if (bct[f] < 0) {
-      const int nb = nbi[f];
+    const int64_t fi = e * F + f;
+    const int nb = p.nbe[fi], bct = p.bct[fi];
+    const bool interior = bct < 0;
+    double kf = 0.0;
+    if (interior) {
       const double kn = nb >= 0 ? p.kappa[nb] : ke;
-      kf[f] = p.mu * (p.face_kappa ? 2.0 * ke * kn / (ke + kn) : 0.5 * (ke + kn));
-    } else if (bct[f] == 0) {
-      kf[f] = p.mu * ke;
-    } else {
-      kf[f] = 0.0;
+      kf = p.mu * (p.face_kappa ? 2.0 * ke * kn / (ke + kn) : 0.5 * (ke + kn));
+    } else if (bct == 0) {
+      kf = p.mu * ke;
     }
+    nbfc[f] = p.nbface[fi];
+    cmb[f] = interior && kf != 0.0 ? (f * F + nbfc[f]) * D + p.aln[fi] : -1;
+    const double* fr = rec + G::Face + f * G::PerFace;
+    const double ks = kf * fr[0], gam = fr[1];
+#pragma unroll
+    for (int j = 0; j < D; ++j) {
+      cd[TB::NV + f * (D + 1) + j] = (interior ? -0.5 : -1.0) * ks * fr[2 + j];
+      co[f][j] = -0.5 * ks * fr[2 + D + j];
+      co[f][D + j] = 0.5 * ks * fr[2 + j];
+    }
+    cd[TB::NV + f * (D + 1) + D] = ks * gam;
+    co[f][2 * D] = -ks * gam;
+  } else if (tid == 32) {
+    const double kv = p.mu * ke * rec[G::Det];
+    int q = 0;
+#pragma unroll
+    for (int i = 0; i < D; ++i)
+#pragma unroll
+      for (int j = i; j < D; ++j) cd[q++] = kv * rec[G::C + i * D + j];
   }
   __syncthreads();
-  const double* C = rec + G::C;
-  const double det_s = rec[G::Det];
-  const int m = tid % N, n = tid / N;
-  const int mn_ = m * N + n, nm_ = n * N + m;
-  double vol = 0.0;
+  double* out = p.blk + (size_t)e * (F + 1) * NN;
+  // face blocks, by class of entry
+#pragma unroll 1
+  for (int cls = 0; cls < 4; ++cls) {
+    const bool mS = !(cls & 2), nS = !(cls & 1);
+    int base = 0;
+#pragma unroll 1
+    for (int f = 0; f < F; ++f) {
+      const int g = nbfc[f], cf = fn.count[f], cg = fn.count[g];
+      const int cm = mS ? cf : N - cf, cn = nS ? cg : N - cg;
+      // first entry of this class in the table: (m on, n on), (m on, n off), ...
+      const int k0 = (cls > 0 ? cf * cg : 0) + (cls > 1 ? cf * (N - cg) : 0) + (cls > 2 ? (N - cf) * cg : 0);
+      const double* T = ftab + TB::Off + (size_t)(cmb[f] < 0 ? 0 : cmb[f]) * TB::NO * NN + k0;
+      for (int k = (tid + NT - base % NT) % NT; k < cm * cn; k += NT) {
+        const int m = fn.node[f][(mS ? 0 : cf) + k % cm], n = fn.node[g][(nS ? 0 : cg) + k / cm];
+        double v = 0.0;
+        if (cmb[f] >= 0) {
+          if (mS) {
 #pragma unroll
-  for (int a = 0; a < D * D; ++a) vol += C[a] * __ldg(ftab + TB::K + a * NN + mn_);
-  double diag = p.mu * p.kappa[e] * det_s * vol;
-  double* out = p.blk + (size_t)e * (F + 1) * N * N;
+            for (int j = 0; j < D; ++j) v = fma(co[f][j], __ldg(T + j * NN + k), v);
+          }
+          if (nS) {
 #pragma unroll
-  for (int f = 0; f < F; ++f) {
-    const double* fr = rec + G::Face + f * G::PerFace;
-    const double sdet = fr[0], gam = fr[1];
-    const double* cf = fr + 2;
-    const double* cn = fr + 2 + D;
-    double off = 0.0;
-    if (kf[f] != 0.0) {
-      const bool interior = bct[f] < 0;
-      const double a = interior ? 0.5 : 1.0;
-      double cs = 0.0, sc = 0.0;
-#pragma unroll
-      for (int jj = 0; jj < D; ++jj) {
-        const double* R = ftab + TB::R + (f * D + jj) * NN;
-        cs += cf[jj] * __ldg(R + mn_);
-        sc += cf[jj] * __ldg(R + nm_);
-      }
-      const double ss = __ldg(ftab + TB::Mf + f * NN + mn_);
-      diag += kf[f] * sdet * (-a * cs - a * sc + gam * ss);
-      if (interior) {
-        const int cmb = (f * F + nbfc[f]) * D + aln[f];
-        double cnb = 0.0, snbv = 0.0;
-#pragma unroll
-        for (int jj = 0; jj < D; ++jj) {
-          cnb += cn[jj] * __ldg(ftab + TB::Q + (cmb * D + jj) * NN + mn_);
-          snbv += cf[jj] * __ldg(ftab + TB::P + (cmb * D + jj) * NN + mn_);
+            for (int j = 0; j < D; ++j) v = fma(co[f][D + j], __ldg(T + (D + j) * NN + k), v);
+          }
+          if (mS && nS) v = fma(co[f][2 * D], __ldg(T + 2 * D * NN + k), v);
         }
-        const double ssnb = __ldg(ftab + TB::S + cmb * NN + mn_);
-        off = kf[f] * sdet * (-0.5 * cnb + 0.5 * snbv - gam * ssnb);
+        out[(size_t)(1 + f) * NN + n * N + m] = v;
       }
+      base += cm * cn;
     }
-    out[(size_t)(1 + f) * N * N + n * N + m] = off;
   }
-  out[n * N + m] = diag;
+  // own block: entries m >= n
+  for (int k = tid; k < TB::NL; k += NT) {
+    int m = (int)((sqrtf(8.0f * k + 1.0f) - 1.0f) * 0.5f);
+    if (m * (m + 1) / 2 > k) --m;
+    if ((m + 1) * (m + 2) / 2 <= k) ++m;
+    const int n = k - m * (m + 1) / 2;
+    double v = 0.0;
+#pragma unroll
+    for (int q = 0; q < TB::ND; ++q) v = fma(cd[q], __ldg(ftab + TB::Diag + q * TB::NL + k), v);
+    out[n * N + m] = v;
+    out[m * N + n] = v;
+  }
+  if (Gout) {
+    constexpr int GG = TB::GG;
+    double* Ge = Gout + (size_t)e * (F + 1) * GG;
+    for (int k = NT - 1 - tid; k < (F + 1) * GG; k += NT) {
+      const int b = k / GG, r = k % GG;
+      double v = 0.0;
+      if (b == 0) {
+#pragma unroll
+        for (int q = 0; q < TB::ND; ++q) v = fma(cd[q], __ldg(ftab + TB::GDiag + q * GG + r), v);
+      } else if (cmb[b - 1] >= 0) {
+        const double* T = ftab + TB::GOff + (size_t)cmb[b - 1] * TB::NO * GG + r;
+#pragma unroll
+        for (int q = 0; q < TB::NO; ++q) v = fma(co[b - 1][q], __ldg(T + q * GG), v);
+      }
+      Ge[k] = v;
+    }
+  }
 }
 
 // Largest deviation of the volume-point Jacobians of an element from its

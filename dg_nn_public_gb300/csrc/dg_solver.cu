@@ -114,6 +114,7 @@ struct dg_ctx {
   bool rap_direct = true;
   int *d_rap_ptr = nullptr, *d_rap_ent = nullptr;
   double* d_rap_G = nullptr;
+  bool rap_G_ready = false;   // the block build has formed the per-block products
   int64_t nface_sh = 0;
   double* d_kappa = nullptr;
   Tables T{};
@@ -393,6 +394,90 @@ __global__ void sfc_level_diag_kernel(const double* __restrict__ val, const int*
   if (i < n) diag[i] = didx[i] >= 0 ? val[didx[i]] : 0.0;
 }
 
+// FastTab of the element (host): the reference matrices, in the order that
+// build_blocks_affine_kernel reads them, and their projections on P1
+template <int D, int N, int F, int VG, int SG>
+void fill_fast_tab(const dg_mesh_desc* md, const int* al, const FaceNodes& fn, std::vector<double>& ft) {
+  using TB = FastTab<D, N, F>;
+  constexpr int NN = N * N, NC = TB::NC;
+  ft.assign(TB::Size, 0.0);
+  auto nlx = [&](int j, int n, int g) { return md->nlx[(j * N + n) * VG + g]; };
+  auto sn = [&](int f, int n, int g) { return md->sn[(f * N + n) * SG + g]; };
+  auto snlx = [&](int f, int j, int n, int g) { return md->snlx[(size_t)f * D * N * SG + (j * N + n) * SG + g]; };
+  std::vector<double> T(NN);   // one matrix, entry (m, n) at [m * N + n]
+  auto project = [&](double* out) {
+    for (int a = 0; a < NC; ++a)
+      for (int c = 0; c < NC; ++c) {
+        double s = 0.0;
+        for (int m = 0; m < N; ++m)
+          for (int n = 0; n < N; ++n) s += md->p1_to_p3[m * NC + a] * T[m * N + n] * md->p1_to_p3[n * NC + c];
+        out[a * NC + c] = s;
+      }
+  };
+  auto put_diag = [&](int q) {
+    double* o = ft.data() + TB::Diag + (size_t)q * TB::NL;
+    for (int m = 0; m < N; ++m)
+      for (int n = 0; n <= m; ++n) *o++ = T[m * N + n];
+    project(ft.data() + TB::GDiag + (size_t)q * TB::GG);
+  };
+  auto put_off = [&](int cmb, int q, int f, int g) {
+    double* o = ft.data() + TB::Off + ((size_t)cmb * TB::NO + q) * NN;
+    const int cf = fn.count[f], cg = fn.count[g];
+    for (int cls = 0; cls < 4; ++cls) {
+      const bool mS = !(cls & 2), nS = !(cls & 1);
+      const int cm = mS ? cf : N - cf, cn = nS ? cg : N - cg;
+      for (int k = 0; k < cm * cn; ++k)
+        *o++ = T[fn.node[f][(mS ? 0 : cf) + k % cm] * N + fn.node[g][(nS ? 0 : cg) + k / cm]];
+    }
+    project(ft.data() + TB::GOff + ((size_t)cmb * TB::NO + q) * TB::GG);
+  };
+  int q = 0;
+  for (int i = 0; i < D; ++i)
+    for (int j = i; j < D; ++j, ++q) {
+      for (int m = 0; m < N; ++m)
+        for (int n = 0; n < N; ++n) {
+          double t = 0.0;
+          for (int g = 0; g < VG; ++g) {
+            t += md->weight[g] * nlx(i, m, g) * nlx(j, n, g);
+            if (i != j) t += md->weight[g] * nlx(j, m, g) * nlx(i, n, g);
+          }
+          T[m * N + n] = t;
+        }
+      put_diag(q);
+    }
+  for (int f = 0; f < F; ++f)
+    for (int j = 0; j <= D; ++j, ++q) {   // j < D: R + R^T, then Mf
+      for (int m = 0; m < N; ++m)
+        for (int n = 0; n < N; ++n) {
+          double t = 0.0;
+          for (int g = 0; g < SG; ++g)
+            t += md->sweight[g] * (j < D ? sn(f, m, g) * snlx(f, j, n, g) + snlx(f, j, m, g) * sn(f, n, g)
+                                         : sn(f, m, g) * sn(f, n, g));
+          T[m * N + n] = t;
+        }
+      put_diag(q);
+    }
+  for (int f = 0; f < F; ++f)
+    for (int h = 0; h < F; ++h)
+      for (int lg = 0; lg < D; ++lg) {
+        const int cmb = (f * F + h) * D + lg;
+        for (int r = 0; r < TB::NO; ++r) {
+          const int j = r % D;
+          for (int m = 0; m < N; ++m)
+            for (int n = 0; n < N; ++n) {
+              double t = 0.0;
+              for (int g = 0; g < SG; ++g) {
+                const int ag = al[lg * SG + g];
+                t += md->sweight[g] * (r < D ? sn(f, m, g) * snlx(h, j, n, ag)
+                                             : (r < 2 * D ? snlx(f, j, m, g) * sn(h, n, ag) : sn(f, m, g) * sn(h, n, ag)));
+              }
+              T[m * N + n] = t;
+            }
+          put_off(cmb, r, f, h);
+        }
+      }
+}
+
 template <int D>
 int launch_build(dg_ctx* c, cudaStream_t st) {
   using E = Elem<D>;
@@ -440,9 +525,11 @@ int launch_build(dg_ctx* c, cudaStream_t st) {
       CKL(c);
     }
     if (c->B > 0)
-      build_blocks_affine_kernel<D, E::N, E::F, E::VG, E::SG><<<(unsigned)c->B, E::N * E::N, 0, st>>>(p, c->d_ftab,
-                                                                                                   c->d_geom);
+      build_blocks_affine_kernel<D, E::N, E::F, E::VG, E::SG><<<(unsigned)c->B, kAffineThreads, 0, st>>>(
+          p, c->d_ftab, c->d_geom, c->d_fnodes, c->d_rap_G);
+    c->rap_G_ready = c->d_rap_G != nullptr;
   } else {
+    c->rap_G_ready = false;
     auto k = build_blocks_kernel<D, E::N, E::F, E::VG, E::SG>;
     CK(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Sm)));
     if (c->B > 0) k<<<(unsigned)c->B, kBuildThreads, sizeof(Sm), st>>>(p, c->d_fnodes);
@@ -1187,63 +1274,10 @@ int dg_create(const dg_mesh_desc* m, const dg_config* cfg, dg_ctx** out) {
       for (int i = 0; i < N; ++i) fnod.slot[f][fnod.node[f][i]] = (signed char)i;
     }
     if ((rc = upload(c.get(), &c->d_fnodes, &fnod, 1))) return rc;
-    // reference matrices of the straight-sided (affine) block build, entry
-    // (m, n) of each N x N matrix at [m * N + n]: K[jj][kk], R[f][jj], Mf[f],
-    // Q[f][fn][al][jj], P[f][fn][al][jj], S[f][fn][al] (see
-    // build_blocks_affine_kernel)
-    const int NN = N * N;
-    const int nK = D * D, nR = F * D, nM = F, nQ = F * F * D * D, nS = F * F * D;
-    std::vector<double> ft((size_t)(nK + nR + nM + 2 * nQ + nS) * NN, 0.0);
-    double* tK = ft.data();
-    double* tR = tK + (size_t)nK * NN;
-    double* tM = tR + (size_t)nR * NN;
-    double* tQ = tM + (size_t)nM * NN;
-    double* tP = tQ + (size_t)nQ * NN;
-    double* tS = tP + (size_t)nQ * NN;
-    auto nlx = [&](int jj, int n, int g) { return m->nlx[(jj * N + n) * VG + g]; };
-    auto sn = [&](int f, int n, int g) { return m->sn[(f * N + n) * SG + g]; };
-    auto snlx = [&](int f, int jj, int n, int g) { return m->snlx[(size_t)f * D * N * SG + (jj * N + n) * SG + g]; };
-    for (int jj = 0; jj < D; ++jj)
-      for (int kk = 0; kk < D; ++kk)
-        for (int a = 0; a < N; ++a)
-          for (int b = 0; b < N; ++b) {
-            double t = 0.0;
-            for (int g = 0; g < VG; ++g) t += m->weight[g] * nlx(jj, a, g) * nlx(kk, b, g);
-            tK[(size_t)(jj * D + kk) * NN + a * N + b] = t;
-          }
-    for (int f = 0; f < F; ++f)
-      for (int a = 0; a < N; ++a)
-        for (int b = 0; b < N; ++b) {
-          double t = 0.0;
-          for (int g = 0; g < SG; ++g) t += m->sweight[g] * sn(f, a, g) * sn(f, b, g);
-          tM[(size_t)f * NN + a * N + b] = t;
-          for (int jj = 0; jj < D; ++jj) {
-            double r = 0.0;
-            for (int g = 0; g < SG; ++g) r += m->sweight[g] * sn(f, a, g) * snlx(f, jj, b, g);
-            tR[(size_t)(f * D + jj) * NN + a * N + b] = r;
-          }
-        }
-    for (int f = 0; f < F; ++f)
-      for (int fn = 0; fn < F; ++fn)
-        for (int lg = 0; lg < D; ++lg) {
-          const int cmb = (f * F + fn) * D + lg;
-          for (int a = 0; a < N; ++a)
-            for (int b = 0; b < N; ++b) {
-              double ts = 0.0;
-              for (int g = 0; g < SG; ++g) ts += m->sweight[g] * sn(f, a, g) * sn(fn, b, al[lg * SG + g]);
-              tS[(size_t)cmb * NN + a * N + b] = ts;
-              for (int jj = 0; jj < D; ++jj) {
-                double tq = 0.0, tp = 0.0;
-                for (int g = 0; g < SG; ++g) {
-                  const int ag = al[lg * SG + g];
-                  tq += m->sweight[g] * sn(f, a, g) * snlx(fn, jj, b, ag);
-                  tp += m->sweight[g] * snlx(f, jj, a, g) * sn(fn, b, ag);
-                }
-                tQ[(size_t)(cmb * D + jj) * NN + a * N + b] = tq;
-                tP[(size_t)(cmb * D + jj) * NN + a * N + b] = tp;
-              }
-            }
-        }
+    // reference matrices of the straight-sided (affine) block build (FastTab)
+    std::vector<double> ft;
+    if (D == 3) fill_fast_tab<3, 20, 4, 24, 12>(m, al.data(), fnod, ft);
+    else fill_fast_tab<2, 10, 3, 12, 4>(m, al.data(), fnod, ft);
     double* dft;
     if ((rc = upload_vec(c.get(), &dft, ft))) return rc;
     c->d_ftab = dft;
@@ -1378,11 +1412,13 @@ int dg_build_operator(dg_ctx* c, void* stream) {
   CK(c, cudaMemsetAsync(c->d_rar, 0, sizeof(double) * c->cola.size(), st));
   if (c->rap_direct && c->d_rap_ptr) {
     const int64_t nb = c->B * (c->F + 1);
-    if (c->D == 3)
+    if (!c->rap_G_ready) bump();
+    if (c->rap_G_ready) {
+      // formed with the blocks (straight-sided build)
+    } else if (c->D == 3)
       block_galerkin_kernel<20, 4><<<nblk(nb, 8), 160, 0, st>>>(c->d_blk, c->T.P, c->d_rap_G, nb);
     else
       block_galerkin_kernel<10, 3><<<nblk(nb, 16), 160, 0, st>>>(c->d_blk, c->T.P, c->d_rap_G, nb);
-    bump();
     rap_gather_kernel<<<nblk((int64_t)c->cola.size(), 128), 128, 0, st>>>(
         c->d_rap_G, c->d_rap_ptr, c->d_rap_ent, c->d_wdg, c->d_nbe, c->F, c->NC, c->d_rar,
         (int64_t)c->cola.size());
