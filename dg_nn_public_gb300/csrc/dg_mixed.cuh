@@ -84,6 +84,7 @@ struct Mixed {
   std::vector<std::vector<int>> g_kern;
   std::vector<bool> g_cond;
   bool cond = true;
+  bool tuned = false;   // launch shapes timed for this context and these options
   // Gram-Schmidt partial sums: one float4 of the vectors per thread,
   // nblk4 = ceil(nonods / 4 / 256) blocks, KMAXV sums per block
   double* part = nullptr;
@@ -900,6 +901,7 @@ int launch_bf16_tma(dg_ctx* c, Mixed& M, const float* x, const float* b, float* 
 // S stages; blocks are copied before the programmatic-launch wait (they are
 // fixed during a solve), x and c gathered after it.
 constexpr int kScVariants = 4;
+constexpr int SC_APPLY = 32;   // flag: x_out = W A x - c instead of the smoothing step
 
 // S_ef = W_e A_ef for the four faces of every element, in FP32 from the FP32
 // smoother matrices (column-major, W(m, n) at [n * 20 + m]) and the FP64
@@ -925,6 +927,111 @@ __global__ void __launch_bounds__(400) scaled_faces_kernel(const float* __restri
 #pragma unroll
     for (int k = 0; k < N; ++k) acc = fmaf(Ws[k * N + m], As[f][n * N + k], acc);
     out[(e * F + f) * N * N + chunk20_index(m, n)] = __float2bfloat16_rn(acc);
+  }
+}
+
+// All reduced-precision copies of an operator build in one pass over the FP64
+// blocks (3D, BF16 bulk-copy preconditioner, block-inverse smoother): the
+// five blocks in FP32 and BF16, W_e = w A_ee^-1 (FP32, Gauss-Jordan without
+// pivoting as block_inverse32_kernel) in FP32 and BF16, and the scaled faces
+// W_e A_ef in BF16, all in the chunked layouts.  One warp per element, lane m
+// = row m: each value is converted once (an FP64 -> FP32 conversion goes to
+// the FP64 pipe), staged in shared memory, and every output row is written in
+// 16-byte pieces.  err as block_inverse32_kernel; scf may be null.
+// Bound by HBM (16.0 KB read, 16.8 KB written per element) and the FP64
+// pipe's conversions.  131,712 tetrahedra: the five kernels of separate
+// passes 3.2 ms, this one 0.82 ms.
+__device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// row m of a block in the BF16 / FP32 chunked layouts
+__device__ __forceinline__ void store_row20(__nv_bfloat16* blk, int m, const float* v) {
+  *(reinterpret_cast<uint4*>(blk) + m) =
+      make_uint4(bf16_pair(v[0], v[1]), bf16_pair(v[2], v[3]), bf16_pair(v[4], v[5]), bf16_pair(v[6], v[7]));
+  *(reinterpret_cast<uint4*>(blk + kC20Off1) + m) =
+      make_uint4(bf16_pair(v[8], v[9]), bf16_pair(v[10], v[11]), bf16_pair(v[12], v[13]), bf16_pair(v[14], v[15]));
+  *(reinterpret_cast<uint2*>(blk + kC20Off2) + m) = make_uint2(bf16_pair(v[16], v[17]), bf16_pair(v[18], v[19]));
+}
+__device__ __forceinline__ void store_row20(float* blk, int m, const float* v) {
+#pragma unroll
+  for (int c = 0; c < 5; ++c)
+    *reinterpret_cast<float4*>(blk + 80 * c + 4 * m) = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+}
+
+constexpr int kCopyWarps = 4;
+__global__ void __launch_bounds__(32 * kCopyWarps) mixed_copies20_kernel(
+    const double* __restrict__ blk, int64_t B, float w, float* __restrict__ blk32, __nv_bfloat16* __restrict__ blk16,
+    float* __restrict__ W32, __nv_bfloat16* __restrict__ W16, __nv_bfloat16* __restrict__ scf, int* __restrict__ err) {
+  constexpr int N = 20, F = 4, NN = N * N;
+  __shared__ __align__(16) float As[kCopyWarps][NN];   // A(m, n) at [n * 20 + m]
+  const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t e = (int64_t)blockIdx.x * kCopyWarps + wi;
+  if (e >= B) return;   // whole warp; no block barrier below
+  float* S = As[wi];
+  const int m = lane < N ? lane : N - 1;   // lanes >= N repeat the last row, write nothing
+  float wr[N];                             // row m of W_e
+#pragma unroll 1
+  for (int b = 0; b <= F; ++b) {
+    const double2* src = reinterpret_cast<const double2*>(blk + (e * (F + 1) + b) * NN);
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 7; ++q) {
+      const int k = lane + 32 * q;
+      if (k < NN / 2) {
+        const double2 v = src[k];
+        *reinterpret_cast<float2*>(S + 2 * k) = make_float2((float)v.x, (float)v.y);
+      }
+    }
+    __syncwarp();
+    float a[N];
+#pragma unroll
+    for (int n = 0; n < N; ++n) a[n] = S[n * N + m];
+    if (lane < N) {
+      store_row20(blk32 + (e * (F + 1) + b) * NN, m, a);
+      store_row20(blk16 + (e * (F + 1) + b) * NN, m, a);
+    }
+    if (b == 0) {
+      bool bad = false;
+      const float dg = S[m * N + m];
+#pragma unroll
+      for (int k = 0; k < N; ++k) {
+        const float piv = __shfl_sync(0xffffffffu, a[k], k);
+        bad |= !(piv > 0.0f);   // uniform: every lane holds the same pivot
+        const float rp = 1.0f / piv;
+        const float f = a[k];
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+          if (n == k) continue;
+          const float pa = __shfl_sync(0xffffffffu, a[n], k) * rp;
+          a[n] = m == k ? pa : fmaf(-f, pa, a[n]);
+        }
+        a[k] = m == k ? rp : -f * rp;
+      }
+#pragma unroll
+      for (int n = 0; n < N; ++n) wr[n] = bad ? (m == n ? w / dg : 0.0f) : w * a[n];
+      if (bad && lane == 0) atomicExch(err, 2);
+      if (lane < N) {
+        store_row20(W32 + e * NN, m, wr);
+        store_row20(W16 + e * NN, m, wr);
+      }
+    } else if (scf) {
+#pragma unroll
+      for (int n = 0; n < N; ++n) {   // column n of A_ef, the same address for all lanes
+        float acc = 0.0f;
+#pragma unroll
+        for (int k = 0; k < N; k += 4) {
+          const float4 v = *reinterpret_cast<const float4*>(S + n * N + k);
+          acc = fmaf(wr[k], v.x, acc);
+          acc = fmaf(wr[k + 1], v.y, acc);
+          acc = fmaf(wr[k + 2], v.z, acc);
+          acc = fmaf(wr[k + 3], v.w, acc);
+        }
+        a[n] = acc;
+      }
+      if (lane < N) store_row20(scf + (e * F + b - 1) * NN, m, a);
+    }
   }
 }
 
@@ -1008,7 +1115,8 @@ __global__ void __launch_bounds__(EPB * 20, MINB) smooth_scaled_tma_kernel(
 #pragma unroll
       for (int f = 0; f < F; ++f)
         if (nbv[f] >= 0) acc = C::dot(C::lds(Se + f * BB, m), xs[le][f], acc);
-      x_out[e * N + m] = xo + wscale * (co - fmaf(w, xo, acc));
+      const float wa = fmaf(w, xo, acc);   // (W A x)_e
+      x_out[e * N + m] = (flags & SC_APPLY) ? wa - co : xo + wscale * (co - wa);
     }
     __syncthreads();   // stage s and xs free again
     if (tid == 0) {
@@ -1026,13 +1134,13 @@ __global__ void __launch_bounds__(EPB * 20, MINB) smooth_scaled_tma_kernel(
 
 template <int EPB, int S, int MINB>
 int launch_scaled_shape(dg_ctx* c, const __nv_bfloat16* sblk, const float* x, const float* cv, float* x_out,
-                        cudaStream_t st, const float* ws) {
+                        cudaStream_t st, const float* ws, int flags) {
   const int64_t ngroups = (c->B + EPB - 1) / EPB;
   const unsigned g = (unsigned)std::min<int64_t>(ngroups, (int64_t)c->nsm * MINB);
   const size_t smem = (size_t)S * EPB * 4 * Chunk20<__nv_bfloat16>::BlockBytes;
   return launch_k(c, smooth_scaled_tma_kernel<EPB, S, MINB>, g, EPB * 20, smem, st, sblk, (const int*)c->d_nbe, x,
                   cv, x_out, (int64_t)c->B, (float)c->mixed_smooth_w, ws, (int*)c->d_err,
-                  c->l2_hint ? (int)RF_STREAM_HINT : 0);
+                  flags | (c->l2_hint ? (int)RF_STREAM_HINT : 0));
 }
 
 template <int EPB, int S, int MINB>
@@ -1045,12 +1153,12 @@ int set_scaled_smem(dg_ctx* c) {
 // launch shapes (elements per group, stages, CTAs per SM) of the scaled-face
 // smoothing kernel, picked by autotune_mixed
 int launch_scaled(dg_ctx* c, const __nv_bfloat16* sblk, const float* x, const float* cv, float* x_out,
-                  cudaStream_t st, const float* ws) {
+                  cudaStream_t st, const float* ws, int flags = 0) {
   switch (c->sc_variant) {
-    case 1: return launch_scaled_shape<8, 2, 3>(c, sblk, x, cv, x_out, st, ws);
-    case 2: return launch_scaled_shape<4, 2, 6>(c, sblk, x, cv, x_out, st, ws);
-    case 3: return launch_scaled_shape<6, 3, 3>(c, sblk, x, cv, x_out, st, ws);
-    default: return launch_scaled_shape<6, 2, 4>(c, sblk, x, cv, x_out, st, ws);
+    case 1: return launch_scaled_shape<8, 2, 3>(c, sblk, x, cv, x_out, st, ws, flags);
+    case 2: return launch_scaled_shape<4, 2, 6>(c, sblk, x, cv, x_out, st, ws, flags);
+    case 3: return launch_scaled_shape<6, 3, 3>(c, sblk, x, cv, x_out, st, ws, flags);
+    default: return launch_scaled_shape<6, 2, 4>(c, sblk, x, cv, x_out, st, ws, flags);
   }
 }
 
@@ -1090,91 +1198,79 @@ __global__ void gj_update_kernel(double* __restrict__ G, int n, int k, const dou
 // ---------------------------------------------------------------------------
 // Blocked Gauss-Jordan inverse of the dense coarse level in FP32 (the
 // inverse is applied in FP32; the level matrix is symmetric positive
-// definite, so no pivoting).  G = [A | I] is n x 2n row-major.  Block step
-// over the rows and columns P = [k0, k0 + b):
-//   C = G[:, P] (copy; D = C[P, :]), Dinv = D^-1 (one CTA),
-//   G[P, :] = Dinv G[P, :],  G[i, :] -= C[i, :] G[P, :] for i not in P.
-// Columns left of k0 are already unit columns and the right half is still
-// zero beyond n + k0 + b in the rows of P, so a step touches the columns
-// [k0, n + k0 + b) only: n^3 FMAs in all, in n / b steps of four launches
-// instead of 2 n launches of the one-pivot form.
+// definite, so no pivoting), in place on an n x n matrix.  Block step over
+// the rows and columns P = [k0, k0 + b), D = A[P, P], R = D^-1 A[P, :]:
+//   B[P, P] = D^-1,  B[P, j] = R[:, j],  B[i, P] = -A[i, P] D^-1,
+//   B[i, j] = A[i, j] - A[i, P] R[:, j]   (i, j not in P).
+// One launch a step, from one buffer to the other, so that every CTA may
+// form D^-1 (one warp, a row per lane in registers) and its columns of R for
+// itself: the steps are a chain of n / 32 launches and their latency is what
+// bounds the inverse (before, a step was four launches, 63 us at n = 1,100,
+// 40 us of it the one-CTA inverse of D, on an augmented matrix that the host
+// assembled and uploaded).
 constexpr int kGjB = 32;
 
-__global__ void gjb_copy_kernel(const float* __restrict__ G, int n, int k0, int b, float* __restrict__ C) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n * b) return;
-  const int i = t / b, q = t % b;
-  C[t] = G[(size_t)i * 2 * n + k0 + q];
-}
-
-// Dinv = D^-1 for D = C[k0 .. k0+b, :] (b <= kGjB), one CTA of 256 threads
-__global__ void __launch_bounds__(256) gjb_dinv_kernel(const float* __restrict__ C, int k0, int b,
-                                                       float* __restrict__ Dinv, int* __restrict__ err) {
-  __shared__ float S[kGjB][2 * kGjB + 1];
-  __shared__ float f[kGjB];
-  for (int t = threadIdx.x; t < b * 2 * b; t += blockDim.x) {
-    const int r = t / (2 * b), j = t % (2 * b);
-    S[r][j] = j < b ? C[(size_t)(k0 + r) * b + j] : (j - b == r ? 1.0f : 0.0f);
-  }
-  __syncthreads();
-  for (int p = 0; p < b; ++p) {
-    const float piv = S[p][p];
-    if (!(piv > 0.0f)) {   // uniform
-      if (threadIdx.x == 0) atomicExch(err, 4);
-      return;
-    }
-    if (threadIdx.x < b) f[threadIdx.x] = S[threadIdx.x][p];
-    __syncthreads();
-    const float rp = 1.0f / piv;
-    for (int j = threadIdx.x; j < 2 * b; j += blockDim.x) S[p][j] *= rp;
-    __syncthreads();
-    for (int t = threadIdx.x; t < b * 2 * b; t += blockDim.x) {
-      const int r = t / (2 * b), j = t % (2 * b);
-      if (r != p) S[r][j] = fmaf(-f[r], S[p][j], S[r][j]);
-    }
-    __syncthreads();
-  }
-  for (int t = threadIdx.x; t < b * b; t += blockDim.x) Dinv[t] = S[t / b][b + t % b];
-}
-
-// G[P, j] = sum_q Dinv[r][q] G[k0 + q][j] for the columns j in [k0, n + k0 + b);
-// one thread per column (reads its b entries, then writes them)
-__global__ void __launch_bounds__(128) gjb_rows_kernel(float* __restrict__ G, int n, int k0, int b,
-                                                       const float* __restrict__ Dinv) {
-  __shared__ float Ds[kGjB * kGjB];
-  for (int t = threadIdx.x; t < b * b; t += blockDim.x) Ds[t] = Dinv[t];
-  __syncthreads();
-  const int j = k0 + blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= min(2 * n, n + k0 + b)) return;
-  float g[kGjB];
-#pragma unroll
-  for (int q = 0; q < kGjB; ++q) g[q] = q < b ? G[(size_t)(k0 + q) * 2 * n + j] : 0.0f;
-  for (int r = 0; r < b; ++r) {
-    float s = 0.0f;
-#pragma unroll
-    for (int q = 0; q < kGjB; ++q) s = fmaf(Ds[r * b + (q < b ? q : 0)], g[q], s);
-    G[(size_t)(k0 + r) * 2 * n + j] = s;
-  }
-}
-
-// G[i, j] -= sum_q C[i][q] G[k0 + q][j] for rows i not in P and columns j in
-// [k0 + b, n + k0 + b); G[i, P] = 0.  64 x 64 tiles, 256 threads of 4 x 4.
-__global__ void __launch_bounds__(256) gjb_update_kernel(float* __restrict__ G, int n, int k0, int b,
-                                                         const float* __restrict__ C) {
+__global__ void __launch_bounds__(256) gjb_step_kernel(const float* __restrict__ A, float* __restrict__ B, int n,
+                                                       int k0, int b, int* __restrict__ err) {
+  __shared__ float Ds[kGjB][kGjB + 1];
   __shared__ float Cs[64][kGjB + 1];
-  __shared__ __align__(16) float Rs[kGjB][64];
-  const int i0 = blockIdx.y * 64, j0 = k0 + b + blockIdx.x * 64;
-  const int jend = min(2 * n, n + k0 + b);
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  for (int t = threadIdx.x; t < 64 * kGjB; t += 256) {
-    const int r = t / kGjB, q = t % kGjB;
-    Cs[r][q] = (i0 + r < n && q < b) ? C[(size_t)(i0 + r) * b + q] : 0.0f;
-  }
-  for (int t = threadIdx.x; t < kGjB * 64; t += 256) {
-    const int q = t / 64, c = t % 64;
-    Rs[q][c] = (q < b && j0 + c < jend) ? G[(size_t)(k0 + q) * 2 * n + j0 + c] : 0.0f;
+  __shared__ __align__(16) float Rw[kGjB][64];   // A[P, j], then R
+  const int i0 = blockIdx.y * 64, j0 = blockIdx.x * 64;
+  const int t = threadIdx.x, lane = t & 31;
+  if (t < 32) {
+    float a[kGjB];   // row `lane` of D, padded with the identity
+#pragma unroll
+    for (int q = 0; q < kGjB; ++q)
+      a[q] = (lane < b && q < b) ? A[(size_t)(k0 + lane) * n + k0 + q] : (lane == q ? 1.0f : 0.0f);
+    bool bad = false;
+#pragma unroll
+    for (int p = 0; p < kGjB; ++p) {
+      const float piv = __shfl_sync(0xffffffffu, a[p], p);
+      bad |= !(piv > 0.0f);
+      const float rp = 1.0f / piv;
+      const float f = a[p];
+#pragma unroll
+      for (int q = 0; q < kGjB; ++q) {
+        if (q == p) continue;
+        const float pr = __shfl_sync(0xffffffffu, a[q], p) * rp;
+        a[q] = lane == p ? pr : fmaf(-f, pr, a[q]);
+      }
+      a[p] = lane == p ? rp : -f * rp;
+    }
+    if (bad && lane == 0) atomicExch(err, 4);
+#pragma unroll
+    for (int q = 0; q < kGjB; ++q) Ds[lane][q] = a[q];
+  } else {
+    for (int k = t - 32; k < 64 * kGjB; k += 224) {
+      const int r = k / kGjB, q = k % kGjB;
+      Cs[r][q] = (i0 + r < n && q < b) ? A[(size_t)(i0 + r) * n + k0 + q] : 0.0f;
+    }
+    for (int k = t - 32; k < kGjB * 64; k += 224) {
+      const int q = k / 64, j = j0 + k % 64;
+      float v = 0.0f;
+      if (q < b && j < n) v = (j >= k0 && j < k0 + b) ? (j - k0 == q ? 1.0f : 0.0f) : A[(size_t)(k0 + q) * n + j];
+      Rw[q][k % 64] = v;
+    }
   }
   __syncthreads();
+  {
+    // R = D^-1 A[P, j]: 8 rows of one column per thread
+    const int c = t % 64, r0 = (t / 64) * 8;
+    float acc[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) acc[u] = 0.0f;
+#pragma unroll 8
+    for (int q = 0; q < kGjB; ++q) {
+      const float v = Rw[q][c];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) acc[u] = fmaf(Ds[r0 + u][q], v, acc[u]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 8; ++u) Rw[r0 + u][c] = acc[u];
+  }
+  __syncthreads();
+  const int tx = t % 16, ty = t / 16;
   float acc[4][4];
 #pragma unroll
   for (int u = 0; u < 4; ++u)
@@ -1182,7 +1278,7 @@ __global__ void __launch_bounds__(256) gjb_update_kernel(float* __restrict__ G, 
     for (int v = 0; v < 4; ++v) acc[u][v] = 0.0f;
 #pragma unroll 8
   for (int q = 0; q < kGjB; ++q) {
-    const float4 rv = *reinterpret_cast<const float4*>(&Rs[q][4 * tx]);
+    const float4 rv = *reinterpret_cast<const float4*>(&Rw[q][4 * tx]);
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const float cv = Cs[4 * ty + u][q];
@@ -1195,24 +1291,32 @@ __global__ void __launch_bounds__(256) gjb_update_kernel(float* __restrict__ G, 
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
     const int i = i0 + 4 * ty + u;
-    if (i >= n || (i >= k0 && i < k0 + b)) continue;
-    float* row = G + (size_t)i * 2 * n;
+    if (i >= n) continue;
+    const bool inP = i >= k0 && i < k0 + b;
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
       const int j = j0 + 4 * tx + v;
-      if (j < jend) row[j] -= acc[u][v];
+      if (j >= n) continue;
+      float o;
+      if (inP) o = Rw[i - k0][4 * tx + v];
+      else o = ((j >= k0 && j < k0 + b) ? 0.0f : A[(size_t)i * n + j]) - acc[u][v];
+      B[(size_t)i * n + j] = o;
     }
-    if (blockIdx.x == 0)   // the block's own columns become zero
-      for (int q = tx; q < b; q += 16) row[k0 + q] = 0.0f;
   }
 }
 
-// inv (n x n FP32) = right half of the FP32 G
-__global__ void gjb_extract_kernel(const float* __restrict__ G, int n, float* __restrict__ inv) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (int64_t)n * n) return;
-  const int64_t i = t / n, j = t % n;
-  inv[t] = G[i * 2 * n + n + j];
+// Dense n x n matrix (row length ld) of an SFC level from its CSR arrays, one
+// warp per row; with unit, the columns n .. 2n of the row become row i of the
+// identity (the augmented form of the one-pivot inverse)
+template <typename T>
+__global__ void dense_fill_kernel(const int* __restrict__ rowptr, const int* __restrict__ col,
+                                  const double* __restrict__ val, int n, int ld, T* __restrict__ G, int unit) {
+  const int i = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
+  if (i >= n) return;   // whole warp
+  T* row = G + (size_t)i * ld;
+  for (int j = lane; j < (unit ? 2 * n : n); j += 32) row[j] = (unit && j == n + i) ? (T)1 : (T)0;
+  __syncwarp();
+  for (int k = rowptr[i] + lane; k < rowptr[i + 1]; k += 32) row[col[k]] = (T)val[k];   // columns of a row differ
 }
 
 // inv (n x n FP32) = right half of G
@@ -1879,6 +1983,24 @@ __global__ void convert_f64_f32_kernel(const ST* __restrict__ a, float* __restri
   if (k < n) b[k] = (float)a[k];
 }
 
+// FP32 copies of SFC level values and diagonals: one grid row per level
+constexpr int kLevCopies = 24;
+struct LevCopies {
+  struct {
+    const double* val;
+    float* val32;
+    const double* diag;
+    float* diag32;
+    int nnz, n;
+  } l[kLevCopies];
+};
+__global__ void lev_copies_kernel(LevCopies p) {
+  const auto& L = p.l[blockIdx.y];
+  const int k0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  for (int k = k0; k < L.nnz; k += stride) L.val32[k] = (float)L.val[k];
+  for (int k = k0; k < L.n; k += stride) L.diag32[k] = (float)L.diag[k];
+}
+
 // Deterministic start vector of the power iteration: a hash of the index
 // mapped to [-1, 1).
 __global__ void probe_init_kernel(float* __restrict__ v, int64_t n) {
@@ -1920,31 +2042,34 @@ int set_smoother_schedule(dg_ctx* c, cudaStream_t st) {
   probe_init_kernel<<<nblk(n, 256), 256, 0, st>>>(v, n);
   bump();
   CK(c, cudaMemsetAsync(zb, 0, sizeof(float) * n, st));
+  // the iterates are not normalised: they grow by w lambda <= 1.6 a step, 1e8
+  // in 40 steps, and an estimate is the ratio of two norms
   if ((rc = norm32(c, v, c->d_scal, st))) return rc;
-  scale_kernel<float><<<nblk(n, 256), 256, 0, st>>>(v, c->d_scal, v, n);
-  bump();
-  // the estimates of a run of steps stay on the device (d_scal[1 + it]) and
+  // the norms of a run of steps stay on the device (d_scal[1 + it]) and
   // are read once per run, not once per step; the stop is the first step
   // it >= 8 whose estimate moved by at most 1e-3 (later steps of the run
   // change nothing that is used)
   constexpr int kMaxIts = 40;
   double lam = 0.0, prev = -1.0;
-  std::vector<double> lams(kMaxIts, 0.0);
+  std::vector<double> nrm(kMaxIts + 1, 0.0);   // nrm[1 + it] = norm after step it
   bool stop = false;
   for (int it0 = 0; it0 < kMaxIts && !stop;) {
     const int run = it0 == 0 ? 9 : std::min(8, kMaxIts - it0);
     for (int it = it0; it < it0 + run; ++it) {
-      if ((rc = smooth_step(c, v, zb, u, st, nullptr))) return rc;   // u = v - W A v (c = W zb = 0)
-      sub_f32_kernel<<<nblk(n, 256), 256, 0, st>>>(v, u, v, n);                 // v <- W A v
-      bump();
+      if (M.sc) {   // W A v in one launch
+        if ((rc = launch_scaled(c, M.scblk16, v, zb, u, st, nullptr, SC_APPLY))) return rc;
+        std::swap(u, v);
+      } else {
+        if ((rc = smooth_step(c, v, zb, u, st, nullptr))) return rc;   // u = v - W A v
+        sub_f32_kernel<<<nblk(n, 256), 256, 0, st>>>(v, u, v, n);       // v <- W A v
+        bump();
+      }
       if ((rc = norm32(c, v, c->d_scal + 1 + it, st))) return rc;
-      scale_kernel<float><<<nblk(n, 256), 256, 0, st>>>(v, c->d_scal + 1 + it, v, n);
-      bump();
     }
-    CK(c, cudaMemcpyAsync(lams.data() + it0, c->d_scal + 1 + it0, sizeof(double) * run, cudaMemcpyDeviceToHost, st));
+    CK(c, cudaMemcpyAsync(nrm.data() + it0, c->d_scal + it0, sizeof(double) * (run + 1), cudaMemcpyDeviceToHost, st));
     CK(c, cudaStreamSynchronize(st));
     for (int it = it0; it < it0 + run; ++it) {
-      lam = lams[it];
+      lam = nrm[1 + it] / nrm[it];
       if (!(lam > 0.0) || !std::isfinite(lam)) return DG_OK;
       if (it >= 8 && std::fabs(lam - prev) <= 1e-3 * lam) {
         stop = true;
@@ -2020,9 +2145,10 @@ int build_mixed(dg_ctx* c, cudaStream_t st) {
                                                                                         M.sblk16, ns);
     bump();
     CKL(c);
-  } else if ((rc = build_blk5(c, st))) {
-    return rc;
   }
+  // one pass over the blocks forms every copy of the default configuration
+  const bool one_pass = c->D == 3 && c->f32_tma && c->pc_bf16() && !M.sf && c->mixed_smoother == 1;
+  if (!M.sf && !one_pass && (rc = build_blk5(c, st))) return rc;
   auto vt = [&](const char* what) {   // verbose phase timings
     if (!c->verbose) return;
     cudaStreamSynchronize(st);
@@ -2035,7 +2161,25 @@ int build_mixed(dg_ctx* c, cudaStream_t st) {
   const double* Wsrc = c->d_W;
   const float* Wsrc32 = nullptr;
   double* Winv = nullptr;
-  if (c->mixed_smoother == 1) {
+  // scaled face blocks of the BF16 bulk-copy smoothing steps (the smoother
+  // must be the damped block inverse: its self block is then w I)
+  M.sc = c->scaled_faces && c->D == 3 && c->precond_bf16 && c->bf16_tma && !M.sf && c->mixed_smoother == 1;
+  if (M.sc) {
+    if (!M.scblk16 && (rc = dalloc(c, &M.scblk16, (size_t)c->B * 4 * 400))) return rc;
+    if (!M.chat && (rc = dalloc(c, &M.chat, (size_t)c->nonods))) return rc;
+  }
+  if (one_pass) {
+    const size_t nb = (size_t)c->B * (c->F + 1) * c->N * c->N;
+    if (!M.blk && (rc = dalloc(c, &M.blk, nb))) return rc;
+    if (!M.blk16 && (rc = dalloc(c, &M.blk16, nb))) return rc;
+    if (!M.W16 && (rc = dalloc(c, &M.W16, nw))) return rc;
+    CK(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), st));
+    mixed_copies20_kernel<<<nblk(c->B, kCopyWarps), 32 * kCopyWarps, 0, st>>>(
+        c->d_blk, c->B, (float)c->mixed_smooth_w, M.blk, M.blk16, M.W, M.W16, M.sc ? M.scblk16 : nullptr, c->d_err);
+    bump();
+    CKL(c);
+    M.has5 = true;
+  } else if (c->mixed_smoother == 1) {
     // scratch kept with the context: a cudaFree here would wait for every
     // stream of the device (other contexts' solves on a serving GPU)
     if (!M.winv && (rc = dalloc(c, &M.winv, nw))) return rc;
@@ -2068,20 +2212,15 @@ int build_mixed(dg_ctx* c, cudaStream_t st) {
     }
     return DG_OK;
   };
-  if ((rc = Wsrc32 ? copies(Wsrc32) : copies(Wsrc))) return rc;
-  if (Winv) {
+  if (!one_pass && (rc = Wsrc32 ? copies(Wsrc32) : copies(Wsrc))) return rc;
+  if (one_pass || Winv) {
     int herr = 0;
     CK(c, cudaMemcpyAsync(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(c, cudaStreamSynchronize(st));
     if (herr) return fail(c, DG_ERR_NUMERIC, "element block with a non-positive pivot (not positive definite)");
   }
   vt("smoother copies");
-  // scaled face blocks of the BF16 bulk-copy smoothing steps (the smoother
-  // must be the damped block inverse: its self block is then w I)
-  M.sc = c->scaled_faces && c->D == 3 && c->precond_bf16 && c->bf16_tma && !M.sf && Wsrc32 != nullptr;
-  if (M.sc) {
-    if (!M.scblk16 && (rc = dalloc(c, &M.scblk16, (size_t)c->B * 4 * 400))) return rc;
-    if (!M.chat && (rc = dalloc(c, &M.chat, (size_t)c->nonods))) return rc;
+  if (M.sc && !one_pass) {
     scaled_faces_kernel<<<(unsigned)c->B, 400, 0, st>>>(Wsrc32, c->d_blk, M.scblk16, (int64_t)c->B);
     bump();
     CKL(c);
@@ -2096,23 +2235,23 @@ int build_mixed(dg_ctx* c, cudaStream_t st) {
       L.rowptr = D.rowptr;
       L.col = D.col;
       L.up = D.up;
-      int nnz = 0;
-      CK(c, cudaMemcpyAsync(&nnz, D.rowptr + D.n, sizeof(int), cudaMemcpyDeviceToHost, st));
-      CK(c, cudaStreamSynchronize(st));
-      if ((rc = dalloc(c, &L.val, (size_t)nnz))) return rc;
+      if ((rc = dalloc(c, &L.val, (size_t)D.nnz))) return rc;
       for (float** t : {&L.diag, &L.e, &L.e2, &L.r, &L.rr})
         if ((rc = dalloc(c, t, (size_t)L.n))) return rc;
     }
   }
-  for (size_t l = 0; l < c->lev.size(); ++l) {
-    Lev32& L = M.lev[l];
-    const DevLevel& D = c->lev[l];
-    int nnz = 0;
-    CK(c, cudaMemcpyAsync(&nnz, D.rowptr + D.n, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(c, cudaStreamSynchronize(st));
-    convert_f64_f32_kernel<<<nblk(nnz, 256), 256, 0, st>>>(D.val, L.val, nnz);
-    bump();
-    convert_f64_f32_kernel<<<nblk(D.n, 256), 256, 0, st>>>(D.diag, L.diag, D.n);
+  for (size_t l0 = 0; l0 < c->lev.size(); l0 += kLevCopies) {
+    // FP32 copies of the level values and diagonals, all levels in one launch
+    LevCopies p;
+    const int cnt = (int)std::min<size_t>(kLevCopies, c->lev.size() - l0);
+    int longest = 1;
+    for (int k = 0; k < cnt; ++k) {
+      const DevLevel& D = c->lev[l0 + k];
+      Lev32& L = M.lev[l0 + k];
+      p.l[k] = {D.val, L.val, D.diag, L.diag, D.nnz, D.n};
+      longest = std::max(longest, std::max(D.nnz, D.n));
+    }
+    lev_copies_kernel<<<dim3((unsigned)std::min(4 * c->nsm, (longest + 255) / 256), cnt), 256, 0, st>>>(p);
     bump();
   }
   if (c->verbose) CK(c, cudaStreamSynchronize(st));
@@ -2126,67 +2265,43 @@ int build_mixed(dg_ctx* c, cudaStream_t st) {
       if (h.sizes[l] <= c->dense_max32) { lc = l; break; }
     if (lc >= 0) {
       const int n = (int)h.sizes[lc];
-      // augmented [A | I] assembled on the host from the level's device CSR
-      // (its values are formed on the device after the first build),
-      // inverted on the GPU
+      // the level's matrix, dense, in scratch kept with the context: two n x n
+      // FP32 buffers, or the FP64 augmented matrix with pivot row and column
       const DevLevel& DL = c->lev[lc];
-      std::vector<int> drp(n + 1);
-      CK(c, cudaMemcpyAsync(drp.data(), DL.rowptr, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost, st));
-      CK(c, cudaStreamSynchronize(st));
-      std::vector<int> dcl(drp[n]);
-      std::vector<double> dvl(drp[n]);
-      CK(c, cudaMemcpyAsync(dcl.data(), DL.col, sizeof(int) * drp[n], cudaMemcpyDeviceToHost, st));
-      CK(c, cudaMemcpyAsync(dvl.data(), DL.val, sizeof(double) * drp[n], cudaMemcpyDeviceToHost, st));
-      CK(c, cudaStreamSynchronize(st));
-      std::vector<double> Gh((size_t)n * 2 * n, 0.0);
-      for (int i = 0; i < n; ++i) {
-        for (int k = drp[i]; k < drp[i + 1]; ++k) Gh[(size_t)i * 2 * n + dcl[k]] += dvl[k];
-        Gh[(size_t)i * 2 * n + n + i] = 1.0;
-      }
-      // augmented matrix and pivot row / column (FP64 form) or the FP32
-      // augmented matrix, panel copy and block inverse, kept with the context
-      const size_t gneed = std::max(Gh.size() + 3 * (size_t)n,
-                                    (Gh.size() + (size_t)kGjB * n + (size_t)kGjB * kGjB + 1) / 2);
+      const size_t nn = (size_t)n * n;
+      const size_t gneed = c->dense_fp64 ? 2 * nn + 3 * (size_t)n : (nn + 1) / 2;
       if (M.gj_cap < gneed) {
         if ((rc = dalloc(c, &M.gj, gneed))) return rc;
         M.gj_cap = gneed;
       }
       if (!M.dense_inv || c->dense_n != n) {
-        if ((rc = dalloc(c, &M.dense_inv, (size_t)n * n))) return rc;
+        if ((rc = dalloc(c, &M.dense_inv, nn))) return rc;
         c->dense_n = n;
       }
       CK(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), st));
       if (c->dense_fp64) {
         // one pivot per launch pair, FP64 (DG_DENSE_FP64=1)
         double* G = M.gj;
-        double* fcol = G + Gh.size();
+        double* fcol = G + 2 * nn;
         double* prow = fcol + n;
-        CK(c, cudaMemcpyAsync(G, Gh.data(), sizeof(double) * Gh.size(), cudaMemcpyHostToDevice, st));
+        dense_fill_kernel<double><<<nblk(n, 8), 256, 0, st>>>(DL.rowptr, DL.col, DL.val, n, 2 * n, G, 1);
         for (int k = 0; k < n; ++k) {
           gj_prep_kernel<<<nblk(2 * n - k > n ? 2 * n - k : n, 256), 256, 0, st>>>(G, n, k, fcol, prow, c->d_err);
           gj_update_kernel<<<dim3(nblk(2 * n - k, 256), n), 256, 0, st>>>(G, n, k, fcol, prow);
         }
-        bump(2 * (long long)n);
+        bump(2 * (long long)n + 1);
         gj_extract_kernel<<<nblk((int64_t)n * n, 256), 256, 0, st>>>(G, n, M.dense_inv);
         bump();
       } else {
-        // blocked FP32 form in the same scratch: G (n x 2n), C (n x kGjB), Dinv
-        float* G = reinterpret_cast<float*>(M.gj);
-        float* C = G + Gh.size();
-        float* Dinv = C + (size_t)n * kGjB;
-        std::vector<float> Gf(Gh.begin(), Gh.end());
-        CK(c, cudaMemcpyAsync(G, Gf.data(), sizeof(float) * Gf.size(), cudaMemcpyHostToDevice, st));
-        for (int k0 = 0; k0 < n; k0 += kGjB) {
-          const int b = std::min(kGjB, n - k0);
-          gjb_copy_kernel<<<nblk((int64_t)n * b, 256), 256, 0, st>>>(G, n, k0, b, C);
-          gjb_dinv_kernel<<<1, 256, 0, st>>>(C, k0, b, Dinv, c->d_err);
-          gjb_rows_kernel<<<nblk(n + b, 128), 128, 0, st>>>(G, n, k0, b, Dinv);
-          gjb_update_kernel<<<dim3((unsigned)((n + 63) / 64), (unsigned)((n + 63) / 64)), 256, 0, st>>>(G, n, k0, b,
-                                                                                                     C);
-          bump(4);
-        }
-        gjb_extract_kernel<<<nblk((int64_t)n * n, 256), 256, 0, st>>>(G, n, M.dense_inv);
-        bump();
+        // blocked FP32 form; an even or odd number of steps must end in dense_inv
+        float* buf[2] = {reinterpret_cast<float*>(M.gj), M.dense_inv};
+        const int steps = (n + kGjB - 1) / kGjB;
+        int cur = steps % 2 == 0 ? 1 : 0;
+        dense_fill_kernel<float><<<nblk(n, 8), 256, 0, st>>>(DL.rowptr, DL.col, DL.val, n, n, buf[cur], 0);
+        for (int k0 = 0; k0 < n; k0 += kGjB, cur ^= 1)
+          gjb_step_kernel<<<dim3(nblk(n, 64), nblk(n, 64)), 256, 0, st>>>(buf[cur], buf[cur ^ 1], n, k0,
+                                                                          std::min(kGjB, n - k0), c->d_err);
+        bump(steps + 1);
       }
       int herr = 0;
       CK(c, cudaMemcpyAsync(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -2786,11 +2901,16 @@ double hessenberg_ls(const std::vector<double>& Hcm, int m, int k, double beta, 
 // Launch-shape autotuner for the single-RHS bulk-copy kernels: times every
 // candidate shape (elements per group, stages, CTAs per SM) of the BF16
 // smoothing step on zeroed scratch vectors with CUDA events (one warm launch,
-// then 5 timed) and keeps the fastest.  Runs once per operator build before
-// any graph capture; cached graphs are dropped when the choice changes.
+// then 5 timed) and keeps the fastest.  Runs once per context and set of
+// options (the time depends on the mesh and the layout of the copies, not on
+// their values: at each rebuild it cost 4 ms of a 49 ms request at 131,712
+// tetrahedra), before any graph capture; cached graphs are dropped when the
+// choice changes.
 int autotune_mixed(dg_ctx* c, cudaStream_t st) {
   if (!c->autotune || c->D != 3 || !c->precond_bf16 || !c->bf16_tma) return DG_OK;
   Mixed& M = mixed_of(c);
+  if (M.tuned) return DG_OK;
+  M.tuned = true;
   const int64_t n = c->nonods;
   CK(c, cudaMemsetAsync(M.t2, 0, sizeof(float) * n, st));
   CK(c, cudaMemsetAsync(M.t3, 0, sizeof(float) * n, st));
@@ -3145,6 +3265,7 @@ extern "C" int dg_set_mixed_options(dg_ctx* c, int32_t smoother, double smooth_w
   c->dense_max32 = dense_max;
   c->mixed_version = -1;   // rebuild the mixed operator copies
   Mixed& M = mixed_of(c);
+  M.tuned = false;
   for (auto& g : M.graphs)
     if (g) cudaGraphExecDestroy(g);
   M.graphs.clear();
