@@ -87,6 +87,25 @@ __device__ __forceinline__ void jacobian(const double* __restrict__ d, int npts,
     }
 }
 
+// The same Jacobian from node positions relative to the element's first node
+// (the derivatives of a constant sum to zero): the products then have the
+// element's size instead of the coordinates', so their rounding does not grow
+// by |x| / h.  The straight-sided build, with one Jacobian per element and no
+// averaging over points, takes this form.
+template <int D, int N>
+__device__ __forceinline__ void jacobian_local(const double* __restrict__ d, int npts, int g, const double* xe,
+                                               double* j) {
+#pragma unroll
+  for (int i = 0; i < D; ++i)
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+      double s = 0.0;
+#pragma unroll 4
+      for (int n = 1; n < N; ++n) s += __ldg(d + (i * N + n) * npts + g) * (xe[k * N + n] - xe[k * N]);
+      j[i * D + k] = s;
+    }
+}
+
 // Face tangents, unit outward normal and area element at a face point.
 template <int D>
 __device__ __forceinline__ double face_normal(const double* j, const double* drst_f, double* nrm) {
@@ -447,7 +466,7 @@ __global__ void __launch_bounds__(128) geom_affine_kernel(BuildParams p, double*
   const Tables& T = p.T;
   double* rec = geom + e * G::Size;
   double j[D * D], Mi[D * D];
-  jacobian<D, N>(T.nlx, VG, 0, p.x + e * D * N, j);
+  jacobian_local<D, N>(T.nlx, VG, 0, p.x + e * D * N, j);
   const double det = inv_det<D>(j, Mi);
   if (!(det > 0.0)) atomicExch(p.err, 1);
   rec[G::Det] = det;
@@ -480,7 +499,7 @@ __global__ void __launch_bounds__(128) geom_affine_kernel(BuildParams p, double*
     const int nb = p.nbe[e * F + f];
     if (nb >= 0) {
       double jn[D * D], mn[D * D];
-      jacobian<D, N>(T.nlx, VG, 0, p.x + (int64_t)nb * D * N, jn);
+      jacobian_local<D, N>(T.nlx, VG, 0, p.x + (int64_t)nb * D * N, jn);
       inv_det<D>(jn, mn);
 #pragma unroll
       for (int jj = 0; jj < D; ++jj) {
@@ -838,7 +857,6 @@ __global__ void __launch_bounds__(EPB* N) residual_kernel(const MT* __restrict__
                                                           int flags, const double* __restrict__ P = nullptr,
                                                           VT* __restrict__ r1 = nullptr,
                                                           const float* __restrict__ wsp = nullptr) {
-  const AT wscale = wsp ? (AT)*wsp : (AT)1;
   __shared__ AT xs[EPB][F + 1][N];
   __shared__ AT rs[EPB][N];
   __shared__ int nbs[EPB][F];
@@ -846,7 +864,8 @@ __global__ void __launch_bounds__(EPB* N) residual_kernel(const MT* __restrict__
   const int64_t e = (int64_t)blockIdx.x * EPB + le;
   const bool valid = e < B;
   const bool zerox = flags & RF_ZEROX;
-  if (valid && m < F) nbs[le][m] = nbe[e * F + m];
+  if (valid && m < F) nbs[le][m] = nbe[e * F + m];   // fixed data: read before the wait
+  pdl_wait_then_trigger();
   __syncthreads();
   if (valid && !zerox) {
     xs[le][0][m] = (AT)x[e * N + m];
@@ -897,6 +916,7 @@ __global__ void __launch_bounds__(EPB* N) residual_kernel(const MT* __restrict__
       AT c = 0;
 #pragma unroll
       for (int n = 0; n < N; ++n) c += (AT)We[n * N + m] * rs[le][n];
+      const AT wscale = wsp ? (AT)*wsp : (AT)1;
       x_out[e * N + m] = (VT)((zerox ? (AT)0 : xs[le][0][m]) + wscale * c);
     }
   }

@@ -186,6 +186,38 @@ __global__ void prolong_cg_kernel(T* __restrict__ x, const T* __restrict__ ecg,
   x[t] = add ? x[t] + v : v;
 }
 
+// x[e][n] += sum_c P[n][c] (w_ec ecg[pos(p1cg[e][c])]): prolong_cg_kernel for
+// the coarse correction, with an element's corner values formed once (threads
+// m < NC) instead of by each of its node threads.  Same products and order.
+template <int N, int NC, int EPB>
+__global__ void __launch_bounds__(EPB* N) prolong_add_kernel(double* __restrict__ x, const double* __restrict__ ecg,
+                                                             const int* __restrict__ pos,
+                                                             const int* __restrict__ p1cg,
+                                                             const double* __restrict__ wdg,
+                                                             const double* __restrict__ P, int64_t B) {
+  __shared__ double vc[EPB][NC];
+  const int le = threadIdx.x / N, n = threadIdx.x % N;
+  const int64_t e = (int64_t)blockIdx.x * EPB + le;
+  const bool valid = e < B;
+  int vp = 0;
+  double w = 0.0;
+  if (valid && n < NC) {
+    vp = pos[p1cg[e * NC + n]];
+    w = wdg[e * NC + n];
+  }
+  double p[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) p[c] = P[n * NC + c];
+  pdl_wait_then_trigger();
+  if (valid && n < NC) vc[le][n] = w * ecg[vp];
+  __syncthreads();
+  if (!valid) return;
+  double v = 0.0;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) v += p[c] * vc[le][c];
+  x[e * N + n] += v;
+}
+
 // value[spidx[k]] += rarm[colidx[k]] for the probe entries of one colour
 __global__ void rar_scatter_kernel(double* __restrict__ value, const double* __restrict__ rarm,
                                    const int* __restrict__ spidx, const int* __restrict__ colidx,
@@ -325,6 +357,65 @@ __global__ void lev_jacobi_kernel(const int* __restrict__ rowptr, const int* __r
   if (rr_out) rr_out[i] = rr;
 }
 
+// SFC-level Jacobi sweep (lev_jacobi_kernel, LPR lanes per row) whose
+// input iterate is formed on the fly from the neighbouring level, so that
+// the transfer between levels needs no launch of its own:
+//   MODE 1 (restriction in): e_in[j] = ea[2j] + ea[2j+1] and
+//     r[i] = eb[2i] + eb[2i+1] (zero pad at n_src; lev_restrict_kernel),
+//     r is stored for the level's later sweeps;
+//   MODE 2 (prolongation in): e_in[j] = ea[j] + eb[up[j]]
+//     (lev_prolong_kernel), r read as given.
+// Then rr = r - A e_in, e_out = e_in + rr / diag * w, rr_out = rr (if set):
+// the same operations as the transfer launch followed by the sweep.
+template <int MODE, typename T = float>
+__global__ void lev_jacobi_x_kernel(const int* __restrict__ rowptr, const int* __restrict__ col,
+                                    const T* __restrict__ val, const T* __restrict__ diag,
+                                    const T* __restrict__ ea, const T* __restrict__ eb,
+                                    const int* __restrict__ up, int n_src, T* __restrict__ r,
+                                    T* __restrict__ e_out, T* __restrict__ rr_out, int n, T w) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = t / LPR, lane = t % LPR;
+  constexpr int PRE = 4;
+  int k0 = 0, k1 = 0;
+  int cpre[PRE];
+  T vpre[PRE];
+  if (i < n) {
+    k0 = rowptr[i] + lane;
+    k1 = rowptr[i + 1];
+  }
+#pragma unroll
+  for (int q = 0; q < PRE; ++q) {
+    const int k = k0 + q * LPR;
+    cpre[q] = k < k1 ? col[k] : 0;
+    vpre[q] = k < k1 ? val[k] : (T)0;
+  }
+  pdl_wait_then_trigger();
+  auto ein = [&](int j) -> T {
+    if (MODE == 1) return ea[2 * j] + (2 * j + 1 < n_src ? ea[2 * j + 1] : (T)0);
+    return ea[j] + eb[up[j]];
+  };
+  T s = 0;
+  if (i < n) {
+#pragma unroll
+    for (int q = 0; q < PRE; ++q)
+      if (k0 + q * LPR < k1) s = fma_t(vpre[q], ein(cpre[q]), s);
+    for (int k = k0 + PRE * LPR; k < k1; k += LPR) s = fma_t(val[k], ein(col[k]), s);
+  }
+#pragma unroll
+  for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, LPR);
+  if (i >= n || lane != 0) return;
+  T ri;
+  if (MODE == 1) {
+    ri = eb[2 * i] + (2 * i + 1 < n_src ? eb[2 * i + 1] : (T)0);
+    r[i] = ri;
+  } else {
+    ri = r[i];
+  }
+  const T rr = ri - s;
+  e_out[i] = fma_t(rr / diag[i], w, ein(i));
+  if (rr_out) rr_out[i] = rr;
+}
+
 // pair sums with a zero pad (F.pad + Conv1d([1, 1], stride 2), :147-153)
 template <typename T = double>
 __global__ void lev_restrict_kernel(const T* __restrict__ rr, const T* __restrict__ e,
@@ -445,6 +536,173 @@ __global__ void reduce_partial_kernel(const double* __restrict__ partial, int nb
     if (take_sqrt) t = sqrt(t);
     out[i] = accumulate ? out[i] + t : t;
   }
+}
+
+// sum over the warp of 8 per-lane values with 9 additions a lane instead of
+// 40 (FP64 additions share the narrow FP64 pipe): halves of the values are
+// exchanged until a lane holds one of them.  Lane l returns the sum of value
+// (l >> 2) & 7 (complete in lanes with l % 4 == 0).
+__device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
+#pragma unroll
+  for (int w = 4, o = 16; w >= 1; w >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int q = 0; q < w; ++q) {
+      const double give = up ? v[q] : v[q + w], keep = up ? v[q + w] : v[q];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  double s = v[0];
+  s += __shfl_down_sync(0xffffffffu, s, 2);
+  s += __shfl_down_sync(0xffffffffu, s, 1);
+  return s;
+}
+
+// partial[bx * KMAXV + i] = this block's slice of V[i] . z for the vectors
+// i of grid row y (8 each), FP64, two entries a load (n even).  z is read once
+// per 8 vectors.  Bound by the FP64 pipe (one FMA per 8 bytes of V).  960,000
+// rows, 15 vectors on average: 41 -> 30 us a pass.
+template <int TB>
+__global__ void __launch_bounds__(TB) mdot8_f64_kernel(const double* __restrict__ V, int64_t ld, int nv,
+                                                       const double* __restrict__ z, int64_t n2,
+                                                       double* __restrict__ partial) {
+  pdl_wait_then_trigger();
+  __shared__ double red[TB / 32][8];
+  const int i0 = blockIdx.y * 8;
+  const int cnt = min(8, nv - i0);
+  double acc[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) acc[q] = 0.0;
+  const double2* z2 = reinterpret_cast<const double2*>(z);
+  if (cnt == 8) {
+    for (int64_t k = (int64_t)blockIdx.x * TB + threadIdx.x; k < n2; k += (int64_t)gridDim.x * TB) {
+      const double2 zv = z2[k];
+      double2 v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = reinterpret_cast<const double2*>(V + (size_t)(i0 + q) * ld)[k];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[q] = fma(v[q].y, zv.y, fma(v[q].x, zv.x, acc[q]));
+    }
+  } else {   // fewer vectors: no FP64 work for the missing ones
+    for (int64_t k = (int64_t)blockIdx.x * TB + threadIdx.x; k < n2; k += (int64_t)gridDim.x * TB) {
+      const double2 zv = z2[k];
+#pragma unroll
+      for (int q = 0; q < 7; ++q)
+        if (q < cnt) {
+          const double2 v = reinterpret_cast<const double2*>(V + (size_t)(i0 + q) * ld)[k];
+          acc[q] = fma(v.y, zv.y, fma(v.x, zv.x, acc[q]));
+        }
+    }
+  }
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const double a = warp_sum8(acc, lane);
+  if ((lane & 3) == 0) red[wid][lane >> 2] = a;
+  __syncthreads();
+  if (threadIdx.x < cnt) {
+    double s = 0.0;
+    for (int w = 0; w < TB / 32; ++w) s += red[w][threadIdx.x];
+    partial[(int64_t)blockIdx.x * KMAXV + i0 + threadIdx.x] = s;
+  }
+}
+
+// z -= sum_i V[i] h[i] (nv <= 256, n even); with want_norm also
+// partial_out[bx * KMAXV] = this block's slice of |z_new|^2.  With nred > 0
+// the coefficients are first summed here from the partial sums of the dots
+// (partial_in, nv <= KMAXV; every block sums them in the same order) and
+// block 0 stores them in h_out: short vectors have few partial sums, and the
+// step saves a launch.
+template <int TB>
+__global__ void __launch_bounds__(TB) axpy8_f64_kernel(const double* __restrict__ V, int64_t ld, int nv,
+                                                       const double* __restrict__ h, double* __restrict__ z,
+                                                       int64_t n2, double* __restrict__ partial_out, int want_norm,
+                                                       const double* __restrict__ partial_in, int nred,
+                                                       double* __restrict__ h_out) {
+  pdl_wait_then_trigger();
+  __shared__ double hs[256];
+  __shared__ double red[TB / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (nred > 0) {
+    for (int i = wid; i < nv; i += TB / 32) {
+      double s = 0.0;
+      for (int b = lane; b < nred; b += 32) s += partial_in[(int64_t)b * KMAXV + i];
+      s = warp_sum(s);
+      if (lane == 0) {
+        hs[i] = s;
+        if (blockIdx.x == 0) h_out[i] = s;
+      }
+    }
+  } else {
+    for (int i = threadIdx.x; i < nv; i += TB) hs[i] = h[i];
+  }
+  __syncthreads();
+  double acc = 0.0;
+  double2* z2 = reinterpret_cast<double2*>(z);
+  for (int64_t k = (int64_t)blockIdx.x * TB + threadIdx.x; k < n2; k += (int64_t)gridDim.x * TB) {
+    double2 zv = z2[k];
+    int i0 = 0;
+    for (; i0 + 8 <= nv; i0 += 8) {
+      double2 v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = reinterpret_cast<const double2*>(V + (size_t)(i0 + q) * ld)[k];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        zv.x = fma(-v[q].x, hs[i0 + q], zv.x);
+        zv.y = fma(-v[q].y, hs[i0 + q], zv.y);
+      }
+    }
+    for (; i0 < nv; ++i0) {
+      const double2 v = reinterpret_cast<const double2*>(V + (size_t)i0 * ld)[k];
+      zv.x = fma(-v.x, hs[i0], zv.x);
+      zv.y = fma(-v.y, hs[i0], zv.y);
+    }
+    z2[k] = zv;
+    if (want_norm) acc = fma(zv.y, zv.y, fma(zv.x, zv.x, acc));
+  }
+  if (!want_norm) return;
+  const double a = warp_sum(acc);
+  if (lane == 0) red[wid] = a;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int w = 0; w < TB / 32; ++w) s += red[w];
+    partial_out[(int64_t)blockIdx.x * KMAXV] = s;
+  }
+}
+
+// End of a CGS2 step, one CTA: Hc[i] = h1[i] + h2[i], Hc[nv] = |z| from the
+// update's partial sums, *inv = 1 / |z|
+__global__ void cgs_finish64_kernel(const double* __restrict__ partial, int nblk, const double* __restrict__ h1,
+                                    const double* __restrict__ h2, int nv, double* __restrict__ Hc,
+                                    double* __restrict__ inv) {
+  pdl_wait_then_trigger();
+  __shared__ double red[32];
+  for (int i = threadIdx.x; i < nv; i += blockDim.x) Hc[i] = h1[i] + h2[i];
+  double s = 0.0;
+  for (int b = threadIdx.x; b < nblk; b += blockDim.x) s += partial[(int64_t)b * KMAXV];
+  s = warp_sum(s);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (lane == 0) red[wid] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int w = 0; w < (int)(blockDim.x + 31) / 32; ++w) t += red[w];
+    t = sqrt(t);
+    Hc[nv] = t;
+    *inv = 1.0 / t;
+  }
+}
+
+// v = z * (*s), two entries a thread: a product with the reciprocal formed
+// once (a division per entry is ~10 instructions of the FP64 pipe: 15 -> 4 us
+// at 960,000 rows)
+__global__ void scale2_f64_kernel(const double* __restrict__ z, const double* __restrict__ s, double* __restrict__ v,
+                                  int64_t n2) {
+  pdl_wait_then_trigger();
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n2) return;
+  const double f = *s;
+  const double2 a = reinterpret_cast<const double2*>(z)[k];
+  reinterpret_cast<double2*>(v)[k] = make_double2(a.x * f, a.y * f);
 }
 
 // v = z / (*den): FP64 vectors divide (bitwise like the reference's
@@ -742,6 +1000,150 @@ __global__ void __launch_bounds__(1024) vcycle_tail_kernel(TailParams<T> p) {
       __syncthreads();
     }
   }
+}
+
+// The coarse tail of the FP64 V-cycle as a matrix.  Levels l0 .. top are a
+// fixed linear map of the level's right-hand side r and starting error e (the
+// reference restricts the error as well), e_out = T [r; e]; in one CTA its
+// ~9 barrier-separated phases per level took 130 us an application (48,000
+// tetrahedra, 290 rows; 190 us with V(3,3) on 2,048 triangles), ten times the
+// rest of the V-cycle.  T is formed once per operator build, one CTA per unit
+// vector with the level vectors in shared memory (4 n_l doubles per level + n
+// scratch), the same operations as vcycle_tail_kernel; column q of T (n rows
+// of ld entries) is the image of unit vector q of [r; e].
+// FP64-pipe bound (1.2 ms for 1,089 rows and columns, 0.4 ms for 579 x 1,158):
+// 4 lanes per row, few reduction steps, and no division per row (a division
+// for one lane of eight cost more than the row's products: 12 ms at 1,158 x
+// 2,316 before).
+constexpr int kColLanes = 4;
+__device__ __forceinline__ void col_jacobi(const TLevel<double>& L, const double* wd, const double* e_in,
+                                           const double* r, double* e_out, double* rr_out) {
+  const int lane = threadIdx.x % kColLanes, groups = blockDim.x / kColLanes;
+  for (int base = 0; base < L.n; base += groups) {
+    const int i = base + (int)threadIdx.x / kColLanes;
+    double s = 0.0;
+    if (i < L.n) {
+      const int k1 = __ldg(L.rowptr + i + 1);
+      for (int k = __ldg(L.rowptr + i) + lane; k < k1; k += kColLanes)
+        s = fma(__ldg(L.val + k), e_in[__ldg(L.col + k)], s);
+    }
+#pragma unroll
+    for (int o = kColLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, kColLanes);
+    if (i < L.n && lane == 0) {
+      const double rr = r[i] - s;
+      e_out[i] = fma(rr, wd[i], e_in[i]);
+      if (rr_out) rr_out[i] = rr;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(512) tail_columns_kernel(TailParams<double> p, double* __restrict__ T, int ld) {
+  extern __shared__ double col_smem[];
+  __shared__ int off[VMAXLEV];   // level l: e at off[l], e2 at + n, r at + 2 n, w / diag at + 3 n
+  const int l0 = p.l0, top = p.top, n0 = p.lev[l0].n, q = blockIdx.x;
+  double* rr = col_smem;         // n0
+  if (threadIdx.x == 0) {
+    int o = n0;
+    for (int l = l0; l <= top; ++l) {
+      off[l] = o;
+      o += 4 * p.lev[l].n;
+    }
+  }
+  __syncthreads();
+  for (int l = l0; l < top; ++l)
+    for (int i = threadIdx.x; i < p.lev[l].n; i += blockDim.x)
+      col_smem[off[l] + 3 * p.lev[l].n + i] = p.w / p.lev[l].diag[i];
+  for (int i = threadIdx.x; i < n0; i += blockDim.x) {
+    col_smem[off[l0] + i] = i + n0 == q ? 1.0 : 0.0;
+    col_smem[off[l0] + 2 * n0 + i] = i == q ? 1.0 : 0.0;
+  }
+  __syncthreads();
+  const int down = (p.pre + 1) & 1, up = (p.pre + 1 + p.post) & 1;   // which of e / e2 holds the result
+  for (int l = l0; l < top; ++l) {
+    const TLevel<double>& L = p.lev[l];
+    double* e = col_smem + off[l];
+    double *ea = e, *eb = e + L.n;
+    for (int it = 0; it <= p.pre; ++it) {   // the last one also forms the residual
+      col_jacobi(L, e + 3 * L.n, ea, e + 2 * L.n, eb, it == p.pre ? rr : nullptr);
+      __syncthreads();
+      double* t = ea; ea = eb; eb = t;
+    }
+    const int nn = p.lev[l + 1].n;
+    double* en = col_smem + off[l + 1];
+    for (int i = threadIdx.x; i < nn; i += blockDim.x) {
+      const int a = 2 * i, b = 2 * i + 1;
+      en[2 * nn + i] = rr[a] + (b < L.n ? rr[b] : 0.0);
+      en[i] = ea[a] + (b < L.n ? ea[b] : 0.0);
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) col_smem[off[top]] = col_smem[off[top] + 2 * p.lev[top].n] / p.lev[top].val[0];
+  __syncthreads();
+  for (int l = top - 1; l >= l0; --l) {
+    const TLevel<double>& L = p.lev[l];
+    double* e = col_smem + off[l];
+    double *ea = e + (down ? L.n : 0), *eb = e + (down ? 0 : L.n);
+    const double* en = col_smem + off[l + 1] + (l + 1 < top && up ? p.lev[l + 1].n : 0);
+    for (int i = threadIdx.x; i < L.n; i += blockDim.x) ea[i] += en[__ldg(L.up + i)];
+    __syncthreads();
+    for (int it = 0; it < p.post; ++it) {
+      col_jacobi(L, e + 3 * L.n, ea, e + 2 * L.n, eb, nullptr);
+      __syncthreads();
+      double* t = ea; ea = eb; eb = t;
+    }
+  }
+  const double* res = col_smem + off[l0] + (l0 < top && up ? n0 : 0);
+  for (int i = threadIdx.x; i < n0; i += blockDim.x) T[(size_t)i * ld + q] = res[i];
+}
+
+// e = T [r; e0]: one warp per row, [r; e0] staged in shared memory (ncol
+// doubles).  With fine > 0, r and e0 are formed there as the pair sums of the
+// finer level's residual and error (fine rows; lev_restrict_kernel), so the
+// restriction needs no launch; e0 is not read when ncol == n (no finer
+// level: the error starts at zero).  The first entries of the fixed row are
+// read before the programmatic-launch wait.
+__global__ void __launch_bounds__(256) dense_tail64_kernel(const double* __restrict__ T, int ld,
+                                                           const double* __restrict__ r,
+                                                           const double* __restrict__ e0, int fine,
+                                                           double* __restrict__ e, int n, int ncol) {
+  extern __shared__ __align__(16) double tail_v[];
+  constexpr int PRE = 16;
+  const int row = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x & 31;
+  const double2* tr = reinterpret_cast<const double2*>(T + (size_t)(row < n ? row : 0) * ld);
+  const int n2 = ld / 2;   // ld even, entry ncol (if ld > ncol) is zero
+  double2 a[PRE];
+#pragma unroll
+  for (int q = 0; q < PRE; ++q) a[q] = lane + 32 * q < n2 ? tr[lane + 32 * q] : make_double2(0.0, 0.0);
+  pdl_wait_then_trigger();
+  for (int k = threadIdx.x; k < ld; k += 256) {
+    double v = 0.0;
+    if (k < ncol) {
+      const double* src = k < n ? r : e0;
+      const int i = k < n ? k : k - n;
+      if (fine > 0) v = src[2 * i] + (2 * i + 1 < fine ? src[2 * i + 1] : 0.0);
+      else v = src[i];
+    }
+    tail_v[k] = v;
+  }
+  __syncthreads();
+  if (row >= n) return;   // whole warp
+  const double2* v2 = reinterpret_cast<const double2*>(tail_v);
+  double s = 0.0, s1 = 0.0;
+#pragma unroll
+  for (int q = 0; q < PRE; ++q)
+    if (lane + 32 * q < n2) {
+      const double2 v = v2[lane + 32 * q];
+      s = fma(a[q].x, v.x, s);
+      s1 = fma(a[q].y, v.y, s1);
+    }
+#pragma unroll 4
+  for (int k = lane + 32 * PRE; k < n2; k += 32) {
+    const double2 t = tr[k], v = v2[k];
+    s = fma(t.x, v.x, s);
+    s1 = fma(t.y, v.y, s1);
+  }
+  s = warp_sum(s + s1);
+  if (lane == 0) e[row] = s;
 }
 
 }  // namespace dg

@@ -115,48 +115,6 @@ __global__ void f64_to_f32_kernel(const double* __restrict__ a, float* __restric
   if (k < n) b[k] = (float)(a[k] * scale);
 }
 
-// Launch on st, as a programmatic dependent launch when c->use_pdl (the
-// kernel's launch overlaps the tail of the preceding kernel; its
-// pdl_wait_then_trigger() keeps the data order).  Used for the chain of
-// kernels of one inner Arnoldi step.
-template <typename... KArgs, typename... Args>
-int launch_k(dg_ctx* c, void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
-             Args... args) {
-  if (grid == 0) return DG_OK;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = c->use_pdl ? 1 : 0;
-  CK(c, cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
-  bump();
-  return DG_OK;
-}
-
-template <typename... KArgs, typename... Args>
-int launch_k2(dg_ctx* c, void (*kern)(KArgs...), dim3 grid, unsigned block, size_t smem, cudaStream_t st,
-              Args... args) {
-  if (grid.x == 0 || grid.y == 0) return DG_OK;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = c->use_pdl ? 1 : 0;
-  CK(c, cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
-  bump();
-  return DG_OK;
-}
-
 // e = Ainv r for a small dense level matrix: one warp per row.  The row of
 // the fixed inverse is read into registers (float4, up to 20 per lane, i.e.
 // n <= 2560 without a second pass) before the programmatic-launch wait, so
@@ -235,65 +193,6 @@ __global__ void dense_matvec_kernel(const float* __restrict__ Ainv, const float*
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   if (lane == 0) e[row] = s;
-}
-
-// SFC-level Jacobi sweep (lev_jacobi_kernel, FP32, LPR lanes per row) whose
-// input iterate is formed on the fly from the neighbouring level, so that
-// the transfer between levels needs no launch of its own:
-//   MODE 1 (restriction in): e_in[j] = ea[2j] + ea[2j+1] and
-//     r[i] = eb[2i] + eb[2i+1] (zero pad at n_src; lev_restrict_kernel),
-//     r is stored for the level's later sweeps;
-//   MODE 2 (prolongation in): e_in[j] = ea[j] + eb[up[j]]
-//     (lev_prolong_kernel), r read as given.
-// Then rr = r - A e_in, e_out = e_in + rr / diag * w, rr_out = rr (if set):
-// the same operations as the transfer launch followed by the sweep.
-template <int MODE>
-__global__ void lev_jacobi_x_kernel(const int* __restrict__ rowptr, const int* __restrict__ col,
-                                    const float* __restrict__ val, const float* __restrict__ diag,
-                                    const float* __restrict__ ea, const float* __restrict__ eb,
-                                    const int* __restrict__ up, int n_src, float* __restrict__ r,
-                                    float* __restrict__ e_out, float* __restrict__ rr_out, int n, float w) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = t / LPR, lane = t % LPR;
-  constexpr int PRE = 4;
-  int k0 = 0, k1 = 0;
-  int cpre[PRE];
-  float vpre[PRE];
-  if (i < n) {
-    k0 = rowptr[i] + lane;
-    k1 = rowptr[i + 1];
-  }
-#pragma unroll
-  for (int q = 0; q < PRE; ++q) {
-    const int k = k0 + q * LPR;
-    cpre[q] = k < k1 ? col[k] : 0;
-    vpre[q] = k < k1 ? val[k] : 0.0f;
-  }
-  pdl_wait_then_trigger();
-  auto ein = [&](int j) -> float {
-    if (MODE == 1) return ea[2 * j] + (2 * j + 1 < n_src ? ea[2 * j + 1] : 0.0f);
-    return ea[j] + eb[up[j]];
-  };
-  float s = 0.0f;
-  if (i < n) {
-#pragma unroll
-    for (int q = 0; q < PRE; ++q)
-      if (k0 + q * LPR < k1) s = __fmaf_rn(vpre[q], ein(cpre[q]), s);
-    for (int k = k0 + PRE * LPR; k < k1; k += LPR) s = __fmaf_rn(val[k], ein(col[k]), s);
-  }
-#pragma unroll
-  for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, LPR);
-  if (i >= n || lane != 0) return;
-  float ri;
-  if (MODE == 1) {
-    ri = eb[2 * i] + (2 * i + 1 < n_src ? eb[2 * i + 1] : 0.0f);
-    r[i] = ri;
-  } else {
-    ri = r[i];
-  }
-  const float rr = ri - s;
-  e_out[i] = __fmaf_rn(rr / diag[i], w, ein(i));
-  if (rr_out) rr_out[i] = rr;
 }
 
 // ---------------------------------------------------------------------------
@@ -1366,13 +1265,9 @@ int launch_residual32(dg_ctx* c, const float* x, const float* b, float* r, float
       return launch_tma<float, 4, 2, 2, true>(c, A, M.W, x, b, r, x_out, flags, M.r1, st, M.sf, ws);
     return launch_tma<float, 4, 2, 3, false>(c, A, M.W, x, b, r, x_out, flags, M.r1, st, M.sf);
   }
-  unsigned g = nblk(c->B, E::EPB);
-  if (g)
-    residual_kernel<E::N, E::F, E::EPB, float, float, float><<<g, E::EPB * E::N, 0, st>>>(
-        M.blk, M.W, c->d_nbe, x, b, r, x_out, c->B, flags, c->T.P, M.r1, ws);
-  bump();
-  CKL(c);
-  return DG_OK;
+  return launch_k(c, residual_kernel<E::N, E::F, E::EPB, float, float, float>, nblk(c->B, E::EPB), E::EPB * E::N, 0,
+                  st, (const float*)M.blk, (const float*)M.W, (const int*)c->d_nbe, x, b, r, x_out, (int64_t)c->B,
+                  flags, (const double*)c->T.P, M.r1, ws);
 }
 
 int residual32(dg_ctx* c, const float* x, const float* b, float* r, float* x_out, int flags, cudaStream_t st,

@@ -158,7 +158,14 @@ struct dg_ctx {
   // SFC V-cycle as one thread-block-cluster kernel (0 = per-level launches)
   int vc_cluster = 0;
   // levels with at most this many rows run in the one-CTA tail kernel
-  int tail_max64 = 320, tail_max32 = 800;
+  // (FP32), or are replaced by their matrix (FP64, ensure_tail64): at most
+  // tail_max64 rows below other levels (a matrix n x 2 n, its build ~ n^2;
+  // 48,000 tetrahedra with 290 / 579 / 1,158 / 2,316 rows: 161.0 / 159.7 /
+  // 159.4 / 160.8 ms a solve), twice that for a whole V-cycle (n x n; 2,048
+  // triangles with 273 / 545 / 1,089 rows: 7.9 / 6.8 / 5.7 ms)
+  int tail_max64 = 640, tail_max32 = 800;
+  int tail_l0 = 0, tail_ld = 0, t64_version = -1;
+  double* d_tail = nullptr;
   // mixed preconditioner: exact (dense inverse) solve on the first SFC level
   // with at most this many rows (0 = keep the V-cycle to the one-node level)
   int dense_max32 = 2400;
@@ -361,6 +368,49 @@ int upload_vec(dg_ctx* c, T** p, const std::vector<T>& v) {
 
 inline cudaStream_t S(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 inline unsigned nblk(int64_t n, int tb) { return (unsigned)((n + tb - 1) / tb); }
+
+// Launch on st, as a programmatic dependent launch when c->use_pdl (the
+// kernel's launch overlaps the tail of the preceding kernel; its
+// pdl_wait_then_trigger() keeps the data order).  Used for the chains of
+// kernels of an Arnoldi step; every kernel launched with it starts with that
+// wait.
+template <typename... KArgs, typename... Args>
+int launch_k(dg_ctx* c, void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+             Args... args) {
+  if (grid == 0) return DG_OK;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = c->use_pdl ? 1 : 0;
+  CK(c, cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
+  bump();
+  return DG_OK;
+}
+
+template <typename... KArgs, typename... Args>
+int launch_k2(dg_ctx* c, void (*kern)(KArgs...), dim3 grid, unsigned block, size_t smem, cudaStream_t st,
+              Args... args) {
+  if (grid.x == 0 || grid.y == 0) return DG_OK;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = c->use_pdl ? 1 : 0;
+  CK(c, cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
+  bump();
+  return DG_OK;
+}
 
 // ---------------------------------------------------------------------------
 // template dispatch on the element type
@@ -581,12 +631,9 @@ int launch_residual(dg_ctx* c, const double* x, const double* b, double* r, doub
     int rc;
     if ((rc = ensure_w64_t<D>(c, st))) return rc;
   }
-  unsigned g = nblk(c->B, E::EPB);
-  if (g) residual_kernel<E::N, E::F, E::EPB><<<g, E::EPB * E::N, 0, st>>>(
-      c->d_blk, c->d_W, c->d_nbe, x, b, r, x_out, c->B, flags, c->T.P, r1);
-  bump();
-  CKL(c);
-  return DG_OK;
+  return launch_k(c, residual_kernel<E::N, E::F, E::EPB>, nblk(c->B, E::EPB), E::EPB * E::N, 0, st,
+                  (const double*)c->d_blk, (const double*)c->d_W, (const int*)c->d_nbe, x, b, r, x_out, (int64_t)c->B,
+                  flags, (const double*)c->T.P, r1, (const float*)nullptr);
 }
 
 // flags RF_*; with RF_RESTRICT, r1 (nele, ncorner) receives the P3->P1
@@ -600,11 +647,9 @@ int residual(dg_ctx* c, const double* x, const double* b, double* r, double* x_o
 // vertex gather of the element restrictions r1 (curve order when sfc_order)
 template <typename T>
 int gather_cg(dg_ctx* c, const T* r1, T* out, bool sfc_order, cudaStream_t st) {
-  gather_cg_kernel<T><<<nblk(c->ncg, 128), 128, 0, st>>>(r1, c->d_gptr, c->d_gent, c->d_wdg,
-                                                         sfc_order ? c->d_pos : nullptr, out, (int)c->ncg);
-  bump();
-  CKL(c);
-  return DG_OK;
+  return launch_k(c, gather_cg_kernel<T>, nblk(c->ncg, 128), 128, 0, st, r1, (const int*)c->d_gptr,
+                  (const int*)c->d_gent, (const double*)c->d_wdg, (const int*)(sfc_order ? c->d_pos : nullptr), out,
+                  (int)c->ncg);
 }
 
 template <int D>
@@ -636,6 +681,15 @@ int launch_prolong(dg_ctx* c, double* x, const double* ecg, bool sfc_order, int 
 int prolong_cg(dg_ctx* c, double* x, const double* ecg, bool sfc_order, int color, bool add, cudaStream_t st) {
   return c->D == 3 ? launch_prolong<3>(c, x, ecg, sfc_order, color, add, st)
                    : launch_prolong<2>(c, x, ecg, sfc_order, color, add, st);
+}
+
+// coarse correction (curve order) added to x
+template <int D>
+int launch_prolong_add(dg_ctx* c, double* x, const double* e_sfc, cudaStream_t st) {
+  using E = Elem<D>;
+  return launch_k(c, prolong_add_kernel<E::N, E::NC, E::EPB>, nblk(c->B, E::EPB), E::EPB * E::N, 0, st, x, e_sfc,
+                  (const int*)c->d_pos, (const int*)c->d_p1cg, (const double*)c->d_wdg, (const double*)c->T.P,
+                  (int64_t)c->B);
 }
 
 // First SFC level handled by the one-CTA tail kernel (<= top; == top means
@@ -709,57 +763,98 @@ int vcycle_cluster(dg_ctx* c, const double* r_sfc, cudaStream_t st) {
   return DG_OK;
 }
 
-// One SFC V-cycle; r_sfc is level-0 input, result left in lev[0].e
+// The matrix of the V-cycle's coarse tail (tail_columns_kernel) for the
+// current operator build, formed on first use: only the FP64 preconditioner
+// reads it.  Entry points that reach vcycle() call it first, outside any
+// capture of their own.
+int ensure_tail64(dg_ctx* c, cudaStream_t st) {
+  if (c->vc_cluster > 0 || c->t64_version == c->build_version) return DG_OK;
+  const int nl = (int)c->lev.size(), l0 = c->tail_l0;
+  if (c->lev.back().n != 1 || nl > VMAXLEV)
+    return fail(c, DG_ERR_STATE, "coarsest SFC level must hold one node");
+  TailParams<double> tp;
+  tp.l0 = l0;
+  tp.top = nl - 1;
+  tp.pre = c->cfg.pre_smooth_its;
+  tp.post = c->cfg.post_smooth_its;
+  tp.w = c->cfg.jac_wei;
+  size_t words = c->lev[l0].n;
+  for (int l = l0; l < nl; ++l) {
+    const DevLevel& L = c->lev[l];
+    tp.lev[l] = TLevel<double>{L.rowptr, L.col, L.val, L.diag, L.up, nullptr, nullptr, nullptr, nullptr, L.n};
+    words += 4 * (size_t)L.n;
+  }
+  const int n = c->lev[l0].n, ncol = l0 > 0 ? 2 * n : n;
+  CK(c, cudaFuncSetAttribute(tail_columns_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(words * sizeof(double))));
+  if (c->tail_ld > ncol) CK(c, cudaMemsetAsync(c->d_tail, 0, sizeof(double) * (size_t)n * c->tail_ld, st));
+  tail_columns_kernel<<<ncol, 512, words * sizeof(double), st>>>(tp, c->d_tail, c->tail_ld);
+  bump();
+  CKL(c);
+  // not a kernel: the next one starts only when the matrix is in memory, also
+  // if it reads it before its programmatic-launch wait
+  CK(c, cudaMemsetAsync(c->d_part, 0, sizeof(double), st));
+  c->t64_version = c->build_version;
+  return DG_OK;
+}
+
+// One SFC V-cycle; r_sfc is level-0 input, result left in lev[0].e.  Sweeps
+// per level with the transfers between levels formed on the fly, then the
+// coarse tail as one matrix product (ensure_tail64).
 int vcycle(dg_ctx* c, const double* r_sfc, cudaStream_t st) {
   if (c->vc_cluster > 0) {
     if (c->lev.back().n != 1) return fail(c, DG_ERR_STATE, "coarsest SFC level must hold one node");
     return vcycle_cluster(c, r_sfc, st);
   }
-  const int nl = (int)c->lev.size();
-  const int top = nl - 1;
   const double w = c->cfg.jac_wei;
-  const int TB = 128;
-  const int l0 = tail_start(c, c->tail_max64);
-  CK(c, cudaMemcpyAsync(c->lev[0].r, r_sfc, sizeof(double) * c->lev[0].n, cudaMemcpyDeviceToDevice, st));
-  CK(c, cudaMemsetAsync(c->lev[0].e, 0, sizeof(double) * c->lev[0].n, st));
-  for (int l = 0; l < std::min(l0, top); ++l) {
+  const int TB = 128, l0 = c->tail_l0, npre = c->cfg.pre_smooth_its, npost = c->cfg.post_smooth_its;
+  int rc;
+  auto rhs_of = [&](int l) -> const double* { return l == 0 ? r_sfc : c->lev[l].r; };
+  for (int l = 0; l < l0; ++l) {
     DevLevel& L = c->lev[l];
-    for (int it = 0; it < c->cfg.pre_smooth_its; ++it) {
-      lev_jacobi_kernel<double><<<nblk((int64_t)L.n * LPR, TB), TB, 0, st>>>(L.rowptr, L.col, L.val, L.diag, L.e, L.r,
-                                                                      L.e2, nullptr, L.n, w); bump();
+    const unsigned g = nblk((int64_t)L.n * LPR, TB);
+    for (int it = 0; it <= npre; ++it) {   // the last sweep also forms the residual (reference quirk)
+      double* keep = it == npre ? L.rr : nullptr;
+      if (it == 0 && l > 0) {
+        const DevLevel& P = c->lev[l - 1];
+        rc = launch_k(c, lev_jacobi_x_kernel<1, double>, g, TB, 0, st, (const int*)L.rowptr, (const int*)L.col,
+                      (const double*)L.val, (const double*)L.diag, (const double*)P.e, (const double*)P.rr,
+                      (const int*)nullptr, P.n, L.r, L.e2, keep, L.n, w);
+      } else {
+        rc = launch_k(c, lev_jacobi_kernel<double>, g, TB, 0, st, (const int*)L.rowptr, (const int*)L.col,
+                      (const double*)L.val, (const double*)L.diag, (const double*)(it == 0 ? nullptr : L.e), rhs_of(l),
+                      L.e2, keep, L.n, w);
+      }
+      if (rc) return rc;
       std::swap(L.e, L.e2);
     }
-    // the residual-forming call also updates e in place (reference quirk)
-    lev_jacobi_kernel<double><<<nblk((int64_t)L.n * LPR, TB), TB, 0, st>>>(L.rowptr, L.col, L.val, L.diag, L.e, L.r,
-                                                                    L.e2, L.rr, L.n, w); bump();
-    std::swap(L.e, L.e2);
-    DevLevel& Nx = c->lev[l + 1];
-    lev_restrict_kernel<double><<<nblk(Nx.n, TB), TB, 0, st>>>(L.rr, L.e, Nx.r, Nx.e, L.n, Nx.n); bump();
   }
-  if (c->lev[top].n != 1) return fail(c, DG_ERR_STATE, "coarsest SFC level must hold one node");
-  if (l0 < top) {
-    TailParams<double> tp;
-    tp.l0 = l0;
-    tp.top = top;
-    tp.pre = c->cfg.pre_smooth_its;
-    tp.post = c->cfg.post_smooth_its;
-    tp.w = w;
-    for (int l = 0; l < nl; ++l) {
-      const DevLevel& L = c->lev[l];
-      tp.lev[l] = TLevel<double>{L.rowptr, L.col, L.val, L.diag, L.up, L.e, L.e2, L.r, L.rr, L.n};
-    }
-    vcycle_tail_kernel<double><<<1, 1024, 0, st>>>(tp);
-    bump();
-  } else {
-    DevLevel& L = c->lev[top];
-    lev_coarse_kernel<double><<<1, 32, 0, st>>>(L.val, L.r, L.e); bump();
+  {
+    DevLevel& L = c->lev[l0];
+    const int ncol = l0 > 0 ? 2 * L.n : L.n;
+    const double* fr = l0 > 0 ? c->lev[l0 - 1].rr : r_sfc;
+    const double* fe = l0 > 0 ? c->lev[l0 - 1].e : nullptr;
+    if ((rc = launch_k(c, dense_tail64_kernel, nblk(L.n, 8), 256, sizeof(double) * c->tail_ld, st,
+                       (const double*)c->d_tail, c->tail_ld, fr, fe, l0 > 0 ? c->lev[l0 - 1].n : 0, L.e, L.n, ncol)))
+      return rc;
   }
-  for (int l = std::min(l0, top) - 1; l >= 0; --l) {
+  for (int l = l0 - 1; l >= 0; --l) {
     DevLevel& L = c->lev[l];
-    lev_prolong_kernel<double><<<nblk(L.n, TB), TB, 0, st>>>(L.e, c->lev[l + 1].e, L.up, L.n); bump();
-    for (int it = 0; it < c->cfg.post_smooth_its; ++it) {
-      lev_jacobi_kernel<double><<<nblk((int64_t)L.n * LPR, TB), TB, 0, st>>>(L.rowptr, L.col, L.val, L.diag, L.e, L.r,
-                                                                      L.e2, nullptr, L.n, w); bump();
+    const double* enext = c->lev[l + 1].e;
+    const unsigned g = nblk((int64_t)L.n * LPR, TB);
+    if (npost == 0 && (rc = launch_k(c, lev_prolong_kernel<double>, nblk(L.n, TB), TB, 0, st, L.e, enext,
+                                     (const int*)L.up, L.n)))
+      return rc;
+    for (int it = 0; it < npost; ++it) {
+      if (it == 0)
+        rc = launch_k(c, lev_jacobi_x_kernel<2, double>, g, TB, 0, st, (const int*)L.rowptr, (const int*)L.col,
+                      (const double*)L.val, (const double*)L.diag, (const double*)L.e, enext, (const int*)L.up, 0,
+                      const_cast<double*>(rhs_of(l)), L.e2, (double*)nullptr, L.n, w);
+      else
+        rc = launch_k(c, lev_jacobi_kernel<double>, g, TB, 0, st, (const int*)L.rowptr, (const int*)L.col,
+                      (const double*)L.val, (const double*)L.diag, (const double*)L.e, rhs_of(l), L.e2,
+                      (double*)nullptr, L.n, w);
+      if (rc) return rc;
       std::swap(L.e, L.e2);
     }
   }
@@ -789,7 +884,8 @@ int precond(dg_ctx* c, const double* r, double* z, cudaStream_t st) {
   if ((rc = residual(c, cur, r, nullptr, nullptr, RF_RESTRICT, st, c->d_r1))) return rc;
   if ((rc = gather_cg<double>(c, c->d_r1, c->d_cg1, true, st))) return rc;
   if ((rc = vcycle(c, c->d_cg1, st))) return rc;
-  if ((rc = prolong_cg(c, cur, c->lev[0].e, true, 0, true, st))) return rc;
+  if ((rc = c->D == 3 ? launch_prolong_add<3>(c, cur, c->lev[0].e, st) : launch_prolong_add<2>(c, cur, c->lev[0].e, st)))
+    return rc;
   // post-smoothing (the reference repeats pre_smooth_its times, :2021)
   for (int it = 0; it < nsm; ++it) {
     double* out = (it == nsm - 1) ? z : other;
@@ -824,11 +920,6 @@ int mdot_t(dg_ctx* c, const VT* V, int nv, const VT* z, double* h, cudaStream_t 
   }
   CKL(c);
   return DG_OK;
-}
-
-int mdot(dg_ctx* c, const double* V, int nv, const double* z, double* h, int accumulate, cudaStream_t st) {
-  (void)accumulate;
-  return mdot_t<double>(c, V, nv, z, h, st);
 }
 
 // Norm of z into *out (device)
@@ -872,7 +963,40 @@ int cgs2_t(dg_ctx* c, VT* Vbase, double* Hbase, int j, VT* z, int m, cudaStream_
   return DG_OK;
 }
 
-int cgs2(dg_ctx* c, int j, double* z, int m, cudaStream_t st) { return cgs2_t<double>(c, c->d_V, c->d_H, j, z, m, st); }
+// ... of the FP64 GMRES: 6 launches for short vectors, 8 for long ones (the
+// partial sums of up to kGsFuse blocks are added up by the update itself)
+constexpr int kGsFuse = 64;
+int cgs2(dg_ctx* c, int j, double* z, int m, cudaStream_t st) {
+  const int nv = j + 1;
+  const int64_t n2 = c->nonods / 2;   // nloc is even
+  double* Hc = c->d_H + (size_t)j * (m + 1);
+  double* inv = c->d_scal + 1;
+  const int nb = (int)std::max<int64_t>(1, std::min<int64_t>(c->nred, (n2 + 2 * RED_TB - 1) / (2 * RED_TB)));
+  const bool fuse = nb <= kGsFuse && nv <= KMAXV;
+  int rc;
+  for (int pass = 0; pass < 2; ++pass) {
+    double* h = pass == 0 ? c->d_h1 : c->d_h2;
+    double* part = c->d_part + (size_t)pass * c->nred * KMAXV;   // the update writes the other half
+    double* part_n = c->d_part + (size_t)(1 - pass) * c->nred * KMAXV;
+    for (int off = 0; off < nv; off += KMAXV) {
+      const int cnt = std::min(KMAXV, nv - off);
+      if ((rc = launch_k2(c, mdot8_f64_kernel<RED_TB>, dim3(nb, (cnt + 7) / 8), RED_TB, 0, st,
+                          (const double*)(c->d_V + (size_t)off * c->nonods), (int64_t)c->nonods, cnt, (const double*)z,
+                          n2, part)))
+        return rc;
+      if (!fuse && (rc = launch_k(c, reduce_partial_kernel, cnt, 128, 0, st, (const double*)part, nb, cnt, h + off, 0, 0)))
+        return rc;
+    }
+    if ((rc = launch_k(c, axpy8_f64_kernel<RED_TB>, nb, RED_TB, 0, st, (const double*)c->d_V, (int64_t)c->nonods, nv,
+                       (const double*)h, z, n2, part_n, pass, (const double*)part, fuse ? nb : 0, h)))
+      return rc;
+  }
+  if ((rc = launch_k(c, cgs_finish64_kernel, 1, 128, 0, st, (const double*)c->d_part, nb, (const double*)c->d_h1,
+                     (const double*)c->d_h2, nv, Hc, inv)))
+    return rc;
+  return launch_k(c, scale2_f64_kernel, nblk(n2, 256), 256, 0, st, (const double*)z, (const double*)inv,
+                  c->d_V + (size_t)nv * c->nonods, n2);
+}
 
 // Modified Gram-Schmidt step in the reference's order
 // (z06/volume_mf_diff.py:1814-1819): for i = 0..j, H[i][j] = z . V[i] then
@@ -1053,7 +1177,7 @@ int dg_create(const dg_mesh_desc* m, const dg_config* cfg, dg_ctx** out) {
   {
     const char* t64 = std::getenv("DG_TAIL_MAX64");
     const char* t32 = std::getenv("DG_TAIL_MAX32");
-    if (t64 && t64[0]) c->tail_max64 = std::atoi(t64);
+    if (t64 && t64[0]) c->tail_max64 = std::min(std::max(std::atoi(t64), 1), 1280);
     if (t32 && t32[0]) c->tail_max32 = std::atoi(t32);
     const char* dm = std::getenv("DG_DENSE_MAX32");
     if (dm && dm[0]) c->dense_max32 = std::atoi(dm);
@@ -1358,7 +1482,7 @@ int dg_create(const dg_mesh_desc* m, const dg_config* cfg, dg_ctx** out) {
   for (double** t : {&c->d_cg1, &c->d_cg2})
     if ((rc = dalloc(c.get(), t, (size_t)c->ncg))) return rc;
   if ((rc = dalloc(c.get(), &c->d_r1, (size_t)c->B * c->NC))) return rc;
-  if ((rc = dalloc(c.get(), &c->d_part, (size_t)c->nred * KMAXV))) return rc;
+  if ((rc = dalloc(c.get(), &c->d_part, (size_t)2 * c->nred * KMAXV))) return rc;
   for (double** t : {&c->d_h1, &c->d_h2, &c->d_y, &c->d_scal})
     if ((rc = dalloc(c.get(), t, 256))) return rc;
   *out = c.release();
@@ -1533,6 +1657,12 @@ int dg_build_operator(dg_ctx* c, void* stream) {
     }
   }
   choose_vcycle_cluster(c);
+  c->tail_l0 = c->lev[0].n <= 2 * c->tail_max64 ? 0 : tail_start(c, c->tail_max64);
+  if (!c->d_tail) {
+    const int nt = c->lev[c->tail_l0].n;
+    c->tail_ld = ((c->tail_l0 > 0 ? 2 * nt : nt) + 1) & ~1;
+    if ((rc = dalloc(c, &c->d_tail, (size_t)nt * c->tail_ld))) return rc;
+  }
   // rows sorted by column (torch CSR from COO) and the diagonal taken, level
   // by level on parallel host threads; then the uploads in level order
   // the fine entries in the order the level sums visit them
@@ -1634,7 +1764,6 @@ int dg_get_bdiag(dg_ctx* c, double* bdiag, double* diag, void* stream) {
   if (!c->built) return fail(c, DG_ERR_STATE, "dg_get_bdiag: operator not built");
   cudaStream_t st = S(stream);
   CK(c, cudaSetDevice(c->dev));
-  const int N = c->N, F = c->F;
   if (c->B > 0) {
     if (c->D == 3)
       copy_bdiag_kernel<20, 4><<<(unsigned)c->B, 128, 0, st>>>(c->d_blk, bdiag, diag);
@@ -1713,9 +1842,10 @@ int dg_precond(dg_ctx* c, const double* r, double* z, void* stream) {
   if (!c->built) return fail(c, DG_ERR_STATE, "dg_precond: operator not built");
   cudaStream_t st = S(stream);
   CK(c, cudaSetDevice(c->dev));
+  int rc;
+  if ((rc = ensure_tail64(c, st))) return rc;
   if (z == r) {
-    int rc = precond(c, r, c->d_t1, st);
-    if (rc) return rc;
+    if ((rc = precond(c, r, c->d_t1, st))) return rc;
     CK(c, cudaMemcpyAsync(z, c->d_t1, sizeof(double) * c->nonods, cudaMemcpyDeviceToDevice, st));
     return DG_OK;
   }
@@ -1727,8 +1857,8 @@ int dg_mg_vcycle(dg_ctx* c, const double* r_sfc, double* e_sfc, void* stream) {
   if (!c->built) return fail(c, DG_ERR_STATE, "dg_mg_vcycle: operator not built");
   cudaStream_t st = S(stream);
   CK(c, cudaSetDevice(c->dev));
-  int rc = vcycle(c, r_sfc, st);
-  if (rc) return rc;
+  int rc;
+  if ((rc = ensure_tail64(c, st)) || (rc = vcycle(c, r_sfc, st))) return rc;
   CK(c, cudaMemcpyAsync(e_sfc, c->lev[0].e, sizeof(double) * c->ncg, cudaMemcpyDeviceToDevice, st));
   return DG_OK;
 }
@@ -1757,7 +1887,7 @@ int dg_gmres(dg_ctx* c, double* x, const double* b, double tol, int32_t m, int32
   cudaStream_t st = S(stream);
   CK(c, cudaSetDevice(c->dev));
   int rc;
-  if ((rc = ensure_krylov(c, m))) return rc;
+  if ((rc = ensure_krylov(c, m)) || (rc = ensure_tail64(c, st))) return rc;
   double* r = c->d_t1;
   double* w = c->d_t2;
   int its = 0;
