@@ -833,14 +833,17 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool full
                : "memory");
 }
 
+// NQ = quads of right-hand sides that are computed (16, or 8 for 32 columns)
+template <int NQ>
 __global__ void __launch_bounds__(128) bdense2_kernel(const float* __restrict__ Ainv, const float* __restrict__ R,
                                                       float* __restrict__ E, int n) {
+  constexpr int RPT = kDnRows * NQ / 128;             // rows per thread: 2 or 1
   extern __shared__ __align__(16) float dn_smem[];
   float* As = dn_smem;                                // [2][kDnRows][kDnK]
   float* Rs = dn_smem + 2 * kDnRows * kDnK;           // [2][kDnK][kNR]
   const int row0 = blockIdx.x * kDnRows;
   const int tid = threadIdx.x;
-  const int ty = tid / 16, tx = tid % 16;             // rows 2 ty, 2 ty + 1; RHS 4 tx .. 4 tx + 3
+  const int ty = tid / NQ, tx = tid % NQ;             // rows RPT ty ..; RHS 4 tx .. 4 tx + 3
   const bool vec = (n & 3) == 0;                      // 16-byte aligned rows of Ainv
   auto stage = [&](int buf, int k0) {
     float* as = As + buf * kDnRows * kDnK;
@@ -856,8 +859,8 @@ __global__ void __launch_bounds__(128) bdense2_kernel(const float* __restrict__ 
           as[r * kDnK + 4 * k4 + u] = (row < n && k + u < n) ? Ainv[(int64_t)row * n + k + u] : 0.0f;
       }
     }
-    for (int i = tid; i < kDnK * (kNR / 4); i += 128) {
-      const int k = i / (kNR / 4), q4 = i % (kNR / 4);
+    for (int i = tid; i < kDnK * NQ; i += 128) {
+      const int k = i / NQ, q4 = i % NQ;
       const bool ok = k0 + k < n;
       cp_async16(rs + k * kNR + 4 * q4, R + (ok ? (int64_t)(k0 + k) * kNR + 4 * q4 : 0), ok);
     }
@@ -879,22 +882,24 @@ __global__ void __launch_bounds__(128) bdense2_kernel(const float* __restrict__ 
     const float* rs = Rs + buf * kDnK * kNR;
     const int kmax = min(kDnK, n - it * kDnK);
     for (int k = 0; k < kmax; ++k) {
-      const float a0 = as[(2 * ty) * kDnK + k], a1 = as[(2 * ty + 1) * kDnK + k];
+      const float a0 = as[(RPT * ty) * kDnK + k], a1 = RPT > 1 ? as[(RPT * ty + 1) * kDnK + k] : 0.0f;
       const float4 rv = reinterpret_cast<const float4*>(rs + k * kNR)[tx];
       acc0.x = fmaf(a0, rv.x, acc0.x);
       acc0.y = fmaf(a0, rv.y, acc0.y);
       acc0.z = fmaf(a0, rv.z, acc0.z);
       acc0.w = fmaf(a0, rv.w, acc0.w);
-      acc1.x = fmaf(a1, rv.x, acc1.x);
-      acc1.y = fmaf(a1, rv.y, acc1.y);
-      acc1.z = fmaf(a1, rv.z, acc1.z);
-      acc1.w = fmaf(a1, rv.w, acc1.w);
+      if (RPT > 1) {
+        acc1.x = fmaf(a1, rv.x, acc1.x);
+        acc1.y = fmaf(a1, rv.y, acc1.y);
+        acc1.z = fmaf(a1, rv.z, acc1.z);
+        acc1.w = fmaf(a1, rv.w, acc1.w);
+      }
     }
     __syncthreads();   // the buffer is refilled by the next stage call
   }
-  const int r0 = row0 + 2 * ty, r1 = r0 + 1;
+  const int r0 = row0 + RPT * ty, r1 = r0 + 1;
   if (r0 < n) reinterpret_cast<float4*>(E + (int64_t)r0 * kNR)[tx] = acc0;
-  if (r1 < n) reinterpret_cast<float4*>(E + (int64_t)r1 * kNR)[tx] = acc1;
+  if (RPT > 1 && r1 < n) reinterpret_cast<float4*>(E + (int64_t)r1 * kNR)[tx] = acc1;
 }
 
 // ---------------------------------------------------------------------------
@@ -957,18 +962,21 @@ __global__ void __launch_bounds__(256) bmdot_kernel(const float* __restrict__ V,
 // quarter / an eighth of the SM's warps).  A thread handles 4 RHS of one row
 // per iteration and at most 8 basis vectors at a time (~64 registers), 256
 // threads per block and 4 blocks per SM, so a block row streams with half
-// the SM's warps, each with 8 16-byte loads in flight.
+// the SM's warps, each with 8 16-byte loads in flight.  NQ = quads of
+// right-hand sides that are computed (16, or 8 for 32 columns).
+template <int NQ>
 __global__ void __launch_bounds__(256, 4) bmdot2_kernel(const float* __restrict__ V, int64_t ld, int nv,
                                                        const float* __restrict__ z, int64_t n,
                                                        double* __restrict__ partial) {
-  __shared__ float4 red[16][8][kNR / 4];
-  const int q4 = threadIdx.x % 16, lane = threadIdx.x / 16;
+  constexpr int RL = 256 / NQ;   // rows in flight
+  __shared__ float4 red[RL][8][NQ];
+  const int q4 = threadIdx.x % NQ, lane = threadIdx.x / NQ;
   const int j0 = blockIdx.y * 8;
   const int cnt = min(8, nv - j0);
   float4 acc[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int64_t row = (int64_t)blockIdx.x * 16 + lane; row < n; row += (int64_t)gridDim.x * 16) {
+  for (int64_t row = (int64_t)blockIdx.x * RL + lane; row < n; row += (int64_t)gridDim.x * RL) {
     const float4 zv = reinterpret_cast<const float4*>(z + row * kNR)[q4];
     float4 v[8];
 #pragma unroll
@@ -986,25 +994,27 @@ __global__ void __launch_bounds__(256, 4) bmdot2_kernel(const float* __restrict_
 #pragma unroll
   for (int j = 0; j < 8; ++j) red[lane][j][q4] = acc[j];
   __syncthreads();
-  for (int o = threadIdx.x; o < cnt * kNR; o += 256) {
-    const int j = o / kNR, q = o % kNR;
+  for (int o = threadIdx.x; o < cnt * NQ * 4; o += 256) {
+    const int j = o / (NQ * 4), q = o % (NQ * 4);
     double sum = 0.0;
-    for (int l = 0; l < 16; ++l) sum += (double)reinterpret_cast<const float*>(&red[l][j][0])[q];
+    for (int l = 0; l < RL; ++l) sum += (double)reinterpret_cast<const float*>(&red[l][j][0])[q];
     partial[((int64_t)blockIdx.x * 32 + j0 + j) * kNR + q] = sum;
   }
 }
 
+template <int NQ>
 __global__ void __launch_bounds__(256, 4) baxpy2_kernel(const float* __restrict__ V, int64_t ld, int nv,
                                                        const double* __restrict__ h, float* __restrict__ z,
                                                        int64_t n, double* __restrict__ partial) {
+  constexpr int RL = 256 / NQ;
   __shared__ float4 hs[32][kNR / 4];
-  __shared__ float4 red[16][kNR / 4];
-  const int q4 = threadIdx.x % 16, lane = threadIdx.x / 16;
+  __shared__ float4 red[RL][NQ];
+  const int q4 = threadIdx.x % NQ, lane = threadIdx.x / NQ;
   for (int o = threadIdx.x; o < 32 * kNR; o += 256)
     reinterpret_cast<float*>(&hs[0][0])[o] = o < nv * kNR ? (float)h[o] : 0.0f;
   __syncthreads();
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int64_t row = (int64_t)blockIdx.x * 16 + lane; row < n; row += (int64_t)gridDim.x * 16) {
+  for (int64_t row = (int64_t)blockIdx.x * RL + lane; row < n; row += (int64_t)gridDim.x * RL) {
     float4* zp = reinterpret_cast<float4*>(z + row * kNR) + q4;
     float4 zv = *zp;
     for (int i0 = 0; i0 < nv; i0 += 8) {
@@ -1030,9 +1040,9 @@ __global__ void __launch_bounds__(256, 4) baxpy2_kernel(const float* __restrict_
   }
   red[lane][q4] = acc;
   __syncthreads();
-  if (threadIdx.x < kNR) {
+  if (threadIdx.x < NQ * 4) {
     double sum = 0.0;
-    for (int l = 0; l < 16; ++l) sum += (double)reinterpret_cast<const float*>(&red[l][0])[threadIdx.x];
+    for (int l = 0; l < RL; ++l) sum += (double)reinterpret_cast<const float*>(&red[l][0])[threadIdx.x];
     partial[(int64_t)blockIdx.x * kNR + threadIdx.x] = sum;
   }
 }
@@ -1168,34 +1178,48 @@ __global__ void bfinish_kernel(const double* __restrict__ partial, int nblk, con
   inv[q] = t > 0.0 ? (float)(1.0 / t) : 0.0f;
 }
 
-// v[row][q] = z[row][q] * inv[q]  (float4; total a multiple of kNR)
+// v[row][q] = z[row][q] * inv[q] for the first ncol columns (float4)
 __global__ void bscale_kernel(const float* __restrict__ z, const float* __restrict__ inv, float* __restrict__ v,
-                              int64_t total) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;   // float4 index
-  if (t * 4 >= total) return;
-  const int q = (int)((t * 4) % kNR);
-  float4 a = reinterpret_cast<const float4*>(z)[t];
+                              int64_t rows, int ncol) {
+  const int nq = ncol / 4;
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t row = t / nq;
+  if (row >= rows) return;
+  const int q = (int)(t - row * nq) * 4;
+  float4 a = *reinterpret_cast<const float4*>(z + row * kNR + q);
   a.x *= inv[q];
   a.y *= inv[q + 1];
   a.z *= inv[q + 2];
   a.w *= inv[q + 3];
-  reinterpret_cast<float4*>(v)[t] = a;
+  *reinterpret_cast<float4*>(v + row * kNR + q) = a;
 }
 
 // d[row][q] += sum_j Z_j[row][q] y[j][q]; y (k <= 32 rows of kNR) is
 // converted to FP32 once per CTA into shared memory, not once per entry
+// (first ncol columns, one float4 per thread, eight loads in flight)
 __global__ void __launch_bounds__(256) bcombine_kernel(const float* __restrict__ Z, int64_t ld, int k,
                                                        const double* __restrict__ y, float* __restrict__ d,
-                                                       int64_t total) {
-  __shared__ float ys[32 * kNR];
+                                                       int64_t rows, int ncol) {
+  __shared__ __align__(16) float ys[32 * kNR];
   for (int o = threadIdx.x; o < k * kNR; o += blockDim.x) ys[o] = (float)y[o];
   __syncthreads();
+  const int nq = ncol / 4;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= total) return;
-  const int q = (int)(t % kNR);
-  float s = d[t];
-  for (int j = 0; j < k; ++j) s += Z[(size_t)j * ld + t] * ys[j * kNR + q];
-  d[t] = s;
+  const int64_t row = t / nq;
+  if (row >= rows) return;
+  const int q = (int)(t - row * nq) * 4;
+  const int64_t o = row * kNR + q;
+  float4 s = *reinterpret_cast<const float4*>(d + o);
+#pragma unroll 8
+  for (int j = 0; j < k; ++j) {
+    const float4 z = *reinterpret_cast<const float4*>(Z + (size_t)j * ld + o);
+    const float4 yv = *reinterpret_cast<const float4*>(ys + j * kNR + q);
+    s.x += z.x * yv.x;
+    s.y += z.y * yv.y;
+    s.z += z.z * yv.z;
+    s.w += z.w * yv.w;
+  }
+  *reinterpret_cast<float4*>(d + o) = s;
 }
 
 // column norms^2 of an interleaved vector: partial[blk * kNR + q]
@@ -1646,7 +1670,10 @@ int bprecond(dg_ctx* c, const float* r, float* z, cudaStream_t st) {
     brestrict_kernel<<<nblk((int64_t)nn * kNR, 256), 256, 0, st>>>(S.lrr[l], S.le[l], S.lr[l + 1], S.le[l + 1], n, nn);
     bump();
   }
-  bdense2_kernel<<<nblk(M.lev[lc].n, kDnRows), 128, kDnSmem, st>>>(M.dense_inv, S.lr[lc], S.le[lc], M.lev[lc].n);
+  if (S.ncol > 32)
+    bdense2_kernel<16><<<nblk(M.lev[lc].n, kDnRows), 128, kDnSmem, st>>>(M.dense_inv, S.lr[lc], S.le[lc], M.lev[lc].n);
+  else
+    bdense2_kernel<8><<<nblk(M.lev[lc].n, kDnRows), 128, kDnSmem, st>>>(M.dense_inv, S.lr[lc], S.le[lc], M.lev[lc].n);
   bump();
   for (int l = lc - 1; l >= 0; --l) {
     const int n = M.lev[l].n;
@@ -1701,9 +1728,15 @@ int bcgs(dg_ctx* c, int j, float* w, int m, cudaStream_t st) {
   if (c->batched_gs2) {
     // low-register forms, 4 blocks per SM
     const int g = 4 * c->nsm;
-    bmdot2_kernel<<<dim3(g, (nv + 7) / 8), 256, 0, st>>>(S.V, ld, nv, w, c->nonods, S.part);
-    breduce2_kernel<<<dim3(nv, kNR / 16), 1024, 0, st>>>(S.part, g, S.h);
-    baxpy2_kernel<<<g, 256, 0, st>>>(S.V, ld, nv, S.h, w, c->nonods, S.part);
+    if (S.ncol > 32) {
+      bmdot2_kernel<16><<<dim3(g, (nv + 7) / 8), 256, 0, st>>>(S.V, ld, nv, w, c->nonods, S.part);
+      breduce2_kernel<<<dim3(nv, 4), 1024, 0, st>>>(S.part, g, S.h);
+      baxpy2_kernel<16><<<g, 256, 0, st>>>(S.V, ld, nv, S.h, w, c->nonods, S.part);
+    } else {
+      bmdot2_kernel<8><<<dim3(g, (nv + 7) / 8), 256, 0, st>>>(S.V, ld, nv, w, c->nonods, S.part);
+      breduce2_kernel<<<dim3(nv, 2), 1024, 0, st>>>(S.part, g, S.h);
+      baxpy2_kernel<8><<<g, 256, 0, st>>>(S.V, ld, nv, S.h, w, c->nonods, S.part);
+    }
     bfinish2_kernel<<<1, 1024, 0, st>>>(S.part, g, S.h, nv, j, m, S.H, S.inv);
   } else {
     bmdot_kernel<<<dim3(S.nblk, (nv + 7) / 8), 256, 0, st>>>(S.V, ld, nv, w, c->nonods, S.part);
@@ -1711,7 +1744,7 @@ int bcgs(dg_ctx* c, int j, float* w, int m, cudaStream_t st) {
     baxpy_kernel<<<S.nblk, 256, 0, st>>>(S.V, ld, nv, S.h, w, c->nonods, S.part);
     bfinish_kernel<<<1, kNR, 0, st>>>(S.part, S.nblk, S.h, nv, j, m, S.H, S.inv);
   }
-  bscale_kernel<<<nblk(ld / 4, 256), 256, 0, st>>>(w, S.inv, S.V + (size_t)nv * ld, ld);
+  bscale_kernel<<<nblk(c->nonods * (S.ncol / 4), 256), 256, 0, st>>>(w, S.inv, S.V + (size_t)nv * ld, c->nonods, S.ncol);
   bump(5);
   CKL(c);
   return DG_OK;
@@ -1726,7 +1759,7 @@ int bstep(dg_ctx* c, int j, int m, cudaStream_t st) {
   float* zj = S.Z + (size_t)j * ld;
   int rc;
   if ((rc = bprecond(c, S.V + (size_t)j * ld, zj, st))) return rc;
-  if ((rc = bres<float>(c, M.blk, M.W, zj, nullptr, S.t1, nullptr, RF_NEG, nullptr, st))) return rc;
+  if ((rc = bapply(c, M.blk, zj, nullptr, S.t1, true, S.ncol, st))) return rc;
   return bcgs(c, j, S.t1, m, st);
 }
 
@@ -1834,7 +1867,8 @@ extern "C" int dg_solve_mixed_batched(dg_ctx* c, double* x, const double* b, int
   CK(c, cudaFuncSetAttribute(bres_tc05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcDyn));
   CK(c, cudaFuncSetAttribute(bres_tcs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsDyn));
   CK(c, cudaFuncSetAttribute(bres_tcw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTwDyn));
-  CK(c, cudaFuncSetAttribute(bdense2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDnSmem));
+  CK(c, cudaFuncSetAttribute(bdense2_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDnSmem));
+  CK(c, cudaFuncSetAttribute(bdense2_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDnSmem));
   if ((rc = autotune_batched(c, M, batch_of(M), st))) return rc;
   if ((rc = ensure_batched_schedule(c, M, batch_of(M), st))) return rc;
   CK(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), st));   // bulk-copy wait time-outs land here
@@ -1908,12 +1942,12 @@ extern "C" int dg_solve_mixed_batched(dg_ctx* c, double* x, const double* b, int
       // V0 = rhs - A d (d = 0 on the first cycle); beta_q = |V0_q|
       if (first_cycle) {
         CK(c, cudaMemcpyAsync(S.V, S.t2, sizeof(float) * ld, cudaMemcpyDeviceToDevice, st));
-      } else if ((rc = bres<float>(c, M.blk, M.W, S.t6, S.t2, S.V, nullptr, 0, nullptr, st))) {
+      } else if ((rc = bapply(c, M.blk, S.t6, S.t2, S.V, false, S.ncol, st))) {
         return rc;
       }
       bnorm_kernel<<<S.nblk, 256, 0, st>>>(S.V, n, S.part);
       bnorm_finish_kernel<<<1, kNR, 0, st>>>(S.part, S.nblk, S.nrm, S.inv);
-      bscale_kernel<<<nblk(ld / 4, 256), 256, 0, st>>>(S.V, S.inv, S.V, ld);
+      bscale_kernel<<<nblk(n * (S.ncol / 4), 256), 256, 0, st>>>(S.V, S.inv, S.V, n, S.ncol);
       bump(3);
       CK(c, cudaMemcpyAsync(nrm.data(), S.nrm, sizeof(double) * kNR, cudaMemcpyDeviceToHost, st));
       CK(c, cudaMemsetAsync(S.H, 0, sizeof(double) * kNR * (m + 1) * m, st));
@@ -1980,7 +2014,7 @@ extern "C" int dg_solve_mixed_batched(dg_ctx* c, double* x, const double* b, int
         if (!(est <= target[q] * beta0[q])) alld = false;
       }
       CK(c, cudaMemcpyAsync(S.y, ybuf.data(), sizeof(double) * 32 * kNR, cudaMemcpyHostToDevice, st));
-      bcombine_kernel<<<nblk(ld, 256), 256, 0, st>>>(S.Z, ld, k, S.y, S.t6, ld);
+      bcombine_kernel<<<nblk(n * (S.ncol / 4), 256), 256, 0, st>>>(S.Z, ld, k, S.y, S.t6, n, S.ncol);
       bump();
       CKL(c);
       inner_done = alld;
@@ -2042,7 +2076,8 @@ int batched_prep(dg_ctx* c, const char* name, cudaStream_t st) {
   CK(c, cudaFuncSetAttribute(bres_tc05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcDyn));
   CK(c, cudaFuncSetAttribute(bres_tcs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsDyn));
   CK(c, cudaFuncSetAttribute(bres_tcw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTwDyn));
-  CK(c, cudaFuncSetAttribute(bdense2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDnSmem));
+  CK(c, cudaFuncSetAttribute(bdense2_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDnSmem));
+  CK(c, cudaFuncSetAttribute(bdense2_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDnSmem));
   return DG_OK;
 }
 
@@ -2055,7 +2090,7 @@ extern "C" int dg_apply_batched(dg_ctx* c, const float* x, float* y, void* strea
   int rc;
   if ((rc = batched_prep(c, "dg_apply_batched", st))) return rc;
   Mixed& M = mixed_of(c);
-  return bres<float>(c, M.blk, M.W, x, nullptr, y, nullptr, RF_NEG, nullptr, st);
+  return bapply(c, M.blk, x, nullptr, y, true, kNR, st);
 }
 
 // One smoothing step of the batched preconditioner with its BF16 copies:

@@ -224,6 +224,110 @@ __global__ void __launch_bounds__(160) bprolong_lane_kernel(float* __restrict__ 
   *xp = xv;
 }
 
+// FP32 operator product for the flexible GMRES, r = b - A x or (neg) A x - b
+// (b null = 0), one warp per element and 32 CP columns (CP per lane).  A block
+// is staged per warp (no CTA barrier) with the next one already in registers;
+// x rows are read by the lanes that use them.  A 16-byte word of the block
+// (four columns of a row, the same for all lanes) feeds 4 CP FMAs, so the
+// FMA pipe bounds it (123 MFMA per element and 64 columns: 150 us at 48,000
+// tetrahedra).  Same sums in the same order as bres_kernel (one CTA per
+// element, x slabs in shared memory: 471 us there, 313 us here; 32 columns of 7,722 elements
+// 82 -> 41 us).
+template <int CP>
+__global__ void __launch_bounds__(128, 5) bapply_kernel(const float* __restrict__ blk, const int* __restrict__ nbe,
+                                                        const float* __restrict__ x, const float* __restrict__ b,
+                                                        float* __restrict__ r, int64_t B, int neg) {
+  constexpr int N = 20, F = 4;
+  __shared__ __align__(16) float As[4][400];
+  const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t e = (int64_t)blockIdx.x * 4 + wi;
+  if (e >= B) return;   // whole warp; no CTA barrier below
+  using XT = typename std::conditional<CP == 2, float2, float>::type;
+  float* S = As[wi];
+  const int4 nb = reinterpret_cast<const int4*>(nbe)[e];
+  const float4* src = reinterpret_cast<const float4*>(blk + e * ((F + 1) * 400));
+  float4 a[4];
+  auto load_a = [&](int f) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (lane + 32 * q < 100) a[q] = __ldg(src + 100 * f + lane + 32 * q);
+  };
+  float acc[N][CP];
+#pragma unroll
+  for (int m = 0; m < N; ++m)
+#pragma unroll
+    for (int i = 0; i < CP; ++i) acc[m][i] = 0.0f;
+  load_a(0);
+#pragma unroll 1
+  for (int f = 0; f <= F; ++f) {
+    const int64_t s = f == 0 ? e : (f == 1 ? nb.x : (f == 2 ? nb.y : (f == 3 ? nb.z : nb.w)));
+    const XT* xp = reinterpret_cast<const XT*>(x + (s < 0 ? e : s) * (N * kNR)) + lane;
+    XT v[2][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[0][i] = xp[i * (kNR / CP)];
+    __syncwarp();   // the previous block has been used
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (lane + 32 * q < 100) reinterpret_cast<float4*>(S)[lane + 32 * q] = a[q];
+    __syncwarp();
+    if (f < F) load_a(f + 1);
+    if (s < 0) continue;
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+      if (c < 4)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[(c + 1) & 1][i] = xp[(4 * (c + 1) + i) * (kNR / CP)];
+      float xv[4][CP];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if constexpr (CP == 2) {
+          xv[i][0] = v[c & 1][i].x;
+          xv[i][1] = v[c & 1][i].y;
+        } else {
+          xv[i][0] = v[c & 1][i];
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < N; ++m) {
+        const float4 av = *reinterpret_cast<const float4*>(S + 80 * c + 4 * m);
+#pragma unroll
+        for (int i = 0; i < CP; ++i) {
+          acc[m][i] = fmaf(av.x, xv[0][i], acc[m][i]);
+          acc[m][i] = fmaf(av.y, xv[1][i], acc[m][i]);
+          acc[m][i] = fmaf(av.z, xv[2][i], acc[m][i]);
+          acc[m][i] = fmaf(av.w, xv[3][i], acc[m][i]);
+        }
+      }
+    }
+  }
+  const float sg = neg ? -1.0f : 1.0f;
+  const int64_t o = e * (N * kNR / CP) + lane;
+#pragma unroll
+  for (int m = 0; m < N; ++m) {
+    if constexpr (CP == 2) {
+      float2 bv = make_float2(0.0f, 0.0f);
+      if (b) bv = reinterpret_cast<const float2*>(b)[o + m * (kNR / 2)];
+      reinterpret_cast<float2*>(r)[o + m * (kNR / 2)] = make_float2(sg * (bv.x - acc[m][0]), sg * (bv.y - acc[m][1]));
+    } else {
+      const float bv = b ? b[o + m * kNR] : 0.0f;
+      r[o + m * kNR] = sg * (bv - acc[m][0]);
+    }
+  }
+}
+
+int bapply(dg_ctx* c, const float* blk, const float* x, const float* b, float* r, bool neg, int ncol,
+           cudaStream_t st) {
+  if (c->B > 0) {
+    if (ncol > 32)
+      bapply_kernel<2><<<nblk(c->B, 4), 128, 0, st>>>(blk, c->d_nbe, x, b, r, c->B, neg ? 1 : 0);
+    else
+      bapply_kernel<1><<<nblk(c->B, 4), 128, 0, st>>>(blk, c->d_nbe, x, b, r, c->B, neg ? 1 : 0);
+  }
+  bump();
+  CKL(c);
+  return DG_OK;
+}
+
 // ncol (32 or kNR): columns to compute
 template <int MODE, bool XL, bool CL, bool OL, bool AL16 = true>
 int launch_bwarp(dg_ctx* c, const __nv_bfloat16* mat, const float* x, const float* cv, float* x_out, float* c_out,
