@@ -1882,23 +1882,44 @@ extern "C" int dg_solve_mixed_batched(dg_ctx* c, double* x, const double* b, int
   std::vector<char> active(kNR, 0);
   for (int q = 0; q < nrhs; ++q) tolv[q] = tol[q];
   std::vector<double> Hh((size_t)kNR * (m + 1) * m), ybuf((size_t)32 * kNR), nrm(kNR), rnew(kNR);
-  // FP64 residuals r_q = b_q - A x_q (one FP64 apply per RHS, bound by the
-  // FP64 pipe) for the RHS in `redo`; the others keep r_q and |r_q|: a zero
-  // start gives r_q = b_q exactly, and an RHS that no refinement step
-  // updated keeps its x_q
+  // FP64 residuals r_q = b_q - A x_q for the RHS in `redo`, all in one
+  // product on the tensor cores (dg_fp64_mma.cuh); the others keep r_q and
+  // |r_q|: a zero start gives r_q = b_q exactly, and an RHS that no refinement
+  // step updated keeps its x_q
   std::vector<char> redo(kNR, 0);
   auto outer_residuals = [&]() -> int {
     int r2;
+    unsigned long long mask = 0;
+    bool copy_all = true;
     for (int q = 0; q < nrhs; ++q) {
-      if (!redo[q]) continue;
-      if (redo[q] == 2) {
-        CK(c, cudaMemcpyAsync(S.r64 + (size_t)q * n, b + (size_t)q * n, sizeof(double) * n, cudaMemcpyDeviceToDevice,
-                              st));
-      } else if ((r2 = residual(c, x + (size_t)q * n, b + (size_t)q * n, S.r64 + (size_t)q * n, nullptr, 0, st))) {
-        return r2;
-      }
-      if ((r2 = norm2(c, S.r64 + (size_t)q * n, c->d_scal + q, st))) return r2;
+      if (redo[q] == 1) mask |= 1ull << q;
+      copy_all = copy_all && redo[q] == 2;
     }
+    if (copy_all) {
+      CK(c, cudaMemcpyAsync(S.r64, b, sizeof(double) * n * nrhs, cudaMemcpyDeviceToDevice, st));
+    } else {
+      for (int q = 0; q < nrhs; ++q)
+        if (redo[q] == 2)
+          CK(c, cudaMemcpyAsync(S.r64 + (size_t)q * n, b + (size_t)q * n, sizeof(double) * n, cudaMemcpyDeviceToDevice,
+                                st));
+    }
+    const int gx = (int)std::max<int64_t>(1, std::min<int64_t>(2 * c->nsm, (n + 255) / 256));
+    if (mask) {
+      if ((r2 = ensure_digits(c, st))) return r2;
+      const int ngr = (nrhs + 15) / 16;
+      int* emax = reinterpret_cast<int*>(S.h);   // scratch between the inner solves, as the basis is
+      unsigned char* xdig = reinterpret_cast<unsigned char*>(S.V);   // (m + 1 >= 2) x 4 bytes per value
+      CK(c, cudaMemsetAsync(emax, 0, sizeof(int) * kNR, st));
+      bexp_kernel<<<dim3(gx, nrhs), 256, 0, st>>>(x, n, emax);
+      x_digits_kernel<<<dim3((unsigned)c->B, ngr), 160, 0, st>>>(x, n, emax, mask, xdig);
+      bres64_mma_kernel<<<nblk(c->B * ngr, 4), 128, 0, st>>>(c->d_adig, c->d_aexp, c->d_nbe, xdig, emax, b, S.r64,
+                                                             c->B, n, ngr, mask);
+      bump(3);
+    }
+    bnorm64_kernel<<<dim3(gx, nrhs), 256, 0, st>>>(S.r64, n, S.part);
+    bnorm_finish_kernel<<<1, kNR, 0, st>>>(S.part, gx, c->d_scal, nullptr);
+    bump(2);
+    CKL(c);
     CK(c, cudaMemcpyAsync(rnew.data(), c->d_scal, sizeof(double) * nrhs, cudaMemcpyDeviceToHost, st));
     CK(c, cudaStreamSynchronize(st));
     for (int q = 0; q < nrhs; ++q)

@@ -1,0 +1,315 @@
+// FP64 block products on the tensor cores, exact in slices.  Included by
+// dg_solver.cu.
+//
+// The FP64 pipe takes 2 FMA per clock and SM, so b - A x with the FP64 blocks
+// runs at that pipe's rate (170 us at 48,000 tetrahedra against 113 us for
+// its bytes), 64 times over for 64 right-hand sides.  Here the operands are
+// cut into eight signed 8-bit digits each (the error-free splitting of Ozaki,
+// Ogita, Oishi and Rump, Numer. Algorithms 59, 2012): a row of
+// [A_e0 .. A_e4] as 2^(ea - 62) times 63-bit integers, ea its largest
+// exponent, and x_q as 2^(ex - 62) times such integers.  A product of two
+// digits is at most 2^14 and a sum over 100 columns and up to 8 digit pairs
+// below 2^24, so mma.sync with FP16 operands (exact integers up to 2,048) and
+// FP32 accumulators adds them without rounding.  Pairs (i, j) of digits with
+// i + j = s share an accumulator; s = 0 .. 7 are kept (36 of 64 pairs, the
+// rest is below 2^-58 of the row's and x's scale) and joined as integers:
+//   A x = 2^(ea + ex - 36) (H + 2^-32 L),
+// H, L 48-bit integers, one FP64 rounding each for the sum and for b - A x.
+// The result is at least as close to the exact one as the FP64 loop's
+// (tested).
+//
+// Digits are stored as bytes d + 128, so that one byte permute with 0x64
+// makes FP16 1024 + 128 + d and one subtraction d.  Eight bytes per value, in
+// the order the mma lanes read them: for a node pair p = 4 r + t (see
+// dg_batched_warp.cuh) 16 bytes, word k = [d_2k(n0), d_2k(n1), d_2k+1(n0),
+// d_2k+1(n1)].
+#pragma once
+
+namespace {
+
+constexpr int kDigBlock = 3200;             // bytes of one block's digits (400 values)
+constexpr int kDigElem = 5 * kDigBlock;     // bytes of an element's blocks
+constexpr uint32_t kZeroDigits = 0x80808080u;
+
+// byte offset of (r, row m, t) in a block's digits: rows of 4 (r < 2) or 2
+// (r = 2) 16-byte pieces
+__device__ __forceinline__ int dig_off(int r, int m, int t) {
+  return r < 2 ? 1280 * r + 64 * m + 16 * t : 2560 + 32 * m + 16 * t;
+}
+
+// |v| 2^k rounded to an integer, with the sign of v (v = its bits; up to 63
+// bits of the integer part are kept by the caller's choice of k): the
+// mantissa shifted by sh = k + E - 1075
+__device__ __forceinline__ long long fixed_point(unsigned long long v, int k) {
+  const int E = (int)((v >> 52) & 2047);
+  unsigned long long M = v & 0xfffffffffffffull;
+  if (E) M |= 0x10000000000000ull;
+  const int sh = k + (E ? E : 1) - 1075;
+  unsigned long long q;
+  if (sh >= 0) q = M << sh;
+  else if (sh > -64) q = ((M >> (-sh - 1)) + 1) >> 1;
+  else q = 0;
+  return (long long)v < 0 ? -(long long)q : (long long)q;
+}
+
+// the 16 bytes of two values' biased digits (u0, u1: digit 0 in the top byte)
+__device__ __forceinline__ uint4 digit_words(unsigned long long u0, unsigned long long u1) {
+  const uint32_t h0 = (uint32_t)(u0 >> 32), l0 = (uint32_t)u0, h1 = (uint32_t)(u1 >> 32), l1 = (uint32_t)u1;
+  uint4 w;   // selectors: byte 3 of an operand is its top byte
+  w.x = __byte_perm(h0, h1, 0x6273);
+  w.y = __byte_perm(h0, h1, 0x4051);
+  w.z = __byte_perm(l0, l1, 0x6273);
+  w.w = __byte_perm(l0, l1, 0x4051);
+  return w;
+}
+
+// FP16 pair of digit 2k (hi = 0) or 2k + 1 (hi = 1) from word k
+template <int HI>
+__device__ __forceinline__ uint32_t digit_pair(uint32_t w) {
+  const uint32_t v = __byte_perm(w, 0x64646464u, HI ? 0x4342 : 0x4140);
+  uint32_t d;
+  asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(v), "r"(0x64806480u));   // - (1024 + 128)
+  return d;
+}
+
+__device__ __forceinline__ void mma_f16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                              uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// 2^e as a double, e clamped to the normal range
+__device__ __forceinline__ double exp2_int(int e) {
+  e = min(max(e, -1022), 1023);
+  return __longlong_as_double((long long)(e + 1023) << 52);
+}
+
+// a 48-bit signed integer as a double, exactly (one FP64 addition)
+__device__ __forceinline__ double int48_to_double(long long v) {
+  return __longlong_as_double(0x4330000000000000ll + (v + (1ll << 51))) - (4503599627370496.0 + 2251799813685248.0);
+}
+
+// sum of four accumulators, 8 bits apart
+__device__ __forceinline__ long long join4(float a, float b, float c, float d) {
+  const long long hi = ((long long)__float2int_rn(a) << 8) + __float2int_rn(b);
+  return (((hi << 8) + __float2int_rn(c)) << 8) + __float2int_rn(d);
+}
+
+// Digits and row exponents of all blocks; one CTA of 128 threads per element.
+// ea[e * 20 + m]: |entries of row m| < 2^ea (0x7fff: a value is not finite).
+__global__ void __launch_bounds__(128) block_digits_kernel(const double* __restrict__ blk,
+                                                           unsigned char* __restrict__ dig, int* __restrict__ ea) {
+  __shared__ unsigned long long v[2000];
+  __shared__ int emax[5][20];
+  __shared__ int er[20];
+  const int64_t e = blockIdx.x;
+  const unsigned long long* src = reinterpret_cast<const unsigned long long*>(blk) + e * 2000;
+  for (int k = threadIdx.x; k < 2000; k += 128) v[k] = src[k];   // entry (m, n) of block b at b * 400 + n * 20 + m
+  __syncthreads();
+  if (threadIdx.x < 100) {
+    const int m = threadIdx.x % 20, b = threadIdx.x / 20;
+    int mx = 1;
+    for (int n = 0; n < 20; ++n) mx = max(mx, (int)((v[b * 400 + n * 20 + m] >> 52) & 2047));
+    emax[b][m] = mx;
+  }
+  __syncthreads();
+  if (threadIdx.x < 20) {
+    int mx = 1;
+    for (int b = 0; b < 5; ++b) mx = max(mx, emax[b][threadIdx.x]);
+    er[threadIdx.x] = mx;
+    ea[e * 20 + threadIdx.x] = mx == 2047 ? 0x7fff : mx - 1022;
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < 1000; k += 128) {   // (block, row, pair)
+    const int b = k / 200, m = (k / 10) % 20, p = k % 10;
+    unsigned long long u[2];
+#pragma unroll
+    for (int d = 0; d < 2; ++d)   // k = 62 - ea
+      u[d] = (unsigned long long)fixed_point(v[b * 400 + (2 * p + d) * 20 + m], 1084 - er[m]) + 0x8080808080808080ull;
+    *reinterpret_cast<uint4*>(dig + e * kDigElem + b * kDigBlock + dig_off(p / 4, m, p % 4)) = digit_words(u[0], u[1]);
+  }
+}
+
+// emax[q] = largest biased exponent of x_q (RHS-major (nrhs, n)); zeroed by
+// the caller, grid (blocks, nrhs)
+__global__ void bexp_kernel(const double* __restrict__ x, int64_t n, int* __restrict__ emax) {
+  const int q = blockIdx.y;
+  const unsigned long long* p = reinterpret_cast<const unsigned long long*>(x) + (int64_t)q * n;
+  int mx = 0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    mx = max(mx, (int)((p[i] >> 52) & 2047));
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if ((threadIdx.x & 31) == 0) atomicMax(emax + q, mx);
+}
+
+// Digits of x for the batched product: per element and 16 right-hand sides
+// [r][RHS parity][lane][16 bytes], lane (g, t) holding right-hand side
+// 16 group + 2 g + parity and nodes 2 (4 r + t), + 1; 2,560 bytes.  One CTA of
+// 160 threads per element, grid y = groups; right-hand sides outside mask
+// get zero digits.
+__global__ void __launch_bounds__(160) x_digits_kernel(const double* __restrict__ x, int64_t n,
+                                                       const int* __restrict__ emax, unsigned long long mask,
+                                                       unsigned char* __restrict__ dig) {
+  const int64_t e = blockIdx.x;
+  const int i = threadIdx.x, gr = blockIdx.y;
+  const int r = i < 128 ? i / 64 : 2, q = i < 128 ? (i / 32) % 2 : (i - 128) / 16;
+  const int l = i < 128 ? i % 32 : (i - 128) % 16;
+  const int g = r < 2 ? l / 4 : l / 2, t = r < 2 ? l % 4 : l % 2;
+  const int col = 16 * gr + 2 * g + q;
+  uint4 w = make_uint4(kZeroDigits, kZeroDigits, kZeroDigits, kZeroDigits);
+  if ((mask >> col) & 1) {
+    const unsigned long long* p =
+        reinterpret_cast<const unsigned long long*>(x) + (int64_t)col * n + e * 20 + 2 * (4 * r + t);
+    const int k = 1084 - max(emax[col], 1);   // 62 - ex
+    w = digit_words((unsigned long long)fixed_point(p[0], k) + 0x8080808080808080ull,
+                    (unsigned long long)fixed_point(p[1], k) + 0x8080808080808080ull);
+  }
+  *reinterpret_cast<uint4*>(dig + (e * gridDim.y + gr) * 2560 + 16 * i) = w;
+}
+
+// r_q = b_q - A x_q for the right-hand sides in mask, RHS-major FP64: one warp
+// per element and 16 right-hand sides, X^T digits as the A operand, the
+// block rows' digits as the B operand.  Bound by the mma.sync rate (36 digit
+// pairs x 3 mma x 8 k-tiles per warp: 1.1 ms at 48,000 tetrahedra x 64 against
+// 10.9 ms for 64 products on the FP64 pipe); 1.94 ms.
+__global__ void __launch_bounds__(128, 2) bres64_mma_kernel(const unsigned char* __restrict__ adig,
+                                                            const int* __restrict__ ea, const int* __restrict__ nbe,
+                                                            const unsigned char* __restrict__ xdig,
+                                                            const int* __restrict__ emax, const double* __restrict__ b,
+                                                            double* __restrict__ r, int64_t B, int64_t n, int ngr,
+                                                            unsigned long long mask) {
+  constexpr int N = 20, NB = 5, NS = 15, KT = 8;
+  const int64_t wid = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int64_t e = wid / ngr;
+  if (e >= B) return;   // whole warp
+  const int gr = (int)(wid - e * ngr);
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int4 nb = reinterpret_cast<const int4*>(nbe)[e];
+  float acc[8][3][4];
+#pragma unroll
+  for (int s = 0; s < 8; ++s)
+#pragma unroll
+    for (int nt = 0; nt < 3; ++nt)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[s][nt][i] = 0.0f;
+  const uint4 z = make_uint4(kZeroDigits, kZeroDigits, kZeroDigits, kZeroDigits);
+  uint4 xw[2][2], aw[3][2];   // raw words of the next k-tile: x (slot, RHS parity), block rows
+  auto load = [&](int kt) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int s = 2 * kt + h;
+      const int bb = s < 2 * NB ? s / 2 : s - 2 * NB, rr = s < 2 * NB ? s % 2 : 2;
+      const bool on = s < NS && (rr < 2 || t < 2);
+      const int64_t src = bb == 0 ? e : (bb == 1 ? nb.x : (bb == 2 ? nb.y : (bb == 3 ? nb.z : nb.w)));
+      xw[h][0] = xw[h][1] = z;
+      if (on && src >= 0) {
+        const unsigned char* p =
+            xdig + (src * ngr + gr) * 2560 + (rr < 2 ? 1024 * rr + 16 * lane : 2048 + 16 * (2 * g + t));
+        xw[h][0] = *reinterpret_cast<const uint4*>(p);
+        xw[h][1] = *reinterpret_cast<const uint4*>(p + (rr < 2 ? 512 : 256));
+      }
+#pragma unroll
+      for (int nt = 0; nt < 3; ++nt) {
+        const int m = 8 * nt + g;
+        aw[nt][h] = (on && m < N) ? __ldg(reinterpret_cast<const uint4*>(adig + e * kDigElem + bb * kDigBlock +
+                                                                        dig_off(rr, m, t)))
+                                  : z;
+      }
+    }
+  };
+  load(0);
+#pragma unroll 1
+  for (int kt = 0; kt < KT; ++kt) {
+    uint32_t xa[8][4];   // A fragments by digit of x
+    uint4 ac[3][2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const uint32_t w[4] = {xw[h][q].x, xw[h][q].y, xw[h][q].z, xw[h][q].w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          xa[2 * k][2 * h + q] = digit_pair<0>(w[k]);
+          xa[2 * k + 1][2 * h + q] = digit_pair<1>(w[k]);
+        }
+      }
+#pragma unroll
+      for (int nt = 0; nt < 3; ++nt) ac[nt][h] = aw[nt][h];
+    }
+    if (kt + 1 < KT) load(kt + 1);   // in flight during the products
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {   // digit of A
+#pragma unroll
+      for (int nt = 0; nt < 3; ++nt) {
+        uint32_t bf[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t w = i / 2 == 0 ? ac[nt][h].x : (i / 2 == 1 ? ac[nt][h].y : (i / 2 == 2 ? ac[nt][h].z : ac[nt][h].w));
+          bf[h] = i % 2 == 0 ? digit_pair<0>(w) : digit_pair<1>(w);
+        }
+#pragma unroll
+        for (int j = 0; j < 8 - i; ++j)
+          mma_f16_16816(acc[i + j][nt], xa[j][0], xa[j][1], xa[j][2], xa[j][3], bf[0], bf[1]);
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {   // right-hand side 2 g + q: accumulators 2 q, 2 q + 1
+    const int col = 16 * gr + 2 * g + q;
+    if (!((mask >> col) & 1)) continue;
+    const int em = emax[col], ex = max(em, 1) - 1022;
+#pragma unroll
+    for (int nt = 0; nt < 3; ++nt) {
+      const int m = 8 * nt + 2 * t;
+      if (m >= N) continue;
+      const int64_t o = (int64_t)col * n + e * N + m;
+      double out[2];
+#pragma unroll
+      for (int d = 0; d < 2; ++d) {
+        const int c = 2 * q + d, ee = ea[e * N + m + d];
+        const double H = int48_to_double(join4(acc[0][nt][c], acc[1][nt][c], acc[2][nt][c], acc[3][nt][c]));
+        const double L = int48_to_double(join4(acc[4][nt][c], acc[5][nt][c], acc[6][nt][c], acc[7][nt][c]));
+        const double sc = em == 2047 || ee == 0x7fff ? __longlong_as_double(0x7ff8000000000000ll) : exp2_int(ee + ex - 36);
+        out[d] = fma(-sc, fma(L, 0x1p-32, H), b[o + d]);
+      }
+      *reinterpret_cast<double2*>(r + o) = make_double2(out[0], out[1]);
+    }
+  }
+}
+
+// partial[blk * 64 + q] = this block's slice of |z_q|^2, z (nrhs, n)
+// RHS-major; grid (blocks, nrhs)
+__global__ void __launch_bounds__(256) bnorm64_kernel(const double* __restrict__ z, int64_t n,
+                                                      double* __restrict__ partial) {
+  __shared__ double red[8];
+  const double* p = z + (int64_t)blockIdx.y * n;
+  double acc = 0.0;
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256)
+    acc = fma(p[i], p[i], acc);
+  acc = warp_sum(acc);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int w = 0; w < 8; ++w) s += red[w];
+    partial[(int64_t)blockIdx.x * 64 + blockIdx.y] = s;
+  }
+}
+
+// block digits of the current operator build (3D), formed on first use and
+// kept with the context
+int ensure_digits(dg_ctx* c, cudaStream_t st) {
+  if (c->dig_version == c->build_version) return DG_OK;
+  int rc;
+  if (!c->d_adig && (rc = dalloc(c, &c->d_adig, (size_t)c->B * kDigElem))) return rc;
+  if (!c->d_aexp && (rc = dalloc(c, &c->d_aexp, (size_t)c->B * 20))) return rc;
+  if (c->B > 0) block_digits_kernel<<<(unsigned)c->B, 128, 0, st>>>(c->d_blk, c->d_adig, c->d_aexp);
+  bump();
+  CKL(c);
+  c->dig_version = c->build_version;
+  return DG_OK;
+}
+
+}  // namespace

@@ -121,6 +121,10 @@ struct dg_ctx {
   FaceNodes* d_fnodes = nullptr;   // nodes on each face (basis not identically zero there)
   double* d_blk = nullptr;
   double* d_W = nullptr;        // (B, N, N) smoother matrices
+  // digit copy of the blocks (dg_fp64_mma.cuh): bytes, row exponents
+  unsigned char* d_adig = nullptr;
+  int* d_aexp = nullptr;
+  int dig_version = -1;
   double* d_detw = nullptr;
   int* d_err = nullptr;
   // boundary faces for the right-hand side
@@ -1108,6 +1112,7 @@ int read_scalar(dg_ctx* c, const double* d, double* h, cudaStream_t st) {
 
 }  // namespace
 
+#include "dg_fp64_mma.cuh"
 #include "dg_mixed.cuh"
 #include "dg_batched.cuh"
 
