@@ -1888,7 +1888,7 @@ extern "C" int dg_solve_mixed_batched(dg_ctx* c, double* x, const double* b, int
   // step updated keeps its x_q
   std::vector<char> redo(kNR, 0);
   auto outer_residuals = [&]() -> int {
-    int r2;
+    int r2 = DG_OK;
     unsigned long long mask = 0;
     bool copy_all = true;
     for (int q = 0; q < nrhs; ++q) {
@@ -1904,8 +1904,13 @@ extern "C" int dg_solve_mixed_batched(dg_ctx* c, double* x, const double* b, int
                                 st));
     }
     const int gx = (int)std::max<int64_t>(1, std::min<int64_t>(2 * c->nsm, (n + 255) / 256));
-    if (mask) {
-      if ((r2 = ensure_digits(c, st))) return r2;
+    if (mask && (r2 = ensure_digits(c, st)) == DG_ERR_ALLOC) {   // no room: one product per RHS
+      for (int q = 0; q < nrhs; ++q)
+        if (redo[q] == 1 &&
+            (r2 = residual(c, x + (size_t)q * n, b + (size_t)q * n, S.r64 + (size_t)q * n, nullptr, 0, st)))
+          return r2;
+    } else if (mask) {
+      if (r2) return r2;
       const int ngr = (nrhs + 15) / 16;
       int* emax = reinterpret_cast<int*>(S.h);   // scratch between the inner solves, as the basis is
       unsigned char* xdig = reinterpret_cast<unsigned char*>(S.V);   // (m + 1 >= 2) x 4 bytes per value

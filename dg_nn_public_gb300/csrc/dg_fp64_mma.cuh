@@ -22,19 +22,19 @@
 // makes FP16 1024 + 128 + d and one subtraction d.  Eight bytes per value, in
 // the order the mma lanes read them: for a node pair p = 4 r + t (see
 // dg_batched_warp.cuh) 16 bytes, word k = [d_2k(n0), d_2k(n1), d_2k+1(n0),
-// d_2k+1(n1)].
+// d_2k+1(n1)]; an element as [slot][row][t], slots 0 .. 9 = (block, r = 0, 1),
+// 10 .. 14 = (block, r = 2, t < 2), so that a load is contiguous across the
+// warp.
 #pragma once
 
 namespace {
 
-constexpr int kDigBlock = 3200;             // bytes of one block's digits (400 values)
-constexpr int kDigElem = 5 * kDigBlock;     // bytes of an element's blocks
+constexpr int kDigElem = 16000;             // bytes of an element's digits
 constexpr uint32_t kZeroDigits = 0x80808080u;
 
-// byte offset of (r, row m, t) in a block's digits: rows of 4 (r < 2) or 2
-// (r = 2) 16-byte pieces
-__device__ __forceinline__ int dig_off(int r, int m, int t) {
-  return r < 2 ? 1280 * r + 64 * m + 16 * t : 2560 + 32 * m + 16 * t;
+// byte offset of (slot, row m, t) in an element's digits
+__device__ __forceinline__ int dig_off(int s, int m, int t) {
+  return s < 10 ? 1280 * s + 64 * m + 16 * t : 12800 + 640 * (s - 10) + 32 * m + 16 * t;
 }
 
 // |v| 2^k rounded to an integer, with the sign of v (v = its bits; up to 63
@@ -69,6 +69,14 @@ __device__ __forceinline__ uint32_t digit_pair(uint32_t w) {
   const uint32_t v = __byte_perm(w, 0x64646464u, HI ? 0x4342 : 0x4140);
   uint32_t d;
   asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(v), "r"(0x64806480u));   // - (1024 + 128)
+  return d;
+}
+
+// the same with the half chosen by the lane (selector 0x4140 or 0x4342)
+__device__ __forceinline__ uint32_t digit_sel(uint32_t w, uint32_t sel) {
+  const uint32_t v = __byte_perm(w, 0x64646464u, sel);
+  uint32_t d;
+  asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(v), "r"(0x64806480u));
   return d;
 }
 
@@ -128,7 +136,8 @@ __global__ void __launch_bounds__(128) block_digits_kernel(const double* __restr
 #pragma unroll
     for (int d = 0; d < 2; ++d)   // k = 62 - ea
       u[d] = (unsigned long long)fixed_point(v[b * 400 + (2 * p + d) * 20 + m], 1084 - er[m]) + 0x8080808080808080ull;
-    *reinterpret_cast<uint4*>(dig + e * kDigElem + b * kDigBlock + dig_off(p / 4, m, p % 4)) = digit_words(u[0], u[1]);
+    *reinterpret_cast<uint4*>(dig + e * kDigElem + dig_off(p < 8 ? 2 * b + p / 4 : 10 + b, m, p % 4)) =
+        digit_words(u[0], u[1]);
   }
 }
 
@@ -213,9 +222,8 @@ __global__ void __launch_bounds__(128, 2) bres64_mma_kernel(const unsigned char*
 #pragma unroll
       for (int nt = 0; nt < 3; ++nt) {
         const int m = 8 * nt + g;
-        aw[nt][h] = (on && m < N) ? __ldg(reinterpret_cast<const uint4*>(adig + e * kDigElem + bb * kDigBlock +
-                                                                        dig_off(rr, m, t)))
-                                  : z;
+        aw[nt][h] =
+            (on && m < N) ? __ldg(reinterpret_cast<const uint4*>(adig + e * kDigElem + dig_off(s, m, t))) : z;
       }
     }
   };
@@ -279,6 +287,264 @@ __global__ void __launch_bounds__(128, 2) bres64_mma_kernel(const unsigned char*
   }
 }
 
+// residual_kernel<20, 4> in FP64 for one right-hand side (same flags; RF_ZEROX
+// has no product and stays there): persistent, one warp per element.  The
+// eight digits of x are the columns of the B operand, so (row, digit of A)
+// pairs are the rows of A: rows 0 .. 15 of one digit are a tile, rows 16 .. 19
+// of four digits another, 10 tiles in all and none of it padding (the other
+// way round, with the digits of x as rows, half of every tile is: 192 mma and
+// 2,800 instructions per element instead of 80 mma: 233 us).  Lane (g, t)
+// then has, for its rows, all digits of A against digits 2 t, 2 t + 1 of x:
+// joined in 32- and 64-bit integers and added over the four lanes.
+// x is scaled by the largest of its 100 values at the element.  The smoother
+// product runs on the FP64 pipe, which the digits leave idle.
+//
+// Bound by HBM (16.0 KB of digits per element, as the FP64 blocks, + 3.2 KB
+// with the smoother).  Every warp streams its own elements' chunks by bulk
+// copies into two shared-memory stages and gathers the next element's x
+// while it works, so no round trip is waited for: 48,000 tetrahedra
+// apply 122 us, smoothing step 147 us (113 / 136 us at HBM rate; FP64 pipe
+// 171 / 206 us); 3,072 tetrahedra 17.0 -> 12.8 us.
+// Waits are bounded: on time-out the warp's remaining rows become NaN.
+constexpr int kR64Warps = 8, kR64Stage = 5760;
+constexpr int kR64Smem = kR64Warps * 2 * kR64Stage;
+
+__global__ void __launch_bounds__(32 * kR64Warps, 2) res64_mma_kernel(
+    const unsigned char* __restrict__ adig, const int* __restrict__ ea, const double* __restrict__ W,
+    const int* __restrict__ nbe, const double* __restrict__ x, const double* __restrict__ b, double* __restrict__ r,
+    double* __restrict__ x_out, int64_t B, int flags, const double* __restrict__ P, double* __restrict__ r1) {
+  constexpr int N = 20, F = 4, NB = 5, NS = 15;
+  extern __shared__ __align__(128) unsigned char r64_smem[];
+  __shared__ __align__(16) uint32_t xw_s[kR64Warps][2][104];   // biased digits of x: upper and lower words
+  __shared__ double rs_s[kR64Warps][N];
+  __shared__ __align__(8) uint64_t bar_s[kR64Warps][2];
+  const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  unsigned char* stage = r64_smem + wi * 2 * kR64Stage;
+  uint64_t* bar = bar_s[wi];
+  const int64_t stride = (int64_t)gridDim.x * kR64Warps;
+  const int64_t e0 = (int64_t)blockIdx.x * kR64Warps + wi;
+  const bool smooth = flags & RF_SMOOTH;
+  const int nch = smooth ? 4 : 3;   // chunks per element: slots 0 - 3, 4 - 7, 8 - 14, the smoother matrix
+  if (lane == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncwarp();
+  if (e0 >= B) return;   // whole warp; no CTA barrier below
+  // lane 0: chunk i of element ce to the stage of running number ci
+  int64_t ce = e0;
+  int ci = 0, cn = 0;   // next chunk to copy: index in its element, running number
+  auto issue = [&]() {
+    if (ce >= B) return;
+    const uint32_t bytes = ci < 2 ? 5120u : (ci == 2 ? 5760u : 3200u);
+    const void* src = ci < 3 ? (const void*)(adig + ce * kDigElem + 5120 * ci) : (const void*)(W + ce * (N * N));
+    mbar_expect_tx(&bar[cn & 1], bytes);
+    bulk_copy_g2s(stage + (cn & 1) * kR64Stage, src, bytes, &bar[cn & 1]);
+    ++cn;
+    if (++ci == nch) {
+      ci = 0;
+      ce += stride;
+    }
+  };
+  if (lane == 0) {
+    issue();
+    issue();
+  }
+  auto load_nb = [&](int64_t e) { return reinterpret_cast<const int4*>(nbe)[e < B ? e : e0]; };
+  int4 nb = load_nb(e0);
+  pdl_wait_then_trigger();   // digits, smoother and neighbours are fixed data, x and b are not
+  const int q8 = g >> 2;     // rows 16 ..: this lane's digits of A are q8, q8 + 2, ...
+  const int m = (t & 1) ? 16 + g : g + 4 * t;   // the row this lane writes
+  const bool mine = t == 0 || t == 2 || (t == 1 && g < 4);
+  const uint32_t tsel = q8 ? 0x4342u : 0x4140u;
+  unsigned long long v[4];
+  double bv;
+  int ee;
+  auto gather = [&](int64_t e) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int k = lane + 32 * q, bb = k / N;
+      v[q] = 0;
+      if (k < NB * N) {
+        const int64_t src = bb == 0 ? e : (bb == 1 ? nb.x : (bb == 2 ? nb.y : (bb == 3 ? nb.z : nb.w)));
+        if (src >= 0) v[q] = reinterpret_cast<const unsigned long long*>(x)[src * N + k - bb * N];
+      }
+    }
+    bv = mine && b ? b[e * N + m] : 0.0;
+    ee = mine ? ea[e * N + m] : 0;
+  };
+  gather(e0);
+  nb = load_nb(e0 + stride);
+  uint32_t(*xw)[104] = xw_s[wi];
+  double* rs = rs_s[wi];
+  bool dead = false;
+  int cc = 0;   // running number of the chunk to use
+  auto wait = [&]() {
+    if (!dead && !mbar_wait_bounded(&bar[cc & 1], (uint32_t)((cc >> 1) & 1))) dead = true;
+    dead = __any_sync(0xffffffffu, dead);
+  };
+  auto done = [&]() {   // the stage has been read: refill it
+    __syncwarp();
+    if (lane == 0 && !dead) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      issue();
+    }
+    ++cc;
+  };
+  for (int64_t e = e0; e < B; e += stride) {
+    int mx = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) mx = max(mx, (int)((v[q] >> 52) & 2047));
+    const int em = max(__reduce_max_sync(0xffffffffu, mx), 1);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int k = lane + 32 * q;
+      if (k < NB * N) {
+        // 2^62 / 2^ex times the value, cut off below its last bit
+        const int E = (int)((v[q] >> 52) & 2047);
+        const unsigned long long M = ((v[q] & 0xfffffffffffffull) | (E ? 0x10000000000000ull : 0ull)) << 9;
+        const unsigned long long p = M >> min(em - max(E, 1), 63);
+        const unsigned long long u = ((long long)v[q] < 0 ? 0ull - p : p) + 0x8080808080808080ull;
+        xw[0][k] = (uint32_t)(u >> 32);
+        xw[1][k] = (uint32_t)u;
+      }
+    }
+    __syncwarp();
+    uint32_t xb[16];   // B fragments (column = digit g) of the 15 slots
+    const uint32_t bsel = (3u - (g & 3)) | ((7u - (g & 3)) << 4);
+#pragma unroll
+    for (int s = 0; s < 16; ++s) {
+      const int bb = s < 2 * NB ? s / 2 : s - 2 * NB, rr = s < 2 * NB ? s % 2 : 2;
+      xb[s] = 0u;
+      if (s < NS && (rr < 2 || t < 2)) {
+        const uint2 p = *reinterpret_cast<const uint2*>(&xw[q8][bb * N + 8 * rr + 2 * t]);
+        xb[s] = digit_pair<0>(__byte_perm(p.x, p.y, bsel));
+      }
+    }
+    const double x_own = __longlong_as_double((long long)v[0]), b_e = bv;   // x_own: lane < N
+    const int ee_e = ee;
+    if (e + stride < B) {   // in flight during the products
+      gather(e + stride);
+      nb = load_nb(e + 2 * stride);
+    }
+    // accumulators start at 1.5 * 2^23: their bits then are integers + kBias
+    constexpr float kStart = 12582912.0f;
+    constexpr int kBias = 0x4b400000;
+    float acc[10][4];
+#pragma unroll
+    for (int i = 0; i < 10; ++i)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[i][c] = kStart;
+#pragma unroll
+    for (int kt = 0; kt < 8; ++kt) {
+      if (kt == 0 || kt == 2 || kt == 4) wait();
+      const unsigned char* A = stage + (cc & 1) * kR64Stage;
+      uint32_t w[3][2][4];   // words of rows g, g + 8, 16 + g % 4 in the two slots
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int s = 2 * kt + h, s0 = kt < 4 ? 4 * (kt / 2) : 8;
+        const int o0 = s0 < 8 || s < 10 ? 1280 * (s - s0) : 2560 + 640 * (s - 10);
+        const bool on = s < NS && (s < 10 || t < 2);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const int row = i == 0 ? g : (i == 1 ? g + 8 : 16 + (g & 3));
+          uint4 a = make_uint4(kZeroDigits, kZeroDigits, kZeroDigits, kZeroDigits);
+          if (on) a = *reinterpret_cast<const uint4*>(A + o0 + (s < 10 ? 64 : 32) * row + 16 * t);
+          w[i][h][0] = a.x;
+          w[i][h][1] = a.y;
+          w[i][h][2] = a.z;
+          w[i][h][3] = a.w;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        mma_f16_16816(acc[2 * k], digit_pair<0>(w[0][0][k]), digit_pair<0>(w[1][0][k]), digit_pair<0>(w[0][1][k]),
+                      digit_pair<0>(w[1][1][k]), xb[2 * kt], xb[2 * kt + 1]);
+        mma_f16_16816(acc[2 * k + 1], digit_pair<1>(w[0][0][k]), digit_pair<1>(w[1][0][k]), digit_pair<1>(w[0][1][k]),
+                      digit_pair<1>(w[1][1][k]), xb[2 * kt], xb[2 * kt + 1]);
+      }
+#pragma unroll
+      for (int k = 0; k < 2; ++k)   // rows 16 ..: row g of the tile has digit 4 k + q8, row g + 8 digit 4 k + 2 + q8
+        mma_f16_16816(acc[8 + k], digit_sel(w[2][0][2 * k], tsel), digit_sel(w[2][0][2 * k + 1], tsel),
+                      digit_sel(w[2][1][2 * k], tsel), digit_sel(w[2][1][2 * k + 1], tsel), xb[2 * kt], xb[2 * kt + 1]);
+      if (kt == 1 || kt == 3 || kt == 7) done();
+    }
+    // P 2^32 + Q = sum_i acc_i 256^(7 - i) for a row and a digit j of x, added
+    // to (H, L) (value H + 2^-32 L) after a shift by 8 j
+    auto val = [&](float a) { return __float_as_int(a) - kBias; };
+    auto add = [&](long long Pv, long long Qv, int d, long long& H, unsigned long long& L) {
+      long long hi = Pv + (Qv >> 32);
+      uint32_t lo = (uint32_t)Qv;
+      if (t >= 2) {   // j >= 4
+        lo = (uint32_t)hi;
+        hi >>= 32;
+      }
+      const int sh = 8 * ((2 * t + d) & 3);
+      L += __funnelshift_r(lo, (uint32_t)hi, sh);
+      H += hi >> sh;
+    };
+    long long Hm[2] = {0, 0}, Ht = 0;
+    unsigned long long Lm[2] = {0, 0}, Lt = 0;
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {   // rows g, g + 8
+        const int c = 2 * q + d;
+        const int p0 = val(acc[0][c]) * 256 + val(acc[1][c]), p1 = val(acc[2][c]) * 256 + val(acc[3][c]);
+        const int p2 = val(acc[4][c]) * 256 + val(acc[5][c]), p3 = val(acc[6][c]) * 256 + val(acc[7][c]);
+        add((long long)p0 * 65536 + p1, (long long)p2 * 65536 + p3, d, Hm[q], Lm[q]);
+      }
+      const int ts = 256 >> (8 * q8);   // digits q8, q8 + 2: 256^3, 256 or 256^2, 1
+      add(((long long)val(acc[8][d]) * 65536 + val(acc[8][2 + d])) * ts,
+          ((long long)val(acc[9][d]) * 65536 + val(acc[9][2 + d])) * ts, d, Ht, Lt);
+    }
+    // over t: lanes t < 2 keep row g, the others row g + 8; rows 16 .. also
+    // over the two digit groups
+    long long Hs = (t & 2) ? Hm[1] : Hm[0];
+    unsigned long long Ls = (t & 2) ? Lm[1] : Lm[0];
+    Hs += __shfl_xor_sync(0xffffffffu, (t & 2) ? Hm[0] : Hm[1], 2);
+    Ls += __shfl_xor_sync(0xffffffffu, (t & 2) ? Lm[0] : Lm[1], 2);
+    Hs += __shfl_xor_sync(0xffffffffu, Hs, 1);
+    Ls += __shfl_xor_sync(0xffffffffu, Ls, 1);
+#pragma unroll
+    for (int o = 1; o <= 16; o = o == 2 ? 16 : 2 * o) {
+      Ht += __shfl_xor_sync(0xffffffffu, Ht, o);
+      Lt += __shfl_xor_sync(0xffffffffu, Lt, o);
+    }
+    const long long H = (t & 1) ? Ht : Hs, L = (long long)((t & 1) ? Lt : Ls);
+    if (mine) {
+      const double sc = dead || em == 2047 || ee_e == 0x7fff ? __longlong_as_double(0x7ff8000000000000ll)
+                                                             : exp2_int(ee_e + em - 1022 - 36);
+      const double res = fma(-sc, fma(int48_to_double(L), 0x1p-32, int48_to_double(H)), b_e);
+      if (r) r[e * N + m] = (flags & RF_NEG) ? -res : res;
+      rs[m] = res;
+    }
+    __syncwarp();
+    if (flags & RF_RESTRICT) {   // P3 -> P1 of the residual: corner t, nodes g, g + 8, g + 16
+      double s = P[g * F + t] * rs[g];
+      s = fma(P[(g + 8) * F + t], rs[g + 8], s);
+      if (g < 4) s = fma(P[(g + 16) * F + t], rs[g + 16], s);
+#pragma unroll
+      for (int o = 16; o >= 4; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (g == 0) r1[e * F + t] = s;
+    }
+    if (smooth) {
+      wait();
+      if (lane < N) {
+        const double* We = reinterpret_cast<const double*>(stage + (cc & 1) * kR64Stage) + lane;
+        double c = 0.0;
+#pragma unroll
+        for (int n = 0; n < N; ++n) c = fma(We[n * N], rs[n], c);
+        x_out[e * N + lane] = x_own + c;
+      }
+      done();
+    }
+  }
+  if (dead && lane == 0)   // this warp's copies in flight, bounded
+    for (int c = cc; c < cn; ++c) (void)mbar_wait_bounded(&bar[c & 1], (uint32_t)((c >> 1) & 1));
+}
+
 // partial[blk * 64 + q] = this block's slice of |z_q|^2, z (nrhs, n)
 // RHS-major; grid (blocks, nrhs)
 __global__ void __launch_bounds__(256) bnorm64_kernel(const double* __restrict__ z, int64_t n,
@@ -298,16 +564,24 @@ __global__ void __launch_bounds__(256) bnorm64_kernel(const double* __restrict__
   }
 }
 
-// block digits of the current operator build (3D), formed on first use and
-// kept with the context
+// Block digits of the current operator build (3D), kept with the context.
+// They take as much memory as the FP64 blocks: where that cannot be had
+// (DG_ERR_ALLOC, no error left behind) the callers keep to the FP64 pipe.
 int ensure_digits(dg_ctx* c, cudaStream_t st) {
   if (c->dig_version == c->build_version) return DG_OK;
-  int rc;
-  if (!c->d_adig && (rc = dalloc(c, &c->d_adig, (size_t)c->B * kDigElem))) return rc;
-  if (!c->d_aexp && (rc = dalloc(c, &c->d_aexp, (size_t)c->B * 20))) return rc;
+  if ((!c->d_adig && dalloc(c, &c->d_adig, (size_t)c->B * kDigElem)) ||
+      (!c->d_aexp && dalloc(c, &c->d_aexp, (size_t)c->B * 20))) {
+    cudaGetLastError();
+    c->err.clear();
+    return DG_ERR_ALLOC;
+  }
   if (c->B > 0) block_digits_kernel<<<(unsigned)c->B, 128, 0, st>>>(c->d_blk, c->d_adig, c->d_aexp);
   bump();
   CKL(c);
+  // not a kernel: a product started next reads the digits before its
+  // programmatic-launch wait
+  CK(c, cudaMemsetAsync(c->d_part, 0, sizeof(double), st));
+  CK(c, cudaFuncSetAttribute(res64_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kR64Smem));
   c->dig_version = c->build_version;
   return DG_OK;
 }

@@ -125,6 +125,11 @@ struct dg_ctx {
   unsigned char* d_adig = nullptr;
   int* d_aexp = nullptr;
   int dig_version = -1;
+  // single-RHS FP64 products take the digits: always after a quadrature build
+  // (which forms them, 0.3 of 12 ms at 48,000 tetrahedra), inside dg_gmres
+  // after an affine one (made per request, where a copy of 0.3 ms would save
+  // four products 0.05 ms each)
+  bool dig_single = false;
   double* d_detw = nullptr;
   int* d_err = nullptr;
   // boundary faces for the right-hand side
@@ -310,6 +315,7 @@ struct dg_ctx {
   cudaGraphExec_t arnoldi_exec = nullptr;
   int arnoldi_m = 0;
   int arnoldi_ortho = 0;
+  bool arnoldi_dig = false;
   const double* arnoldi_vptr = nullptr;
   // mixed-precision state (dg_mixed.cuh) and operator versions
   void* mixed_state = nullptr;
@@ -375,9 +381,8 @@ inline unsigned nblk(int64_t n, int tb) { return (unsigned)((n + tb - 1) / tb); 
 
 // Launch on st, as a programmatic dependent launch when c->use_pdl (the
 // kernel's launch overlaps the tail of the preceding kernel; its
-// pdl_wait_then_trigger() keeps the data order).  Used for the chains of
-// kernels of an Arnoldi step; every kernel launched with it starts with that
-// wait.
+// pdl_wait_then_trigger() keeps the data order).  Used for the chain of
+// kernels of a mixed inner Arnoldi step.
 template <typename... KArgs, typename... Args>
 int launch_k(dg_ctx* c, void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
              Args... args) {
@@ -394,6 +399,21 @@ int launch_k(dg_ctx* c, void (*kern)(KArgs...), unsigned grid, unsigned block, s
   cfg.numAttrs = c->use_pdl ? 1 : 0;
   CK(c, cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
   bump();
+  return DG_OK;
+}
+
+// Plain launch.  The FP64 chain and the triangles' block products take it:
+// with programmatic dependent launches the FP64 GMRES was slower at every
+// size (2,048 triangles 5.24 -> 5.49 ms; 3,072 / 10,368 / 48,000 tetrahedra
+// 15.1 -> 19.4, 36.5 -> 43.0, 120.9 -> 131.1 ms), the mixed solve on 97 x 61 x 2
+// triangles 3.00 -> 3.28 ms with them on its block products.
+template <typename... KArgs, typename... Args>
+int launch_p(dg_ctx* c, void (*kern)(KArgs...), dim3 grid, unsigned block, size_t smem, cudaStream_t st,
+             Args... args) {
+  if (grid.x == 0 || grid.y == 0) return DG_OK;
+  kern<<<grid, block, smem, st>>>(static_cast<KArgs>(args)...);
+  bump();
+  CKL(c);
   return DG_OK;
 }
 
@@ -428,6 +448,13 @@ template <>
 struct Elem<2> {
   static constexpr int N = 10, F = 3, VG = 12, SG = 4, NC = 3, EPB = 16;
 };
+
+}  // namespace
+
+#include "dg_async.cuh"
+#include "dg_fp64_mma.cuh"
+
+namespace {
 
 // SFC level values from the Galerkin values: entry d is the sum of
 // rar[vk[j]] for j in [vptr[d], vptr[d+1]), left to right (the host
@@ -635,7 +662,13 @@ int launch_residual(dg_ctx* c, const double* x, const double* b, double* r, doub
     int rc;
     if ((rc = ensure_w64_t<D>(c, st))) return rc;
   }
-  return launch_k(c, residual_kernel<E::N, E::F, E::EPB>, nblk(c->B, E::EPB), E::EPB * E::N, 0, st,
+  // tetrahedra: the product from the digit copy
+  if (D == 3 && c->dig_single && c->dig_version == c->build_version && !(flags & RF_ZEROX))
+    return launch_p(c, res64_mma_kernel, (unsigned)std::min<int64_t>(nblk(c->B, kR64Warps), 2 * c->nsm),
+                    32 * kR64Warps, kR64Smem, st, (const unsigned char*)c->d_adig,
+                    (const int*)c->d_aexp, (const double*)c->d_W, (const int*)c->d_nbe, x, b, r, x_out, (int64_t)c->B,
+                    flags, (const double*)c->T.P, r1);
+  return launch_p(c, residual_kernel<E::N, E::F, E::EPB>, nblk(c->B, E::EPB), E::EPB * E::N, 0, st,
                   (const double*)c->d_blk, (const double*)c->d_W, (const int*)c->d_nbe, x, b, r, x_out, (int64_t)c->B,
                   flags, (const double*)c->T.P, r1, (const float*)nullptr);
 }
@@ -651,7 +684,7 @@ int residual(dg_ctx* c, const double* x, const double* b, double* r, double* x_o
 // vertex gather of the element restrictions r1 (curve order when sfc_order)
 template <typename T>
 int gather_cg(dg_ctx* c, const T* r1, T* out, bool sfc_order, cudaStream_t st) {
-  return launch_k(c, gather_cg_kernel<T>, nblk(c->ncg, 128), 128, 0, st, r1, (const int*)c->d_gptr,
+  return launch_p(c, gather_cg_kernel<T>, nblk(c->ncg, 128), 128, 0, st, r1, (const int*)c->d_gptr,
                   (const int*)c->d_gent, (const double*)c->d_wdg, (const int*)(sfc_order ? c->d_pos : nullptr), out,
                   (int)c->ncg);
 }
@@ -691,7 +724,7 @@ int prolong_cg(dg_ctx* c, double* x, const double* ecg, bool sfc_order, int colo
 template <int D>
 int launch_prolong_add(dg_ctx* c, double* x, const double* e_sfc, cudaStream_t st) {
   using E = Elem<D>;
-  return launch_k(c, prolong_add_kernel<E::N, E::NC, E::EPB>, nblk(c->B, E::EPB), E::EPB * E::N, 0, st, x, e_sfc,
+  return launch_p(c, prolong_add_kernel<E::N, E::NC, E::EPB>, nblk(c->B, E::EPB), E::EPB * E::N, 0, st, x, e_sfc,
                   (const int*)c->d_pos, (const int*)c->d_p1cg, (const double*)c->d_wdg, (const double*)c->T.P,
                   (int64_t)c->B);
 }
@@ -821,11 +854,11 @@ int vcycle(dg_ctx* c, const double* r_sfc, cudaStream_t st) {
       double* keep = it == npre ? L.rr : nullptr;
       if (it == 0 && l > 0) {
         const DevLevel& P = c->lev[l - 1];
-        rc = launch_k(c, lev_jacobi_x_kernel<1, double>, g, TB, 0, st, (const int*)L.rowptr, (const int*)L.col,
+        rc = launch_p(c, lev_jacobi_x_kernel<1, double>, g, TB, 0, st, (const int*)L.rowptr, (const int*)L.col,
                       (const double*)L.val, (const double*)L.diag, (const double*)P.e, (const double*)P.rr,
                       (const int*)nullptr, P.n, L.r, L.e2, keep, L.n, w);
       } else {
-        rc = launch_k(c, lev_jacobi_kernel<double>, g, TB, 0, st, (const int*)L.rowptr, (const int*)L.col,
+        rc = launch_p(c, lev_jacobi_kernel<double>, g, TB, 0, st, (const int*)L.rowptr, (const int*)L.col,
                       (const double*)L.val, (const double*)L.diag, (const double*)(it == 0 ? nullptr : L.e), rhs_of(l),
                       L.e2, keep, L.n, w);
       }
@@ -838,7 +871,7 @@ int vcycle(dg_ctx* c, const double* r_sfc, cudaStream_t st) {
     const int ncol = l0 > 0 ? 2 * L.n : L.n;
     const double* fr = l0 > 0 ? c->lev[l0 - 1].rr : r_sfc;
     const double* fe = l0 > 0 ? c->lev[l0 - 1].e : nullptr;
-    if ((rc = launch_k(c, dense_tail64_kernel, nblk(L.n, 8), 256, sizeof(double) * c->tail_ld, st,
+    if ((rc = launch_p(c, dense_tail64_kernel, nblk(L.n, 8), 256, sizeof(double) * c->tail_ld, st,
                        (const double*)c->d_tail, c->tail_ld, fr, fe, l0 > 0 ? c->lev[l0 - 1].n : 0, L.e, L.n, ncol)))
       return rc;
   }
@@ -846,16 +879,16 @@ int vcycle(dg_ctx* c, const double* r_sfc, cudaStream_t st) {
     DevLevel& L = c->lev[l];
     const double* enext = c->lev[l + 1].e;
     const unsigned g = nblk((int64_t)L.n * LPR, TB);
-    if (npost == 0 && (rc = launch_k(c, lev_prolong_kernel<double>, nblk(L.n, TB), TB, 0, st, L.e, enext,
+    if (npost == 0 && (rc = launch_p(c, lev_prolong_kernel<double>, nblk(L.n, TB), TB, 0, st, L.e, enext,
                                      (const int*)L.up, L.n)))
       return rc;
     for (int it = 0; it < npost; ++it) {
       if (it == 0)
-        rc = launch_k(c, lev_jacobi_x_kernel<2, double>, g, TB, 0, st, (const int*)L.rowptr, (const int*)L.col,
+        rc = launch_p(c, lev_jacobi_x_kernel<2, double>, g, TB, 0, st, (const int*)L.rowptr, (const int*)L.col,
                       (const double*)L.val, (const double*)L.diag, (const double*)L.e, enext, (const int*)L.up, 0,
                       const_cast<double*>(rhs_of(l)), L.e2, (double*)nullptr, L.n, w);
       else
-        rc = launch_k(c, lev_jacobi_kernel<double>, g, TB, 0, st, (const int*)L.rowptr, (const int*)L.col,
+        rc = launch_p(c, lev_jacobi_kernel<double>, g, TB, 0, st, (const int*)L.rowptr, (const int*)L.col,
                       (const double*)L.val, (const double*)L.diag, (const double*)L.e, rhs_of(l), L.e2,
                       (double*)nullptr, L.n, w);
       if (rc) return rc;
@@ -984,21 +1017,21 @@ int cgs2(dg_ctx* c, int j, double* z, int m, cudaStream_t st) {
     double* part_n = c->d_part + (size_t)(1 - pass) * c->nred * KMAXV;
     for (int off = 0; off < nv; off += KMAXV) {
       const int cnt = std::min(KMAXV, nv - off);
-      if ((rc = launch_k2(c, mdot8_f64_kernel<RED_TB>, dim3(nb, (cnt + 7) / 8), RED_TB, 0, st,
+      if ((rc = launch_p(c, mdot8_f64_kernel<RED_TB>, dim3(nb, (cnt + 7) / 8), RED_TB, 0, st,
                           (const double*)(c->d_V + (size_t)off * c->nonods), (int64_t)c->nonods, cnt, (const double*)z,
                           n2, part)))
         return rc;
-      if (!fuse && (rc = launch_k(c, reduce_partial_kernel, cnt, 128, 0, st, (const double*)part, nb, cnt, h + off, 0, 0)))
+      if (!fuse && (rc = launch_p(c, reduce_partial_kernel, cnt, 128, 0, st, (const double*)part, nb, cnt, h + off, 0, 0)))
         return rc;
     }
-    if ((rc = launch_k(c, axpy8_f64_kernel<RED_TB>, nb, RED_TB, 0, st, (const double*)c->d_V, (int64_t)c->nonods, nv,
+    if ((rc = launch_p(c, axpy8_f64_kernel<RED_TB>, nb, RED_TB, 0, st, (const double*)c->d_V, (int64_t)c->nonods, nv,
                        (const double*)h, z, n2, part_n, pass, (const double*)part, fuse ? nb : 0, h)))
       return rc;
   }
-  if ((rc = launch_k(c, cgs_finish64_kernel, 1, 128, 0, st, (const double*)c->d_part, nb, (const double*)c->d_h1,
+  if ((rc = launch_p(c, cgs_finish64_kernel, 1, 128, 0, st, (const double*)c->d_part, nb, (const double*)c->d_h1,
                      (const double*)c->d_h2, nv, Hc, inv)))
     return rc;
-  return launch_k(c, scale2_f64_kernel, nblk(n2, 256), 256, 0, st, (const double*)z, (const double*)inv,
+  return launch_p(c, scale2_f64_kernel, nblk(n2, 256), 256, 0, st, (const double*)z, (const double*)inv,
                   c->d_V + (size_t)nv * c->nonods, n2);
 }
 
@@ -1042,7 +1075,8 @@ int arnoldi_steps(dg_ctx* c, int m, cudaStream_t st) {
 
 int run_arnoldi(dg_ctx* c, int m, cudaStream_t st) {
   if (!c->use_graph) return arnoldi_steps(c, m, st);
-  if (!c->arnoldi_exec || c->arnoldi_m != m || c->arnoldi_vptr != c->d_V || c->arnoldi_ortho != c->gmres_ortho) {
+  if (!c->arnoldi_exec || c->arnoldi_m != m || c->arnoldi_vptr != c->d_V || c->arnoldi_ortho != c->gmres_ortho ||
+      c->arnoldi_dig != c->dig_single) {
     if (c->arnoldi_exec) {
       cudaGraphExecDestroy(c->arnoldi_exec);
       c->arnoldi_exec = nullptr;
@@ -1066,6 +1100,7 @@ int run_arnoldi(dg_ctx* c, int m, cudaStream_t st) {
     c->arnoldi_m = m;
     c->arnoldi_vptr = c->d_V;
     c->arnoldi_ortho = c->gmres_ortho;
+    c->arnoldi_dig = c->dig_single;
   }
   CK(c, cudaGraphLaunch(c->arnoldi_exec, st));
   bump(c->arnoldi_kernels);
@@ -1112,7 +1147,6 @@ int read_scalar(dg_ctx* c, const double* d, double* h, cudaStream_t st) {
 
 }  // namespace
 
-#include "dg_fp64_mma.cuh"
 #include "dg_mixed.cuh"
 #include "dg_batched.cuh"
 
@@ -1536,6 +1570,11 @@ int dg_build_operator(dg_ctx* c, void* stream) {
   if (c->d_geom) c->geom_ok = true;
   c->built = true;   // blocks are usable from here on (the probes below apply them)
   ++c->build_version;
+  c->dig_single = false;
+  if (c->D == 3 && (c->fast_build != 1 || c->general_build)) {
+    if ((rc = ensure_digits(c, st)) && rc != DG_ERR_ALLOC) return rc;
+    c->dig_single = rc == DG_OK;
+  }
   // colour-probe Galerkin operator on P1CG (volume_mf_diff.py:1696-1754), or
   // the same product formed directly from the blocks
   CK(c, cudaMemsetAsync(c->d_rar, 0, sizeof(double) * c->cola.size(), st));
@@ -1893,6 +1932,15 @@ int dg_gmres(dg_ctx* c, double* x, const double* b, double tol, int32_t m, int32
   CK(c, cudaSetDevice(c->dev));
   int rc;
   if ((rc = ensure_krylov(c, m)) || (rc = ensure_tail64(c, st))) return rc;
+  struct DigGuard {   // products from the digits for the length of this call
+    dg_ctx* c;
+    bool keep;
+    ~DigGuard() { c->dig_single = keep; }
+  } guard{c, c->dig_single};
+  if (c->D == 3) {
+    if ((rc = ensure_digits(c, st)) && rc != DG_ERR_ALLOC) return rc;
+    c->dig_single = rc == DG_OK;
+  }
   double* r = c->d_t1;
   double* w = c->d_t2;
   int its = 0;

@@ -6,7 +6,10 @@ b = A x rounded to FP64, b - A x is the products' own error (and half an ulp
 of b): its norm from the digit product has to be at most that of the FP64
 loop (dg_residual).  Vectors: N(0, 1); smooth; magnitudes spread over 12
 decades with zeros.  Meshes of 6 and 48 elements (boundary faces, one to
-several warps), 1 to 64 right-hand sides (groups of 16 with remainders)."""
+several warps), 1 to 64 right-hand sides (groups of 16 with remainders).
+
+The FP64 loop is that of an affine build, whose single products stay on it;
+a quadrature build's take the digits."""
 import numpy as np
 import pytest
 
@@ -17,12 +20,13 @@ from dg_nn_public_gb300 import element, mesh, sfc  # noqa: E402
 from dg_nn_public_gb300.solver import DGSolver, SolverConfig  # noqa: E402
 
 
-def _operator(n):
+def _operator(n, build="affine"):
     m = mesh.build_mesh("tet", n, seed=2)
     s = DGSolver(m, sfc.hilbert_sfc_order(m.cg_coords), SolverConfig(pre_smooth_its=2, post_smooth_its=2),
                  element.p3_element(3))
     s.set_kappa(np.exp(np.random.default_rng(1).standard_normal(m.nele)))
     s.set_face_kappa("harmonic")
+    s.set_build_mode(build)
     s.build_operator()
     A = np.empty((s.nonods, s.nonods))
     for j in range(s.nonods):
@@ -64,3 +68,53 @@ def test_batched_residual_nonfinite():
     with pytest.raises(Exception, match="non-finite"):
         s.solve_mixed_batched(x, torch.ones_like(x), 1e-10)
     s.close()
+
+
+def _loop(A, x, b):
+    """Norm of b - A x from an FP64 multiply-add chain per row, in column order."""
+    A, r = A.astype(np.float64), np.zeros_like(b)
+    cols = [np.nonzero(a)[0] for a in A]
+    for i, c in enumerate(cols):
+        acc = 0.0
+        for j in c:
+            acc += A[i, j] * x[j]
+        r[i] = b[i] - acc
+    return r
+
+
+@pytest.mark.parametrize("n", [1, 2])
+def test_single_product_flags(n):
+    """dg_residual from the digits: error against extended precision at most
+    the FP64 chain's, its smoothing step against the same step from that
+    residual (FP64 products of 20 terms: 1e-13 of the largest), the
+    preconditioner (restriction of the residual) against the affine build's
+    (blocks equal to 1e-13: 1e-10 of the largest)."""
+    s, A = _operator(n, "quadrature")
+    a = _operator(n, "affine")[0]
+    K, d = s.bdiag()
+    for kind in ("normal", "smooth", "spread"):
+        x = _vectors(s.nonods, 3, kind)[2]
+        b = (A @ x.astype(np.longdouble)).astype(np.float64)
+        xt, bt = torch.tensor(x, device="cuda:0"), torch.tensor(b, device="cuda:0")
+        r = s.residual(xt, bt)
+        chain = _loop(A, x, b)
+        print(kind, "digits / chain: %.3f" % (float(torch.linalg.norm(r)) / np.linalg.norm(chain)))
+        assert float(torch.linalg.norm(r)) <= np.linalg.norm(chain)
+        y = s.apply(xt)
+        assert torch.equal(y, -s.residual(xt, torch.zeros_like(xt)))
+        b2 = torch.tensor(_vectors(s.nonods, 5, "normal")[4], device="cuda:0") * float(y.abs().max())
+        out = torch.empty_like(xt)
+        r2 = s.residual(xt, b2, x_out=out, smooth=True).view(-1, 20)
+        c = torch.zeros_like(r2)
+        for _ in range(3):
+            c = c + (2.0 / 3.0) * (r2 - torch.bmm(K, c.unsqueeze(2)).squeeze(2)) / d
+        ref = xt.view(-1, 20) + (2.0 / 3.0) * c
+        assert float(torch.abs(out.view(-1, 20) - ref).max()) <= 1e-13 * float(torch.abs(ref).max())
+    f = torch.tensor(_vectors(s.nonods, 3, "normal")[1], device="cuda:0")
+    z, za = s.precond(f), a.precond(f)
+    assert float(torch.abs(z - za).max()) <= 1e-10 * float(torch.abs(za).max())
+    x = torch.zeros_like(f)
+    x[5] = float("nan")
+    assert not bool(torch.isfinite(s.residual(x, f)).all())
+    s.close()
+    a.close()
