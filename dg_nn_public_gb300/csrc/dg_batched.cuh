@@ -2007,7 +2007,7 @@ extern "C" int dg_solve_mixed_batched(dg_ctx* c, double* x, const double* b, int
             std::vector<double> Hq(Hh.begin() + (size_t)q * (m + 1) * m, Hh.begin() + (size_t)(q + 1) * (m + 1) * m);
             std::vector<double> yq;
             bool ok = true;
-            const double est = hessenberg_ls(Hq, m, k, nrm[q], yq, ok);
+            const double est = hessenberg_ls(Hq.data(), m, k, nrm[q], yq, ok);
             if (!ok || !(est <= target[q] * beta0[q])) {
               all = false;
               int need = 5;
@@ -2031,7 +2031,7 @@ extern "C" int dg_solve_mixed_batched(dg_ctx* c, double* x, const double* b, int
         std::vector<double> Hq(Hh.begin() + (size_t)q * (m + 1) * m, Hh.begin() + (size_t)(q + 1) * (m + 1) * m);
         std::vector<double> yq;
         bool ok = true;
-        const double est = hessenberg_ls(Hq, m, k, nrm[q], yq, ok);
+        const double est = hessenberg_ls(Hq.data(), m, k, nrm[q], yq, ok);
         if (!ok) {
           active[q] = 0;   // breakdown of this RHS: keep its current iterate
           continue;
@@ -2170,10 +2170,7 @@ extern "C" int dg_set_batched_kernel(dg_ctx* c, int32_t variant) {
     c->batched_pinned = true;
   }
   Mixed& M = mixed_of(c);
-  for (auto& g : M.graphs)
-    if (g) cudaGraphExecDestroy(g);
-  M.graphs.clear();
-  M.g_m = 0;
+  drop_graphs(M);
   return DG_OK;
 }
 
