@@ -17,6 +17,7 @@ namespace dg {
 
 struct Tables {
   const double* n;        // (N, VG)
+  const double* mass;     // (N, N) sum_g weight_g n_m n_n
   const double* nlx;      // (D, N, VG)
   const double* weight;   // (VG)
   const double* sn;       // (F, N, SG)

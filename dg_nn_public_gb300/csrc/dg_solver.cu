@@ -131,6 +131,7 @@ struct dg_ctx {
   // four products 0.05 ms each)
   bool dig_single = false;
   double* d_detw = nullptr;
+  double w0 = 0.0;            // weight[0] of the element quadrature
   int* d_err = nullptr;
   // boundary faces for the right-hand side
   int nbf = 0;
@@ -653,6 +654,32 @@ int ensure_w64_t(dg_ctx* c, cudaStream_t st) {
 }
 
 int ensure_w64(dg_ctx* c, cudaStream_t st) { return c->D == 3 ? ensure_w64_t<3>(c, st) : ensure_w64_t<2>(c, st); }
+
+// Elements a block of the right-hand-side kernels (320 threads)
+template <int D>
+constexpr int kRhsElements = D == 3 ? 16 : 32;
+
+template <int D>
+int launch_rhs(dg_ctx* c, const double* f, const double* g, const double* gn, double* b, cudaStream_t st) {
+  using E = Elem<D>;
+  if (c->B > 0) {
+    constexpr int EPB = kRhsElements<D>;
+    rhs_mass_kernel<E::N, E::VG, EPB>
+        <<<(unsigned)std::min<int64_t>(nblk(c->B, EPB), 4 * (int64_t)c->nsm), EPB * E::N, 0, st>>>(
+            c->T.n, c->T.mass, c->T.weight, c->w0 != 0.0 ? 1.0 / c->w0 : 0.0, c->d_detw, f, b, c->B);
+    bump();
+    CKL(c);
+  }
+  if (c->nbf > 0 && (g || gn)) {
+    constexpr int FPB = kRhsElements<D> / 2;
+    rhs_bface_kernel<E::N, E::SG, E::F, FPB><<<nblk(c->nbf, FPB), FPB * E::N, 0, st>>>(
+        c->T.sn, c->d_bf_elem, c->d_bf_face, c->d_bf_type, c->d_bf_sw, c->d_bf_gn, c->d_bf_gam, c->d_kappa, g, gn, b,
+        c->nbf, c->cfg.mu_f);
+    bump();
+    CKL(c);
+  }
+  return DG_OK;
+}
 
 template <int D>
 int launch_residual(dg_ctx* c, const double* x, const double* b, double* r, double* x_out, int flags,
@@ -1348,6 +1375,7 @@ int dg_create(const dg_mesh_desc* m, const dg_config* cfg, dg_ctx** out) {
     }
   }
   c->nbf = (int)c->bf_elem.size();
+  c->w0 = m->weight[0];
   c->p1cg.assign(m->p1cg, m->p1cg + c->B * c->NC);
   c->sfc.assign(m->sfc_order, m->sfc_order + c->ncg);
   for (int64_t v : c->p1cg)
@@ -1397,6 +1425,15 @@ int dg_create(const dg_mesh_desc* m, const dg_config* cfg, dg_ctx** out) {
     double* p;
     if ((rc = upload(c.get(), &p, m->n, (size_t)N * VG))) return rc;
     c->T.n = p;
+    std::vector<double> mass((size_t)N * N);
+    for (int i = 0; i < N; ++i)
+      for (int j = 0; j < N; ++j) {
+        double t = 0.0;
+        for (int g = 0; g < VG; ++g) t += m->weight[g] * m->n[i * VG + g] * m->n[j * VG + g];
+        mass[(size_t)i * N + j] = t;
+      }
+    if ((rc = upload(c.get(), &p, mass.data(), mass.size()))) return rc;
+    c->T.mass = p;
     if ((rc = upload(c.get(), &p, m->nlx, (size_t)D * N * VG))) return rc;
     c->T.nlx = p;
     if ((rc = upload(c.get(), &p, m->weight, (size_t)VG))) return rc;
@@ -1852,33 +1889,8 @@ int dg_apply(dg_ctx* c, const double* x, double* y, void* stream) {
 int dg_rhs(dg_ctx* c, const double* f, const double* g, const double* gn, double* b, void* stream) {
   if (!c || !f || !b) return set_thread_error(DG_ERR_ARG, "dg_rhs: null argument");
   if (!c->built) return fail(c, DG_ERR_STATE, "dg_rhs: operator not built");
-  cudaStream_t st = S(stream);
   CK(c, cudaSetDevice(c->dev));
-  if (c->D == 3) {
-    using E = Elem<3>;
-    rhs_mass_kernel<E::N, E::VG, E::EPB><<<nblk(c->B, E::EPB), E::EPB * E::N, 0, st>>>(c->T.n, c->d_detw, f, b, c->B); bump();
-  } else {
-    using E = Elem<2>;
-    rhs_mass_kernel<E::N, E::VG, E::EPB><<<nblk(c->B, E::EPB), E::EPB * E::N, 0, st>>>(c->T.n, c->d_detw, f, b, c->B); bump();
-  }
-  CKL(c);
-  for (int mode = 0; mode < 2; ++mode) {
-    const double* src = mode == 0 ? g : gn;
-    if (!src || c->nbf == 0) continue;
-    for (int fsel = 0; fsel < c->F; ++fsel) {
-      if (c->D == 3)
-        rhs_bface_kernel<20, 12><<<nblk(c->nbf, 8), 8 * 20, 0, st>>>(
-            c->T.sn, c->d_bf_elem, c->d_bf_face, c->d_bf_type, c->d_bf_sw, c->d_bf_gn, c->d_bf_gam, c->d_kappa, src,
-            b, c->nbf, fsel, mode, c->cfg.mu_f);
-      else
-        rhs_bface_kernel<10, 4><<<nblk(c->nbf, 16), 16 * 10, 0, st>>>(
-            c->T.sn, c->d_bf_elem, c->d_bf_face, c->d_bf_type, c->d_bf_sw, c->d_bf_gn, c->d_bf_gam, c->d_kappa, src,
-            b, c->nbf, fsel, mode, c->cfg.mu_f);
-      bump();
-      CKL(c);
-    }
-  }
-  return DG_OK;
+  return c->D == 3 ? launch_rhs<3>(c, f, g, gn, b, S(stream)) : launch_rhs<2>(c, f, g, gn, b, S(stream));
 }
 
 int dg_precond(dg_ctx* c, const double* r, double* z, void* stream) {
