@@ -22,7 +22,8 @@ LIB = os.path.join(LIBDIR, "libdgsip.so")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 SOURCES = ["dg_host.cpp", "dg_serve.cpp", "dg_solver.cu"]
 HEADERS = ["dg_internal.h", "dg_kernels.cuh", "dg_kernels2.cuh", "dg_mixed.cuh", "dg_batched.cuh", "dg_batched_tc.cuh",
-           "dg_batched_warp.cuh", "dg_async.cuh", "dg_fp64_mma.cuh", "dg_noalloc.cuh", "dg_vcycle_cluster.cuh"]
+           "dg_batched_warp.cuh", "dg_async.cuh", "dg_fp64_mma.cuh", "dg_noalloc.cuh", "dg_vcycle_cluster.cuh",
+           "dg_mixed2d.cuh"]
 
 
 def _nvcc() -> str:

@@ -49,6 +49,8 @@ struct Mixed {
   // scaled face blocks S_ef = W_e A_ef (BF16, chunked, four per element) and
   // c = W b of the current preconditioner application; sc = in use
   __nv_bfloat16* scblk16 = nullptr;
+  float* scblk32 = nullptr;   // triangles: FP32 scaled faces (sct: in use)
+  bool sct = false;
   float* chat = nullptr;
   bool sc = false;
   std::vector<Lev32> lev;
@@ -1209,6 +1211,12 @@ void destroy_mixed(dg_ctx* c) {
   c->mixed_state = nullptr;
 }
 
+}  // namespace
+
+#include "dg_mixed2d.cuh"
+
+namespace {
+
 template <int D>
 int launch_residual32(dg_ctx* c, const float* x, const float* b, float* r, float* x_out, int flags,
                       cudaStream_t st, const float* ws = nullptr) {
@@ -1220,6 +1228,7 @@ int launch_residual32(dg_ctx* c, const float* x, const float* b, float* r, float
       return launch_tma<float, 4, 2, 2, true>(c, A, M.W, x, b, r, x_out, flags, M.r1, st, M.sf, ws);
     return launch_tma<float, 4, 2, 3, false>(c, A, M.W, x, b, r, x_out, flags, M.r1, st, M.sf);
   }
+  if (D == 2 && !(flags & (RF_SMOOTH | RF_ZEROX))) return launch_tri_residual(c, M.blk, x, b, r, flags, M.r1, st);
   return launch_p(c, residual_kernel<E::N, E::F, E::EPB, float, float, float>, nblk(c->B, E::EPB), E::EPB * E::N, 0,
                   st, (const float*)M.blk, (const float*)M.W, (const int*)c->d_nbe, x, b, r, x_out, (int64_t)c->B,
                   flags, (const double*)c->T.P, M.r1, ws);
@@ -1760,6 +1769,7 @@ int mixed_steps(const dg_ctx* c) {
 int smooth_step(dg_ctx* c, const float* x, const float* rhs, float* x_out, cudaStream_t st, const float* ws) {
   Mixed& M = mixed_of(c);
   if (M.sc) return launch_scaled(c, M.scblk16, x, rhs, x_out, st, ws);
+  if (M.sct) return launch_tri_scaled(c, M.scblk32, x, rhs, x_out, st, ws);
   return residual_pc(c, x, rhs, nullptr, x_out, RF_SMOOTH, st, ws);
 }
 
@@ -1777,10 +1787,12 @@ int precond32(dg_ctx* c, const float* r, float* z, cudaStream_t st) {
   };
   // scaled-face steps: the zero-start step also keeps c = W r, which every
   // later step reads in place of r
-  const float* rs = M.sc ? M.chat : r;
+  const float* rs = M.sc || M.sct ? M.chat : r;
   if (nsm > 0) {
     if (M.sc) {
       if ((rc = launch_bf16_tma(c, M, nullptr, r, nullptr, cur, RF_ZEROX | RF_SMOOTH, st, ws(0), M.chat))) return rc;
+    } else if (M.sct) {
+      if ((rc = launch_tri_zero_start(c, M.W, r, M.chat, cur, st, ws(0)))) return rc;
     } else if ((rc = residual_pc(c, nullptr, r, nullptr, cur, RF_ZEROX | RF_SMOOTH, st, ws(0)))) {
       return rc;
     }
@@ -1909,6 +1921,9 @@ int set_smoother_schedule(dg_ctx* c, cudaStream_t st) {
       if (M.sc) {   // W A v in one launch
         if ((rc = launch_scaled(c, M.scblk16, v, zb, u, st, nullptr, SC_APPLY))) return rc;
         std::swap(u, v);
+      } else if (M.sct) {
+        if ((rc = launch_tri_scaled(c, M.scblk32, v, zb, u, st, nullptr, SC_APPLY))) return rc;
+        std::swap(u, v);
       } else {
         if ((rc = smooth_step(c, v, zb, u, st, nullptr))) return rc;   // u = v - W A v
         sub_f32_kernel<<<nblk(n, 256), 256, 0, st>>>(v, u, v, n);       // v <- W A v
@@ -2018,6 +2033,12 @@ int build_mixed(dg_ctx* c, cudaStream_t st) {
     if (!M.scblk16 && (rc = dalloc(c, &M.scblk16, (size_t)c->B * 4 * 400))) return rc;
     if (!M.chat && (rc = dalloc(c, &M.chat, (size_t)c->nonods))) return rc;
   }
+  // scaled face blocks in FP32 on triangles, same condition on the smoother
+  M.sct = c->scaled_faces && c->D == 2 && c->mixed_smoother == 1;
+  if (M.sct) {
+    if (!M.scblk32 && (rc = dalloc(c, &M.scblk32, (size_t)c->B * 3 * 100))) return rc;
+    if (!M.chat && (rc = dalloc(c, &M.chat, (size_t)c->nonods))) return rc;
+  }
   if (one_pass) {
     const size_t nb = (size_t)c->B * (c->F + 1) * c->N * c->N;
     if (!M.blk && (rc = dalloc(c, &M.blk, nb))) return rc;
@@ -2075,6 +2096,11 @@ int build_mixed(dg_ctx* c, cudaStream_t st) {
     bump();
     CKL(c);
     vt("scaled face blocks");
+  }
+  if (M.sct && c->B > 0) {
+    tri_scaled_faces_kernel<<<(unsigned)c->B, 100, 0, st>>>(Wsrc32, c->d_blk, M.scblk32);
+    bump();
+    CKL(c);
   }
   if (M.lev.size() != c->lev.size()) {
     M.lev.assign(c->lev.size(), Lev32());
