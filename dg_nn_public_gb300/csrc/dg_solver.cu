@@ -37,10 +37,7 @@ struct DevLevel {
   int* vptr = nullptr;
   int* vk = nullptr;
   int* didx = nullptr;
-  // coarse levels (long lists: one device thread would sum thousands of
-  // values in sequence) keep their lists on the host and are summed there
-  bool host_sum = false;
-  std::vector<int> h_vptr, h_vk, h_didx;
+  int longest = 0;   // longest list; above kLongList the coarse-level kernel sums the level
   int* rowptr = nullptr;
   int* col = nullptr;
   double* val = nullptr;
@@ -327,7 +324,6 @@ struct dg_ctx {
   // the SFC level structure and summation lists are on the device: later
   // builds form the level values there (no RAR download, host sums, upload)
   bool lev_maps_ready = false;
-  double* rar_pinned = nullptr;   // pinned host copy of the Galerkin values (host-summed levels)
   // geometry record of the affine build (GeomRec), formed once per context;
   // geom_ok once a build that formed it passed the Jacobian check
   double* d_geom = nullptr;
@@ -474,6 +470,59 @@ __global__ void sfc_level_diag_kernel(const double* __restrict__ val, const int*
                                       double* __restrict__ diag) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) diag[i] = didx[i] >= 0 ? val[didx[i]] : 0.0;
+}
+
+// Levels with a list above kLongList: one thread would add up to all Galerkin
+// values in sequence, so a warp takes an entry, or, with a list above
+// kWideList, a CTA.  Lane-strided partial sums and a fixed reduction: the same
+// bits every time, the first build's included.  All such levels in one launch;
+// the diagonals in a second one (grid row = level).  Bound by the latency of
+// the gathers of the topmost level, whose one entry sums every value.  On host
+// threads, from a pinned copy, 2,197 vertices took 0.8 ms of a rebuild with the
+// copies: a request with new kappa there 6.48 -> 5.65 ms, 40.6 -> 39.7 on 24,389.
+constexpr int kLongList = 64, kWideList = 1024, kLongLevels = 24;
+struct LongLevels {
+  struct {
+    const int *vptr, *vk, *didx;
+    double *val, *diag;
+    int nnz, n, first, wide;   // first = the level's first CTA
+  } l[kLongLevels];
+  int cnt;
+};
+
+__global__ void __launch_bounds__(256) sfc_long_values_kernel(const double* __restrict__ rar, LongLevels p) {
+  int k = 0;
+  while (k + 1 < p.cnt && (int)blockIdx.x >= p.l[k + 1].first) ++k;
+  const auto& L = p.l[k];
+  __shared__ double red[8];
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  const int d = L.wide ? (int)blockIdx.x - L.first : ((int)blockIdx.x - L.first) * 8 + wid;
+  const int t0 = L.wide ? t : lane, step = L.wide ? 256 : 32;
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  if (d < L.nnz) {
+    const int j1 = L.vptr[d + 1];
+    int j = L.vptr[d] + t0;
+    for (; j + 3 * step < j1; j += 4 * step)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) s[u] += rar[L.vk[j + u * step]];
+    for (; j < j1; j += step) s[0] += rar[L.vk[j]];
+  }
+  double v = warp_sum((s[0] + s[1]) + (s[2] + s[3]));
+  if (L.wide) {   // uniform over the CTA
+    if (lane == 0) red[wid] = v;
+    __syncthreads();
+    v = t < 8 ? red[t] : 0.0;
+    if (wid == 0) v = warp_sum(v);
+    if (t == 0 && d < L.nnz) L.val[d] = v;
+  } else if (lane == 0 && d < L.nnz) {
+    L.val[d] = v;
+  }
+}
+
+__global__ void sfc_long_diag_kernel(LongLevels p) {
+  const auto& L = p.l[blockIdx.y];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < L.n; i += gridDim.x * blockDim.x)
+    L.diag[i] = L.didx[i] >= 0 ? L.val[L.didx[i]] : 0.0;
 }
 
 // FastTab of the element (host): the reference matrices, in the order that
@@ -654,6 +703,29 @@ int ensure_w64_t(dg_ctx* c, cudaStream_t st) {
 }
 
 int ensure_w64(dg_ctx* c, cudaStream_t st) { return c->D == 3 ? ensure_w64_t<3>(c, st) : ensure_w64_t<2>(c, st); }
+
+// values and diagonals of the levels with long lists
+int long_level_sums(dg_ctx* c, cudaStream_t st) {
+  for (size_t l = 0; l < c->lev.size();) {
+    LongLevels p;
+    p.cnt = 0;
+    int ctas = 0, rows = 1;
+    for (; l < c->lev.size() && p.cnt < kLongLevels; ++l) {
+      const DevLevel& L = c->lev[l];
+      if (L.longest <= kLongList) continue;
+      const int wide = L.longest > kWideList;
+      p.l[p.cnt++] = {L.vptr, L.vk, L.didx, L.val, L.diag, L.nnz, L.n, ctas, wide};
+      ctas += wide ? L.nnz : (L.nnz + 7) / 8;
+      rows = std::max(rows, L.n);
+    }
+    if (p.cnt == 0) continue;
+    sfc_long_values_kernel<<<(unsigned)ctas, 256, 0, st>>>(c->d_rar, p);
+    sfc_long_diag_kernel<<<dim3((unsigned)std::min((rows + 255) / 256, 4 * c->nsm), p.cnt), 256, 0, st>>>(p);
+    bump(2);
+  }
+  CKL(c);
+  return DG_OK;
+}
 
 // Elements a block of the right-hand-side kernels (320 threads)
 template <int D>
@@ -1195,7 +1267,6 @@ void dg_destroy(dg_ctx* ctx) {
   if (ctx->arnoldi_exec) cudaGraphExecDestroy(ctx->arnoldi_exec);
   destroy_mixed(ctx);
   if (ctx->cap_stream) cudaStreamDestroy(ctx->cap_stream);
-  if (ctx->rar_pinned) cudaFreeHost(ctx->rar_pinned);
   for (void* p : ctx->allocs) cudaFree(p);
   cudaSetDevice(cur);
   delete ctx;
@@ -1643,50 +1714,18 @@ int dg_build_operator(dg_ctx* c, void* stream) {
   SfcHierarchy& h = c->sfc_h;
   if (c->lev_maps_ready) {
     // SFC level values and diagonals from the Galerkin values, on the device,
-    // in the host builder's summation order (same bits)
+    // lists up to kLongList in the host builder's summation order (same bits)
     const double t_probes = ms_since(t0);
-    bool any_host = false;
     for (int l = 0; l < h.nlevel; ++l) {
       DevLevel& L = c->lev[l];
-      if (L.host_sum) {
-        any_host = true;
-        continue;
-      }
+      if (L.longest > kLongList) continue;
       if (L.nnz > 0)
         sfc_level_values_kernel<<<nblk(L.nnz, 256), 256, 0, st>>>(c->d_rar, L.vptr, L.vk, L.nnz, L.val);
       sfc_level_diag_kernel<<<nblk(L.n, 256), 256, 0, st>>>(L.val, L.didx, L.n, L.diag);
       bump(2);
     }
     CKL(c);
-    if (any_host) {
-      if (!c->rar_pinned) CK(c, cudaMallocHost((void**)&c->rar_pinned, sizeof(double) * c->cola.size()));
-      CK(c, cudaMemcpyAsync(c->rar_pinned, c->d_rar, sizeof(double) * c->cola.size(), cudaMemcpyDeviceToHost, st));
-      CK(c, cudaStreamSynchronize(st));
-      struct HV {
-        std::vector<double> val, diag;
-      };
-      std::vector<HV> hv(h.nlevel);
-      parallel_for(h.nlevel, [&](int l) {
-        const DevLevel& L = c->lev[l];
-        if (!L.host_sum) return;
-        HV& o = hv[l];
-        o.val.resize(L.nnz);
-        for (int d = 0; d < L.nnz; ++d) {
-          int j = L.h_vptr[d];
-          double sum = c->rar_pinned[L.h_vk[j]];
-          for (++j; j < L.h_vptr[d + 1]; ++j) sum += c->rar_pinned[L.h_vk[j]];
-          o.val[d] = sum;
-        }
-        o.diag.resize(L.n);
-        for (int i = 0; i < L.n; ++i) o.diag[i] = L.h_didx[i] >= 0 ? o.val[L.h_didx[i]] : 0.0;
-      });
-      for (int l = 0; l < h.nlevel; ++l) {
-        const DevLevel& L = c->lev[l];
-        if (!L.host_sum) continue;
-        CK(c, cudaMemcpyAsync(L.val, hv[l].val.data(), sizeof(double) * L.nnz, cudaMemcpyHostToDevice, st));
-        CK(c, cudaMemcpyAsync(L.diag, hv[l].diag.data(), sizeof(double) * L.n, cudaMemcpyHostToDevice, st));
-      }
-    }
+    if ((rc = long_level_sums(c, st))) return rc;
     CK(c, cudaStreamSynchronize(st));
     if (c->verbose)
       std::fprintf(stderr, "[dg_build_operator] ms: blocks %.2f, colour probes %.2f, SFC level values (device) %.2f\n",
@@ -1816,22 +1855,17 @@ int dg_build_operator(dg_ctx* c, void* stream) {
     L.nnz = (int)U.cl.size();
     int maxlen = 0;
     for (int d = 0; d < L.nnz; ++d) maxlen = std::max(maxlen, U.vptr[d + 1] - U.vptr[d]);
-    L.host_sum = maxlen > 64;
-    if (L.host_sum) {
-      L.h_vptr = U.vptr;
-      L.h_vk = U.vkl;
-      L.h_didx = U.didx;
-    } else {
-      if (!L.vptr) {
-        if ((rc = dalloc(c, &L.vptr, U.vptr.size()))) return rc;
-        if ((rc = dalloc(c, &L.vk, std::max<size_t>(U.vkl.size(), 1)))) return rc;
-        if ((rc = dalloc(c, &L.didx, std::max<size_t>(U.didx.size(), 1)))) return rc;
-      }
-      CK(c, cudaMemcpyAsync(L.vptr, U.vptr.data(), sizeof(int) * U.vptr.size(), cudaMemcpyHostToDevice, st));
-      CK(c, cudaMemcpyAsync(L.vk, U.vkl.data(), sizeof(int) * U.vkl.size(), cudaMemcpyHostToDevice, st));
-      CK(c, cudaMemcpyAsync(L.didx, U.didx.data(), sizeof(int) * U.didx.size(), cudaMemcpyHostToDevice, st));
+    L.longest = maxlen;
+    if (!L.vptr) {
+      if ((rc = dalloc(c, &L.vptr, U.vptr.size()))) return rc;
+      if ((rc = dalloc(c, &L.vk, std::max<size_t>(U.vkl.size(), 1)))) return rc;
+      if ((rc = dalloc(c, &L.didx, std::max<size_t>(U.didx.size(), 1)))) return rc;
     }
+    CK(c, cudaMemcpyAsync(L.vptr, U.vptr.data(), sizeof(int) * U.vptr.size(), cudaMemcpyHostToDevice, st));
+    CK(c, cudaMemcpyAsync(L.vk, U.vkl.data(), sizeof(int) * U.vkl.size(), cudaMemcpyHostToDevice, st));
+    CK(c, cudaMemcpyAsync(L.didx, U.didx.data(), sizeof(int) * U.didx.size(), cudaMemcpyHostToDevice, st));
   }
+  if ((rc = long_level_sums(c, st))) return rc;   // as later builds form them
   CK(c, cudaStreamSynchronize(st));
   c->lev_maps_ready = true;
   if (c->verbose)
