@@ -798,12 +798,13 @@ template <typename VT = double>
 __global__ void scale_kernel(const VT* __restrict__ z, const double* __restrict__ den,
                              VT* __restrict__ v, int64_t n) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
   if constexpr (sizeof(VT) == 8) {
-    v[k] = z[k] / (VT)(*den);
+    if (k < n) v[k] = z[k] / (VT)(*den);
   } else {
-    const VT inv = (VT)(1.0 / *den);
-    v[k] = z[k] * inv;
+    __shared__ VT inv;   // one FP64 division a CTA: a warp's takes the FP64 pipe as long as the CTA's loads
+    if (threadIdx.x == 0) inv = (VT)(1.0 / *den);
+    __syncthreads();
+    if (k < n) v[k] = z[k] * inv;
   }
 }
 

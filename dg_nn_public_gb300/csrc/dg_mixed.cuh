@@ -1260,37 +1260,40 @@ int residual_pc(dg_ctx* c, const float* x, const float* b, float* r, float* x_ou
   return residual32(c, x, b, r, x_out, flags, st, ws);
 }
 
-// P1 -> P3 prolongation of the coarse correction (mixed path, 3D):
-// x[e][n] += sum_c P[n][c] (w_ec ecg[pos(p1cg[e][c])]).  8 elements per CTA;
-// the 4 corner values of an element are formed once (threads m < 4) instead
-// of by each of its 20 node threads.  Same products and summation order as
-// prolong_cg_kernel.  The corner indices are fixed data, read before the
-// programmatic-launch wait.
-__global__ void __launch_bounds__(160) prolong_cg32_kernel(float* __restrict__ x, const float* __restrict__ ecg,
+// x[e][n] += sum_c P[n][c] (w_ec ecg[pos(p1cg[e][c])]) on tetrahedra: five
+// threads an element, four consecutive nodes each, so that x moves in 16-byte
+// pieces and the corner indices and weights in one load.  Same products and
+// summation order as prolong_cg_kernel.  Indices, weights and P are fixed
+// data, read before the programmatic-launch wait.  Bound by its three
+// dependent loads and, on large meshes, by HBM.  384,000 tetrahedra: with a
+// thread a node and the corner values through shared memory 51 us, now 24.
+__global__ void __launch_bounds__(320) prolong_cg32_kernel(float* __restrict__ x, const float* __restrict__ ecg,
                                                            const int* __restrict__ pos, const int* __restrict__ p1cg,
                                                            const float* __restrict__ wdg,
                                                            const float* __restrict__ P, int64_t B) {
-  __shared__ float vc[8][4];
-  const int le = threadIdx.x / 20, n = threadIdx.x % 20;
-  const int64_t e = (int64_t)blockIdx.x * 8 + le;
+  const int64_t k = (int64_t)blockIdx.x * 320 + threadIdx.x;   // float4 k of x
+  const int64_t e = k / 5;
+  const int n0 = (int)(k - e * 5) * 4;
   const bool valid = e < B;
-  int vp = 0;
-  float w = 0.0f;
-  if (valid && n < 4) {
-    vp = pos[p1cg[e * 4 + n]];
-    w = (float)wdg[e * 4 + n];
+  int4 vp = make_int4(0, 0, 0, 0);
+  float4 w = make_float4(0.f, 0.f, 0.f, 0.f), p[4];
+  if (valid) {
+    vp = __ldg(reinterpret_cast<const int4*>(p1cg) + e);
+    w = __ldg(reinterpret_cast<const float4*>(wdg) + e);
+    vp = make_int4(__ldg(pos + vp.x), __ldg(pos + vp.y), __ldg(pos + vp.z), __ldg(pos + vp.w));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) p[i] = __ldg(reinterpret_cast<const float4*>(P) + n0 + i);
   }
-  float p[4];
-#pragma unroll
-  for (int c2 = 0; c2 < 4; ++c2) p[c2] = (float)P[n * 4 + c2];
   pdl_wait_then_trigger();
-  if (valid && n < 4) vc[le][n] = w * ecg[vp];
-  __syncthreads();
   if (!valid) return;
-  float v = 0.0f;
-#pragma unroll
-  for (int c2 = 0; c2 < 4; ++c2) v += p[c2] * vc[le][c2];
-  x[e * 20 + n] += v;
+  const float4 v = make_float4(w.x * ecg[vp.x], w.y * ecg[vp.y], w.z * ecg[vp.z], w.w * ecg[vp.w]);
+  float4 o = reinterpret_cast<float4*>(x)[k];
+  auto dot = [&](const float4& q) { return fmaf(q.w, v.w, fmaf(q.z, v.z, fmaf(q.y, v.y, q.x * v.x))); };
+  o.x += dot(p[0]);
+  o.y += dot(p[1]);
+  o.z += dot(p[2]);
+  o.w += dot(p[3]);
+  reinterpret_cast<float4*>(x)[k] = o;
 }
 
 // vertex gather of the element P1 restrictions (mixed path): one warp per
@@ -1340,7 +1343,7 @@ int launch_transfer32(dg_ctx* c, const float* r, float* cg_out, float* x_add, co
   } else {
     int rc;
     if (D == 3)
-      rc = launch_k(c, prolong_cg32_kernel, nblk(c->B, 8), 160, 0, st, x_add, e_sfc, (const int*)c->d_pos,
+      rc = launch_k(c, prolong_cg32_kernel, nblk(c->B, 64), 320, 0, st, x_add, e_sfc, (const int*)c->d_pos,
                     (const int*)c->d_p1cg, (const float*)c->d_wdg32, (const float*)c->d_P32, (int64_t)c->B);
     else
       rc = launch_k(c, prolong_cg_kernel<E::N, E::NC, float>, nblk(c->B * E::N, 256), 256, 0, st, x_add, e_sfc,
@@ -2337,6 +2340,12 @@ __global__ void __launch_bounds__(TB) axpy8_f32_kernel(const float* __restrict__
   }
 }
 
+// Threads of the kernels that add nblk block sums: a thread's loads are
+// scattered (one sector each), so the sum is bound by how many a thread does
+// one after another.  7,500 blocks (384,000 tetrahedra): cgs_finish_kernel with
+// 256 threads 19 us, with 1,024 10 us.
+inline unsigned reduce_threads(int nblk) { return nblk > 512 ? 1024u : 256u; }
+
 // Hessenberg column j: Hc[i] = h1[i] (+ h2[i] when h2) for i < nv;
 // Hc[nv] = |z| = sqrt(sum of the norm partials); *inv = 1 / |z| in FP32.
 // One block, fixed summation order.
@@ -2523,7 +2532,7 @@ int mdot4_f32(dg_ctx* c, const float* V, int nv, const float* z, double* h, cuda
     if ((rc = launch_k2(c, mdot8_f32_kernel<RED_TB>, dim3(M.nblk4, (cnt + 7) / 8), RED_TB, 0, st,
                         (const float*)(V + (size_t)off * c->nonods), (int64_t)c->nonods, cnt, z, n4, M.part)))
       return rc;
-    if ((rc = launch_k(c, reduce_partial_kernel, cnt, 256, 0, st, (const double*)M.part, M.nblk4, cnt, h + off, 0,
+    if ((rc = launch_k(c, reduce_partial_kernel, cnt, reduce_threads(M.nblk4), 0, st, (const double*)M.part, M.nblk4, cnt, h + off, 0,
                        0)))
       return rc;
   }
@@ -2559,7 +2568,7 @@ int cgs2_32(dg_ctx* c, int j, float* w, int m, cudaStream_t st) {
     if ((rc = launch_k(c, axpy8_f32_kernel<RED_TB>, M.nblk4, RED_TB, 0, st, (const float*)M.V, (int64_t)c->nonods,
                        nv, (const double*)(two ? c->d_h2 : c->d_h1), w, n4, M.part, 1)))
       return rc;
-    if ((rc = launch_k(c, cgs_finish_kernel, 1, 256, 0, st, (const double*)M.part, M.nblk4, (const double*)c->d_h1,
+    if ((rc = launch_k(c, cgs_finish_kernel, 1, reduce_threads(M.nblk4), 0, st, (const double*)M.part, M.nblk4, (const double*)c->d_h1,
                        two ? (const double*)c->d_h2 : (const double*)nullptr, nv, Hc, inv)))
       return rc;
   }
