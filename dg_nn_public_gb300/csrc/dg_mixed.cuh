@@ -1812,7 +1812,7 @@ int precond32(dg_ctx* c, const float* r, float* z, cudaStream_t st) {
   } else if (M.dense_l > 0 && c->vc32_fused) {
     if ((rc = vcycle32_fused(c, st))) return rc;     // gather included
   } else {
-    float* cg_dst = M.dense_l > 0 ? M.lev[0].r : M.cg1;
+    float* cg_dst = M.dense_l >= 0 ? M.lev[0].r : M.cg1;
     if ((rc = launch_k(c, gather_cg32_kernel, nblk(c->ncg, 8), 256, 0, st, (const float*)M.r1,
                        (const int*)c->d_gptr, (const int*)c->d_gent, (const float*)c->d_wdg32, (const int*)c->d_pos,
                        cg_dst, (int)c->ncg, (const float*)nullptr, (float*)nullptr, (float*)nullptr, 0.0f)))
