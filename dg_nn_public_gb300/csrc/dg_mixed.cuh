@@ -1051,7 +1051,7 @@ __global__ void gj_update_kernel(double* __restrict__ G, int n, int k, const dou
 // itself: the steps are a chain of n / 32 launches and their latency is what
 // bounds the inverse (before, a step was four launches, 63 us at n = 1,100,
 // 40 us of it the one-CTA inverse of D, on an augmented matrix that the host
-// assembled and uploaded).
+// assembled and uploaded; now 16 us).
 constexpr int kGjB = 32;
 
 __global__ void __launch_bounds__(256) gjb_step_kernel(const float* __restrict__ A, float* __restrict__ B, int n,
@@ -2216,7 +2216,7 @@ int ensure_krylov32(dg_ctx* c, int m) {
   if ((rc = dalloc(c, &M.H, (size_t)(m + 1) * m))) return rc;
   if (!M.part) {
     M.nblk4 = (int)((c->nonods / 4 + RED_TB - 1) / RED_TB);
-    if ((rc = dalloc(c, &M.part, (size_t)std::max(M.nblk4, 1) * KMAXV))) return rc;
+    if ((rc = dalloc(c, &M.part, (size_t)std::max(M.nblk4, 1) * KMAXV * 2))) return rc;
     if ((rc = dalloc(c, &M.gs_cnt, 64))) return rc;
     CK(c, cudaMemset(M.gs_cnt, 0, sizeof(unsigned) * 64));
   }
@@ -2291,15 +2291,32 @@ __global__ void __launch_bounds__(TB) mdot8_f32_kernel(const float* __restrict__
 
 // z -= sum_i V[i] h[i] (nv <= 256); with want_norm also
 // partial[bx * KMAXV] = this block's slice of |z_new|^2 (FP32 within a warp,
-// FP64 across warps)
+// FP64 across warps).  With nred > 0 (nv <= KMAXV) h is formed here, as the sum
+// of the nred block sums partial_in, in the same order by every block; block 0
+// writes it to h_out.
 template <int TB>
 __global__ void __launch_bounds__(TB) axpy8_f32_kernel(const float* __restrict__ V, int64_t ld, int nv,
                                                        const double* __restrict__ h, float* __restrict__ z,
-                                                       int64_t n4, double* __restrict__ partial, int want_norm) {
+                                                       int64_t n4, double* __restrict__ partial, int want_norm,
+                                                       const double* __restrict__ partial_in, int nred,
+                                                       double* __restrict__ h_out) {
   pdl_wait_then_trigger();
   __shared__ float hs[256];
   __shared__ float red[TB / 32];
-  for (int i = threadIdx.x; i < nv; i += TB) hs[i] = (float)h[i];
+  if (nred > 0) {
+#pragma unroll 4
+    for (int i = threadIdx.x >> 5; i < nv; i += TB / 32) {
+      double s = 0.0;
+      for (int b = threadIdx.x & 31; b < nred; b += 32) s += partial_in[(int64_t)b * KMAXV + i];
+      s = warp_sum(s);
+      if ((threadIdx.x & 31) == 0) {
+        hs[i] = (float)s;
+        if (blockIdx.x == 0) h_out[i] = s;
+      }
+    }
+  } else {
+    for (int i = threadIdx.x; i < nv; i += TB) hs[i] = (float)h[i];
+  }
   __syncthreads();
   float acc = 0.0f;
   float4* z4 = reinterpret_cast<float4*>(z);
@@ -2383,6 +2400,38 @@ __global__ void scale4_f32_kernel(const float* __restrict__ z, const float* __re
   a.z *= s;
   a.w *= s;
   reinterpret_cast<float4*>(v)[k] = a;
+}
+
+// cgs_finish_kernel and scale4_f32_kernel in one launch for at most 256 block
+// sums: every CTA adds them (one load a thread, one fixed order), block 0 writes
+// the Hessenberg column.
+__global__ void __launch_bounds__(256) cgs_scale_f32_kernel(const double* __restrict__ partial, int nblk,
+                                                            const double* __restrict__ h1,
+                                                            const double* __restrict__ h2, int nv,
+                                                            double* __restrict__ Hc, const float* __restrict__ z,
+                                                            float* __restrict__ v, int64_t n4) {
+  pdl_wait_then_trigger();
+  __shared__ double red[8];
+  __shared__ float inv;
+  const int t = threadIdx.x;
+  const int64_t k = (int64_t)blockIdx.x * 256 + t;
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (k < n4) a = reinterpret_cast<const float4*>(z)[k];
+  const double s = warp_sum(t < nblk ? partial[(int64_t)t * KMAXV] : 0.0);
+  if ((t & 31) == 0) red[t >> 5] = s;
+  if (blockIdx.x == 0)
+    for (int i = t; i < nv; i += 256) Hc[i] = h2 ? h1[i] + h2[i] : h1[i];
+  __syncthreads();
+  if (t == 0) {
+    double q = 0.0;
+    for (int w = 0; w < 8; ++w) q += red[w];
+    q = sqrt(q);
+    if (blockIdx.x == 0) Hc[nv] = q;
+    inv = (float)(1.0 / q);
+  }
+  __syncthreads();
+  if (k < n4)
+    reinterpret_cast<float4*>(v)[k] = make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv);
 }
 
 // The same dots with the block reduction fused: each CTA writes its partial
@@ -2515,8 +2564,17 @@ __global__ void __launch_bounds__(TB) axpy8f_f32_kernel(const float* __restrict_
   }
 }
 
-// h[0..nv) = V^T z with the float4 kernels (nv <= KMAXV per call)
-int mdot4_f32(dg_ctx* c, const float* V, int nv, const float* z, double* h, cudaStream_t st) {
+// Up to kFoldBlocks block sums axpy8_f32_kernel adds those of the dots itself,
+// in every CTA, and up to 256 cgs_scale_f32_kernel those of |w|^2: a launch
+// costs an iteration about 2 us, the sums less than that while a warp adds at
+// most four (dots) or a thread one (norm).  Above, the separate kernels.
+// 3,072 tetrahedra (60 blocks) 2.22 -> 2.17 ms, 11,834 triangles (116) 2.28 ->
+// 2.25, a request on 10,368 tetrahedra (203, norm only) 5.65 -> 5.57.
+constexpr int kFoldBlocks = 128;
+
+// h[0..nv) = V^T z with the float4 kernels (nv <= KMAXV per call); fold: only
+// the block sums, in M.part (nv <= KMAXV)
+int mdot4_f32(dg_ctx* c, const float* V, int nv, const float* z, double* h, cudaStream_t st, bool fold) {
   const int64_t n4 = c->nonods / 4;
   for (int off = 0; off < nv; off += KMAXV) {
     const int cnt = std::min(KMAXV, nv - off);
@@ -2532,8 +2590,9 @@ int mdot4_f32(dg_ctx* c, const float* V, int nv, const float* z, double* h, cuda
     if ((rc = launch_k2(c, mdot8_f32_kernel<RED_TB>, dim3(M.nblk4, (cnt + 7) / 8), RED_TB, 0, st,
                         (const float*)(V + (size_t)off * c->nonods), (int64_t)c->nonods, cnt, z, n4, M.part)))
       return rc;
-    if ((rc = launch_k(c, reduce_partial_kernel, cnt, reduce_threads(M.nblk4), 0, st, (const double*)M.part, M.nblk4, cnt, h + off, 0,
-                       0)))
+    if (fold) continue;
+    if ((rc = launch_k(c, reduce_partial_kernel, cnt, reduce_threads(M.nblk4), 0, st, (const double*)M.part,
+                       M.nblk4, cnt, h + off, 0, 0)))
       return rc;
   }
   return DG_OK;
@@ -2550,26 +2609,37 @@ int cgs2_32(dg_ctx* c, int j, float* w, int m, cudaStream_t st) {
   double* Hc = M.H + (size_t)j * (m + 1);
   const bool two = c->mixed_cgs_passes != 1;
   float* inv = reinterpret_cast<float*>(c->d_scal + 1);
+  const bool fold = !c->gs_fused && nv <= KMAXV && M.nblk4 <= kFoldBlocks;
+  const int nred = fold ? M.nblk4 : 0;
+  double* npart = M.part + (size_t)M.nblk4 * KMAXV;   // block sums of |w|^2: M.part is still being read
+  auto update = [&](double* h, int want_norm) {
+    return launch_k(c, axpy8_f32_kernel<RED_TB>, M.nblk4, RED_TB, 0, st, (const float*)M.V, (int64_t)c->nonods, nv,
+                    (const double*)h, w, n4, npart, want_norm, (const double*)M.part, nred, h);
+  };
   int rc;
-  if ((rc = mdot4_f32(c, M.V, nv, w, c->d_h1, st))) return rc;
+  if ((rc = mdot4_f32(c, M.V, nv, w, c->d_h1, st, fold))) return rc;
   if (two) {
-    if ((rc = launch_k(c, axpy8_f32_kernel<RED_TB>, M.nblk4, RED_TB, 0, st, (const float*)M.V, (int64_t)c->nonods,
-                       nv, (const double*)c->d_h1, w, n4, M.part, 0)))
-      return rc;
-    if ((rc = mdot4_f32(c, M.V, nv, w, c->d_h2, st))) return rc;
+    if ((rc = update(c->d_h1, 0))) return rc;
+    if ((rc = mdot4_f32(c, M.V, nv, w, c->d_h2, st, fold))) return rc;
   }
+  double* hl = two ? c->d_h2 : c->d_h1;
+  const double* h2 = two ? c->d_h2 : nullptr;
   if (c->gs_fused) {
     // the last update with |w|^2 and the Hessenberg column in one launch
     if ((rc = launch_k(c, axpy8f_f32_kernel<RED_TB>, M.nblk4, RED_TB, 0, st, (const float*)M.V, (int64_t)c->nonods,
-                       nv, (const double*)(two ? c->d_h2 : c->d_h1), w, n4, M.part, (const double*)c->d_h1,
-                       two ? (const double*)c->d_h2 : (const double*)nullptr, Hc, inv, M.gs_cnt + 32)))
+                       nv, (const double*)hl, w, n4, M.part, (const double*)c->d_h1, h2, Hc, inv, M.gs_cnt + 32)))
       return rc;
   } else {
-    if ((rc = launch_k(c, axpy8_f32_kernel<RED_TB>, M.nblk4, RED_TB, 0, st, (const float*)M.V, (int64_t)c->nonods,
-                       nv, (const double*)(two ? c->d_h2 : c->d_h1), w, n4, M.part, 1)))
-      return rc;
-    if ((rc = launch_k(c, cgs_finish_kernel, 1, reduce_threads(M.nblk4), 0, st, (const double*)M.part, M.nblk4, (const double*)c->d_h1,
-                       two ? (const double*)c->d_h2 : (const double*)nullptr, nv, Hc, inv)))
+    if ((rc = update(hl, 1))) return rc;
+    if (M.nblk4 <= 256) {
+      if ((rc = launch_k(c, cgs_scale_f32_kernel, nblk(n4, 256), 256, 0, st, (const double*)npart, M.nblk4,
+                         (const double*)c->d_h1, h2, nv, Hc, (const float*)w, M.V + (size_t)nv * c->nonods, n4)))
+        return rc;
+      CKL(c);
+      return DG_OK;
+    }
+    if ((rc = launch_k(c, cgs_finish_kernel, 1, reduce_threads(M.nblk4), 0, st, (const double*)npart, M.nblk4,
+                       (const double*)c->d_h1, h2, nv, Hc, inv)))
       return rc;
   }
   if ((rc = launch_k(c, scale4_f32_kernel, nblk(n4, 256), 256, 0, st, (const float*)w, (const float*)inv,
