@@ -389,8 +389,8 @@ def batched_leg(args, s, m, dofs, dev, stream, ws, R64=None, RMX=None):
                                                                  "tcgen05_bulk")
     sc_us = None
     if scaled:
-        # the steps after the zero-start one (3 of the 5 BF16 launches of a
-        # preconditioner application): bsc_mma_kernel alone, CUDA events
+        # one scaled-face step after the zero-start one (node-major iterates):
+        # bwarp_kernel alone, CUDA events
         g = torch.Generator(device=dev).manual_seed(1)
         xs = torch.randn(dofs * 64, dtype=torch.float32, device=dev, generator=g)
         cs = torch.randn(dofs * 64, dtype=torch.float32, device=dev, generator=g)

@@ -648,7 +648,7 @@ __device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
 // partial[bx * KMAXV + i] = this block's slice of V[i] . z for the vectors
 // i of grid row y (8 each), FP64, two entries a load (n even).  z is read once
 // per 8 vectors.  Bound by the FP64 pipe (one FMA per 8 bytes of V).  960,000
-// rows, 15 vectors on average: 41 -> 30 us a pass.
+// rows, 15 vectors on average: 41 -> 39 us a pass (axpy8_f64_kernel 47 -> 33).
 template <int TB>
 __global__ void __launch_bounds__(TB) mdot8_f64_kernel(const double* __restrict__ V, int64_t ld, int nv,
                                                        const double* __restrict__ z, int64_t n2,
@@ -1099,10 +1099,9 @@ __global__ void __launch_bounds__(1024) vcycle_tail_kernel(TailParams<T> p) {
 // vector with the level vectors in shared memory (4 n_l doubles per level + n
 // scratch), the same operations as vcycle_tail_kernel; column q of T (n rows
 // of ld entries) is the image of unit vector q of [r; e].
-// FP64-pipe bound (1.2 ms for 1,089 rows and columns, 0.4 ms for 579 x 1,158):
-// 4 lanes per row, few reduction steps, and no division per row (a division
-// for one lane of eight cost more than the row's products: 12 ms at 1,158 x
-// 2,316 before).
+// FP64-pipe bound: 4 lanes per row, few reduction steps, and no division per
+// row (a division for one lane of eight cost more than the row's products: 12
+// ms at 1,158 x 2,316, about 1 ms without it).
 constexpr int kColLanes = 4;
 __device__ __forceinline__ void col_jacobi(const TLevel<double>& L, const double* wd, const double* e_in,
                                            const double* r, double* e_out, double* rr_out) {

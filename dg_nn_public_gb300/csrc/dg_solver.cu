@@ -399,11 +399,11 @@ int launch_k(dg_ctx* c, void (*kern)(KArgs...), unsigned grid, unsigned block, s
   return DG_OK;
 }
 
-// Plain launch.  The FP64 chain and the triangles' block products take it:
-// with programmatic dependent launches the FP64 GMRES was slower at every
-// size (2,048 triangles 5.24 -> 5.49 ms; 3,072 / 10,368 / 48,000 tetrahedra
-// 15.1 -> 19.4, 36.5 -> 43.0, 120.9 -> 131.1 ms), the mixed solve on 97 x 61 x 2
-// triangles 3.00 -> 3.28 ms with them on its block products.
+// Plain launch.  The FP64 chain takes it: with programmatic dependent launches
+// the FP64 GMRES was slower at every size (2,048 triangles 5.24 -> 5.49 ms;
+// 3,072 / 10,368 / 48,000 tetrahedra 15.1 -> 19.4, 36.5 -> 43.0, 120.9 -> 131.1
+// ms), and so was residual_kernel in FP32 on triangles, which loads nothing
+// ahead of its wait (11,834 of them: 3.00 -> 3.28 ms a mixed solve).
 template <typename... KArgs, typename... Args>
 int launch_p(dg_ctx* c, void (*kern)(KArgs...), dim3 grid, unsigned block, size_t smem, cudaStream_t st,
              Args... args) {
