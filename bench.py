@@ -276,13 +276,12 @@ def config_block(args, m, extra=None):
 # 20^3 Kuhn-cube workload (48,000 tets): dram__bytes_read.sum +
 # dram__bytes_write.sum of a capture on the 18^3 mesh (34,992 tets) scaled
 # by the element count (scaled-face step: profiles/smooth_scaled_tma_kernel_n18.md;
-# BF16 step, FP32 apply, FP64 residual: profiles/residual_tma_kernel_c2.md);
-# other workloads report null.
+# BF16 step, FP32 apply: profiles/residual_tma_kernel_c2.md); other kernels
+# and workloads report null.
 TRAFFIC_C2 = {
     "smooth_scaled": {"bytes_per_launch": 166.7e6},
     "smooth_pc": {"bytes_per_launch": 240.2e6},
     "apply_f32": {"bytes_per_launch": 393.4e6},
-    "apply_f64": {"bytes_per_launch": 773.9e6},
 }
 
 
@@ -419,10 +418,9 @@ def batched_leg(args, s, m, dofs, dev, stream, ws, R64=None, RMX=None):
         "speedup_vs_single_mixed": (ws * args.nrhs * dofs * args.steps / tb) / RMX["value"] if RMX else None,
         "speedup_vs_fp64": (ws * args.nrhs * dofs * args.steps / tb) / R64["value"] if R64 else None,
         "method": "lockstep flexible GMRES(%d) on RHS-interleaved FP32 vectors; BF16 block smoothing on "
-                  "tensor cores (x split into BF16 hi+lo; zero-start step and restriction by the kernel the "
-                  "autotuner chose among CUDA cores, mma.sync tiles, mma.sync bulk-copy and tcgen05 forms; the "
-                  "other smoothing steps on the scaled face blocks W_e A_ef with mma.sync), FP32 apply on CUDA "
-                  "cores; per-RHS FP64 refinement" % args.batched_m}
+                  "tensor cores (x split into BF16 hi+lo, one warp per element and 32 columns with mma.sync; the "
+                  "smoothing steps after the zero-start one on the scaled face blocks W_e A_ef), FP32 apply on "
+                  "CUDA cores; FP64 refinement residuals from 8-bit digits with mma.sync" % args.batched_m}
 
 
 def run_ours(args):
@@ -650,8 +648,8 @@ def run_ours(args):
         xa = torch.randn(dofs, dtype=torch.float64, device=dev)
         y64 = torch.empty_like(xa)
         t64 = time_launch(lambda: s.apply(xa, y64))
-        rooflines.append(("apply_f64", "residual_kernel<20,4,8> (stored-block FP64 apply of the plain FP64 "
-                          "path)", nbytes64, t64, 2.0 * N * N * (m.nele + s_int)))
+        rooflines.append(("apply_f64", "stored-block FP64 apply of the plain FP64 path (res64_mma_kernel on "
+                          "the blocks' digits, residual_kernel without them)", nbytes64, t64, 2.0 * N * N * (m.nele + s_int)))
         # per inner iteration: preconditioner + apply; the rest is Gram-Schmidt,
         # Hessenberg updates and the refinement steps
         t_pc = time_launch(lambda: s.precond_f32(bs, xo))
@@ -663,7 +661,7 @@ def run_ours(args):
         xa = torch.randn(dofs, dtype=torch.float64, device=dev)
         ya = torch.empty_like(xa)
         t = time_launch(lambda: s.apply(xa, ya))
-        rooflines.append(("apply_f64", "residual_kernel<20,4,8> (stored-block FP64 apply)", nbytes64, t,
+        rooflines.append(("apply_f64", "stored-block FP64 apply (res64_mma_kernel or residual_kernel)", nbytes64, t,
                           2.0 * N * N * (m.nele + s_int)))
 
     def roof(entry):
