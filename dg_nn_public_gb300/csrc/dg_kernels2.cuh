@@ -692,6 +692,23 @@ __global__ void __launch_bounds__(TB) mdot8_f64_kernel(const double* __restrict_
   }
 }
 
+// Sum over nred blocks of the dots' partial sums of vector i = threadIdx.x /
+// (TB / KMAXV), in each of its TB / KMAXV threads: all vectors at once, so that
+// the loads of a thread are the only chain.
+template <int TB>
+__device__ __forceinline__ double fold_dots(const double* __restrict__ partial, int nred, int nv) {
+  constexpr int G = TB / KMAXV;
+  const int i = threadIdx.x / G, g = threadIdx.x % G;
+  double s = 0.0;
+  if (i < nv) {
+#pragma unroll 8
+    for (int b = g; b < nred; b += G) s += partial[(int64_t)b * KMAXV + i];
+  }
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
 // z -= sum_i V[i] h[i] (nv <= 256, n even); with want_norm also
 // partial_out[bx * KMAXV] = this block's slice of |z_new|^2.  With nred > 0
 // the coefficients are first summed here from the partial sums of the dots
@@ -709,14 +726,11 @@ __global__ void __launch_bounds__(TB) axpy8_f64_kernel(const double* __restrict_
   __shared__ double red[TB / 32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (nred > 0) {
-    for (int i = wid; i < nv; i += TB / 32) {
-      double s = 0.0;
-      for (int b = lane; b < nred; b += 32) s += partial_in[(int64_t)b * KMAXV + i];
-      s = warp_sum(s);
-      if (lane == 0) {
-        hs[i] = s;
-        if (blockIdx.x == 0) h_out[i] = s;
-      }
+    const double t = fold_dots<TB>(partial_in, nred, nv);
+    const int i = threadIdx.x / (TB / KMAXV);
+    if (threadIdx.x % (TB / KMAXV) == 0 && i < nv) {
+      hs[i] = t;
+      if (blockIdx.x == 0) h_out[i] = t;
     }
   } else {
     for (int i = threadIdx.x; i < nv; i += TB) hs[i] = h[i];
