@@ -1904,7 +1904,7 @@ extern "C" int dg_solve_mixed_batched(dg_ctx* c, double* x, const double* b, int
                                 st));
     }
     const int gx = (int)std::max<int64_t>(1, std::min<int64_t>(2 * c->nsm, (n + 255) / 256));
-    if (mask && (r2 = ensure_digits(c, st)) == DG_ERR_ALLOC) {   // no room: one product per RHS
+    if (mask && (r2 = ensure_digits(c, st)) == kNoDigits) {   // one product per RHS
       for (int q = 0; q < nrhs; ++q)
         if (redo[q] == 1 &&
             (r2 = residual(c, x + (size_t)q * n, b + (size_t)q * n, S.r64 + (size_t)q * n, nullptr, 0, st)))
@@ -1912,14 +1912,11 @@ extern "C" int dg_solve_mixed_batched(dg_ctx* c, double* x, const double* b, int
     } else if (mask) {
       if (r2) return r2;
       const int ngr = (nrhs + 15) / 16;
-      int* emax = reinterpret_cast<int*>(S.h);   // scratch between the inner solves, as the basis is
-      unsigned char* xdig = reinterpret_cast<unsigned char*>(S.V);   // (m + 1 >= 2) x 4 bytes per value
-      CK(c, cudaMemsetAsync(emax, 0, sizeof(int) * kNR, st));
-      bexp_kernel<<<dim3(gx, nrhs), 256, 0, st>>>(x, n, emax);
-      x_digits_kernel<<<dim3((unsigned)c->B, ngr), 160, 0, st>>>(x, n, emax, mask, xdig);
-      bres64_mma_kernel<<<nblk(c->B * ngr, 4), 128, 0, st>>>(c->d_adig, c->d_aexp, c->d_nbe, xdig, emax, b, S.r64,
+      unsigned* xe = reinterpret_cast<unsigned*>(S.V);   // scratch between the inner solves
+      x_exponents_kernel<<<dim3(nblk(c->B, 16), ngr), 256, 0, st>>>(x, n, c->B, ngr, mask, xe);
+      bres64_mma_kernel<<<nblk(c->B * ngr, 4), 128, 0, st>>>(c->d_adig, c->d_aexp, c->d_blk, c->d_nbe, x, xe, b, S.r64,
                                                              c->B, n, ngr, mask);
-      bump(3);
+      bump(2);
     }
     bnorm64_kernel<<<dim3(gx, nrhs), 256, 0, st>>>(S.r64, n, S.part);
     bnorm_finish_kernel<<<1, kNR, 0, st>>>(S.part, gx, c->d_scal, nullptr);

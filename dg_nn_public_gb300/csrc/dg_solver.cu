@@ -122,6 +122,7 @@ struct dg_ctx {
   unsigned char* d_adig = nullptr;
   int* d_aexp = nullptr;
   int dig_version = -1;
+  bool dig_few64 = false;   // few elements of this build have to be taken in FP64
   // single-RHS FP64 products take the digits: always after a quadrature build
   // (which forms them, 0.3 of 12 ms at 48,000 tetrahedra), inside dg_gmres
   // after an affine one (made per request, where a copy of 0.3 ms would save
@@ -765,8 +766,8 @@ int launch_residual(dg_ctx* c, const double* x, const double* b, double* r, doub
   if (D == 3 && c->dig_single && c->dig_version == c->build_version && !(flags & RF_ZEROX))
     return launch_p(c, res64_mma_kernel, (unsigned)std::min<int64_t>(nblk(c->B, kR64Warps), 2 * c->nsm),
                     32 * kR64Warps, kR64Smem, st, (const unsigned char*)c->d_adig,
-                    (const int*)c->d_aexp, (const double*)c->d_W, (const int*)c->d_nbe, x, b, r, x_out, (int64_t)c->B,
-                    flags, (const double*)c->T.P, r1);
+                    (const int*)c->d_aexp, (const double*)c->d_blk, (const double*)c->d_W, (const int*)c->d_nbe, x, b, r,
+                    x_out, (int64_t)c->B, flags, (const double*)c->T.P, r1);
   return launch_p(c, residual_kernel<E::N, E::F, E::EPB>, nblk(c->B, E::EPB), E::EPB * E::N, 0, st,
                   (const double*)c->d_blk, (const double*)c->d_W, (const int*)c->d_nbe, x, b, r, x_out, (int64_t)c->B,
                   flags, (const double*)c->T.P, r1, (const float*)nullptr);
@@ -1688,7 +1689,7 @@ int dg_build_operator(dg_ctx* c, void* stream) {
   ++c->build_version;
   c->dig_single = false;
   if (c->D == 3 && (c->fast_build != 1 || c->general_build)) {
-    if ((rc = ensure_digits(c, st)) && rc != DG_ERR_ALLOC) return rc;
+    if ((rc = ensure_digits(c, st)) > 0) return rc;
     c->dig_single = rc == DG_OK;
   }
   // colour-probe Galerkin operator on P1CG (volume_mf_diff.py:1696-1754), or
@@ -1992,7 +1993,7 @@ int dg_gmres(dg_ctx* c, double* x, const double* b, double tol, int32_t m, int32
     ~DigGuard() { c->dig_single = keep; }
   } guard{c, c->dig_single};
   if (c->D == 3) {
-    if ((rc = ensure_digits(c, st)) && rc != DG_ERR_ALLOC) return rc;
+    if ((rc = ensure_digits(c, st)) > 0) return rc;
     c->dig_single = rc == DG_OK;
   }
   double* r = c->d_t1;
