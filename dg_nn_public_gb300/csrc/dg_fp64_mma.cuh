@@ -92,10 +92,16 @@ __device__ __forceinline__ void mma_f16_16816(float (&c)[4], uint32_t a0, uint32
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// 2^e as a double, e clamped to the normal range
-__device__ __forceinline__ double exp2_int(int e) {
-  e = min(max(e, -1022), 1023);
-  return __longlong_as_double((long long)(e + 1023) << 52);
+// 2^e as a double, -1022 <= e <= 1023
+__device__ __forceinline__ double exp2_int(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
+
+// b - 2^e v for |v| < 2^49, 0 or at least 2^-32: one rounding.  2^e need not
+// be a number where 2^e v is one, so it goes in as two factors; beyond the
+// clamp the product is below half of the smallest subnormal, or infinite.
+__device__ __forceinline__ double sub_scaled(double b, int e, double v) {
+  e = min(max(e, -1200), 1100);
+  const int h = e >> 1;
+  return fma(-exp2_int(e - h), v * exp2_int(h), b);
 }
 
 // a 48-bit signed integer as a double, exactly (one FP64 addition)
@@ -363,7 +369,7 @@ __global__ void __launch_bounds__(128, 2) bres64_mma_kernel(
         const int c = 2 * q + d;
         const double H = int48_to_double(join4(acc[0][nt][c], acc[1][nt][c], acc[2][nt][c], acc[3][nt][c]));
         const double L = int48_to_double(join4(acc[4][nt][c], acc[5][nt][c], acc[6][nt][c], acc[7][nt][c]));
-        out[d] = fma(-exp2_int(ea[e * N + m + d] + ex - 36), fma(L, 0x1p-32, H), b[o + d]);
+        out[d] = sub_scaled(b[o + d], ea[e * N + m + d] + ex - 36, fma(L, 0x1p-32, H));
       }
       *reinterpret_cast<double2*>(r + o) = make_double2(out[0], out[1]);
     }
@@ -674,10 +680,8 @@ __global__ void __launch_bounds__(32 * kR64Warps, 2) res64_mma_kernel(
         Lt += __shfl_xor_sync(0xffffffffu, Lt, o);
       }
       const long long H = (t & 1) ? Ht : Hs, L = (long long)((t & 1) ? Lt : Ls);
-      if (mine) {
-        const double sc = exp2_int(ee_e + em - 1022 - 36);
-        res = fma(-sc, fma(int48_to_double(L), 0x1p-32, int48_to_double(H)), b_e);
-      }
+      if (mine)
+        res = sub_scaled(b_e, ee_e + em - 1022 - 36, fma(int48_to_double(L), 0x1p-32, int48_to_double(H)));
     }
     if (dead) res = __longlong_as_double(0x7ff8000000000000ll);
     if (mine) {
