@@ -900,6 +900,12 @@ int vcycle_cluster(dg_ctx* c, const double* r_sfc, cudaStream_t st) {
   return DG_OK;
 }
 
+// Limit of tail_max64, and the shared memory that tail_columns_kernel needs at
+// most under it: 2 kTailRows rows of the first level, fewer than that and one
+// per level below it, four doubles a row and one more of the first level.
+constexpr int kTailRows = 1280;
+constexpr int kTailSmem = 8 * (9 * 2 * kTailRows + 4 * VMAXLEV);
+
 // The matrix of the V-cycle's coarse tail (tail_columns_kernel) for the
 // current operator build, formed on first use: only the FP64 preconditioner
 // reads it.  Entry points that reach vcycle() call it first, outside any
@@ -922,8 +928,9 @@ int ensure_tail64(dg_ctx* c, cudaStream_t st) {
     words += 4 * (size_t)L.n;
   }
   const int n = c->lev[l0].n, ncol = l0 > 0 ? 2 * n : n;
-  CK(c, cudaFuncSetAttribute(tail_columns_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(words * sizeof(double))));
+  // one value for every context: the attribute is the function's, and another
+  // thread's context may set it between this line and the launch
+  CK(c, cudaFuncSetAttribute(tail_columns_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem));
   if (c->tail_ld > ncol) CK(c, cudaMemsetAsync(c->d_tail, 0, sizeof(double) * (size_t)n * c->tail_ld, st));
   tail_columns_kernel<<<ncol, 512, words * sizeof(double), st>>>(tp, c->d_tail, c->tail_ld);
   bump();
@@ -1323,7 +1330,7 @@ int dg_create(const dg_mesh_desc* m, const dg_config* cfg, dg_ctx** out) {
   {
     const char* t64 = std::getenv("DG_TAIL_MAX64");
     const char* t32 = std::getenv("DG_TAIL_MAX32");
-    if (t64 && t64[0]) c->tail_max64 = std::min(std::max(std::atoi(t64), 1), 1280);
+    if (t64 && t64[0]) c->tail_max64 = std::min(std::max(std::atoi(t64), 1), kTailRows);
     if (t32 && t32[0]) c->tail_max32 = std::atoi(t32);
     const char* dm = std::getenv("DG_DENSE_MAX32");
     if (dm && dm[0]) c->dense_max32 = std::atoi(dm);
