@@ -173,6 +173,7 @@ struct dg_ctx {
   // triangles with 273 / 545 / 1,089 rows: 7.9 / 6.8 / 5.7 ms)
   int tail_max64 = 640, tail_max32 = 800;
   int tail_l0 = 0, tail_ld = 0, t64_version = -1;
+  bool tail_now = false;   // the current call's V-cycles use it (ensure_tail64)
   double* d_tail = nullptr;
   // mixed preconditioner: exact (dense inverse) solve on the first SFC level
   // with at most this many rows (0 = keep the V-cycle to the one-node level)
@@ -398,6 +399,19 @@ int launch_k(dg_ctx* c, void (*kern)(KArgs...), unsigned grid, unsigned block, s
   CK(c, cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
   bump();
   return DG_OK;
+}
+
+// Whether the caller is capturing st into a graph of its own.  A captured call
+// holds no pointer to data that is formed per operator build outside the call
+// (digits, coarse tail matrix): it would be stale in a replay after a rebuild.
+bool user_capture(dg_ctx* c, cudaStream_t st) {
+  if (c->cap_stream && st == c->cap_stream) return false;   // the library's own graphs
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &s) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return s != cudaStreamCaptureStatusNone;
 }
 
 // Plain launch.  The FP64 chain takes it: with programmatic dependent launches
@@ -763,7 +777,7 @@ int launch_residual(dg_ctx* c, const double* x, const double* b, double* r, doub
     if ((rc = ensure_w64_t<D>(c, st))) return rc;
   }
   // tetrahedra: the product from the digit copy
-  if (D == 3 && c->dig_single && c->dig_version == c->build_version && !(flags & RF_ZEROX))
+  if (D == 3 && c->dig_single && c->dig_version == c->build_version && !(flags & RF_ZEROX) && !user_capture(c, st))
     return launch_p(c, res64_mma_kernel, (unsigned)std::min<int64_t>(nblk(c->B, kR64Warps), 2 * c->nsm),
                     32 * kR64Warps, kR64Smem, st, (const unsigned char*)c->d_adig,
                     (const int*)c->d_aexp, (const double*)c->d_blk, (const double*)c->d_W, (const int*)c->d_nbe, x, b, r,
@@ -909,9 +923,11 @@ constexpr int kTailSmem = 8 * (9 * 2 * kTailRows + 4 * VMAXLEV);
 // The matrix of the V-cycle's coarse tail (tail_columns_kernel) for the
 // current operator build, formed on first use: only the FP64 preconditioner
 // reads it.  Entry points that reach vcycle() call it first, outside any
-// capture of their own.
+// capture of their own; under the caller's capture the one-CTA kernel takes the
+// tail instead.
 int ensure_tail64(dg_ctx* c, cudaStream_t st) {
-  if (c->vc_cluster > 0 || c->t64_version == c->build_version) return DG_OK;
+  c->tail_now = !user_capture(c, st);
+  if (c->vc_cluster > 0 || !c->tail_now || c->t64_version == c->build_version) return DG_OK;
   const int nl = (int)c->lev.size(), l0 = c->tail_l0;
   if (c->lev.back().n != 1 || nl > VMAXLEV)
     return fail(c, DG_ERR_STATE, "coarsest SFC level must hold one node");
@@ -942,16 +958,47 @@ int ensure_tail64(dg_ctx* c, cudaStream_t st) {
   return DG_OK;
 }
 
+// Levels l0 .. top of the V-cycle in one CTA from their matrices, with the
+// restriction into level l0; up to kTailOneCta rows (130 us on 290).
+constexpr int kTailOneCta = 320;
+int vcycle_tail(dg_ctx* c, int l0, const double* r_sfc, cudaStream_t st) {
+  const int nl = (int)c->lev.size(), top = nl - 1;
+  DevLevel& L = c->lev[l0];
+  if (c->lev[top].n != 1) return fail(c, DG_ERR_STATE, "coarsest SFC level must hold one node");
+  if (l0 == 0) {
+    CK(c, cudaMemcpyAsync(L.r, r_sfc, sizeof(double) * L.n, cudaMemcpyDeviceToDevice, st));
+    CK(c, cudaMemsetAsync(L.e, 0, sizeof(double) * L.n, st));
+  } else {
+    const DevLevel& P = c->lev[l0 - 1];
+    const int rc = launch_p(c, lev_restrict_kernel<double>, nblk(L.n, 128), 128, 0, st, (const double*)P.rr,
+                            (const double*)P.e, L.r, L.e, P.n, L.n);
+    if (rc) return rc;
+  }
+  if (l0 == top) return launch_p(c, lev_coarse_kernel<double>, 1, 32, 0, st, (const double*)L.val, (const double*)L.r, L.e);
+  TailParams<double> tp;
+  tp.l0 = l0;
+  tp.top = top;
+  tp.pre = c->cfg.pre_smooth_its;
+  tp.post = c->cfg.post_smooth_its;
+  tp.w = c->cfg.jac_wei;
+  for (int l = 0; l < nl; ++l) {
+    const DevLevel& D = c->lev[l];
+    tp.lev[l] = TLevel<double>{D.rowptr, D.col, D.val, D.diag, D.up, D.e, D.e2, D.r, D.rr, D.n};
+  }
+  return launch_p(c, vcycle_tail_kernel<double>, 1, 1024, 0, st, tp);
+}
+
 // One SFC V-cycle; r_sfc is level-0 input, result left in lev[0].e.  Sweeps
 // per level with the transfers between levels formed on the fly, then the
-// coarse tail as one matrix product (ensure_tail64).
+// coarse tail as one matrix product (ensure_tail64), or in one CTA.
 int vcycle(dg_ctx* c, const double* r_sfc, cudaStream_t st) {
   if (c->vc_cluster > 0) {
     if (c->lev.back().n != 1) return fail(c, DG_ERR_STATE, "coarsest SFC level must hold one node");
     return vcycle_cluster(c, r_sfc, st);
   }
   const double w = c->cfg.jac_wei;
-  const int TB = 128, l0 = c->tail_l0, npre = c->cfg.pre_smooth_its, npost = c->cfg.post_smooth_its;
+  const int TB = 128, npre = c->cfg.pre_smooth_its, npost = c->cfg.post_smooth_its;
+  const int l0 = c->tail_now ? c->tail_l0 : tail_start(c, kTailOneCta);
   int rc;
   auto rhs_of = [&](int l) -> const double* { return l == 0 ? r_sfc : c->lev[l].r; };
   for (int l = 0; l < l0; ++l) {
@@ -973,7 +1020,9 @@ int vcycle(dg_ctx* c, const double* r_sfc, cudaStream_t st) {
       std::swap(L.e, L.e2);
     }
   }
-  {
+  if (!c->tail_now) {
+    if ((rc = vcycle_tail(c, l0, r_sfc, st))) return rc;
+  } else {
     DevLevel& L = c->lev[l0];
     const int ncol = l0 > 0 ? 2 * L.n : L.n;
     const double* fr = l0 > 0 ? c->lev[l0 - 1].rr : r_sfc;
