@@ -33,7 +33,7 @@
 
 namespace {
 
-constexpr int kDigElem = 16000;             // bytes of an element's digits
+constexpr int kDigElem = 16000;             // bytes of an element's digits (digit_bytes)
 constexpr uint32_t kZeroDigits = 0x80808080u;
 
 // byte offset of (slot, row m, t) in an element's digits
@@ -733,17 +733,27 @@ __global__ void __launch_bounds__(256) bnorm64_kernel(const double* __restrict__
 }
 
 // Block digits of the current operator build (3D), kept with the context.
-// kNoDigits: not to be used, because the memory cannot be had (they take as
-// much as the FP64 blocks; no error left behind) or because over a quarter of
-// the elements would be taken in FP64 anyway; the callers keep to the FP64 pipe.
+// kNoDigits: not to be used, because there is no room for them (no error left
+// behind) or because over a quarter of the elements would be taken in FP64
+// anyway; the callers keep to the FP64 pipe.  They take as much memory as the
+// FP64 blocks and are formed before what a solve must have, about as much again
+// for a mixed solve, so room is three times their size; dalloc gives them back
+// when something else does not fit after all.
 constexpr int kNoDigits = -1;
 int ensure_digits(dg_ctx* c, cudaStream_t st) {
   if (c->dig_version == c->build_version) return c->dig_few64 ? DG_OK : kNoDigits;
-  if ((!c->d_adig && dalloc(c, &c->d_adig, (size_t)c->B * kDigElem)) ||
-      (!c->d_aexp && dalloc(c, &c->d_aexp, (size_t)c->B * 20 + 1))) {
-    cudaGetLastError();
-    c->err.clear();
-    return kNoDigits;
+  if (!c->d_adig) {
+    const int64_t bytes = digit_bytes(c);
+    size_t room = 0, total = 0;
+    CK(c, cudaMemGetInfo(&room, &total));
+    if (c->mem_limit > 0) room = std::min<size_t>(room, (size_t)std::max<int64_t>(c->mem_limit - c->dev_bytes, 0));
+    if ((int64_t)(room / 3) < bytes || dev_malloc(c, (void**)&c->d_adig, (size_t)bytes) != cudaSuccess) {
+      cudaGetLastError();
+      c->d_adig = nullptr;
+      return kNoDigits;
+    }
+    c->dev_bytes += bytes;
+    c->d_aexp = reinterpret_cast<int*>(c->d_adig + c->B * kDigElem);
   }
   int* nfp64 = c->d_aexp + (size_t)c->B * 20;
   CK(c, cudaMemsetAsync(nfp64, 0, sizeof(int), st));

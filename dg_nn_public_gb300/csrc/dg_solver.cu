@@ -84,7 +84,8 @@ struct dg_ctx {
   std::vector<int> bf_elem, bf_face, bf_type;
   // device allocations (released in dg_destroy)
   std::vector<void*> allocs;
-  int64_t dev_bytes = 0;   // sum of the allocations in allocs (freed only by dg_destroy)
+  int64_t dev_bytes = 0;   // sum of the allocations in allocs (freed only by dg_destroy) and of the digits
+  int64_t mem_limit = 0;   // DG_MEM_LIMIT: more than this in all fails as if the device were full (0 = no limit)
   double* d_x = nullptr;
   int *d_nbe = nullptr, *d_nbface = nullptr, *d_aln = nullptr, *d_bct = nullptr;
   // shared-face tables of the reduced-precision copies (3D): d_fref5[e][j]
@@ -351,11 +352,42 @@ int fail(dg_ctx* c, int code, const std::string& msg) {
 
 #define CKL(ctx) CK(ctx, cudaGetLastError())
 
+// bytes of the digit copy of the blocks: 16,000 an element, 20 row exponents an
+// element, the count of the elements taken in FP64 (dg_fp64_mma.cuh)
+int64_t digit_bytes(const dg_ctx* c) { return c->B * (16000 + 80) + 16; }
+
+cudaError_t dev_malloc(dg_ctx* c, void** p, size_t bytes) {
+  if (c->mem_limit > 0 && c->dev_bytes + (int64_t)bytes > c->mem_limit) return cudaErrorMemoryAllocation;
+  return cudaMalloc(p, bytes);
+}
+
+// The digit copy of the blocks is the one buffer that every caller has another
+// way for; it is outside allocs and given back when another one does not fit.
+void release_digits(dg_ctx* c) {
+  cudaDeviceSynchronize();   // no product is reading them
+  if (c->d_adig) {
+    cudaFree(c->d_adig);
+    c->dev_bytes -= digit_bytes(c);
+  }
+  c->d_adig = nullptr;
+  c->d_aexp = nullptr;
+  c->dig_version = -1;
+  if (c->arnoldi_exec) {   // its products read them
+    cudaGraphExecDestroy(c->arnoldi_exec);
+    c->arnoldi_exec = nullptr;
+  }
+}
+
 template <typename T>
 int dalloc(dg_ctx* c, T** p, size_t count) {
   *p = nullptr;
   if (count == 0) count = 1;
-  cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
+  cudaError_t e = dev_malloc(c, (void**)p, count * sizeof(T));
+  if (e == cudaErrorMemoryAllocation && c->d_adig) {   // the digits can be done without
+    cudaGetLastError();
+    release_digits(c);
+    e = dev_malloc(c, (void**)p, count * sizeof(T));
+  }
   if (e != cudaSuccess) return fail(c, DG_ERR_ALLOC, std::string("cudaMalloc: ") + cudaGetErrorString(e));
   c->allocs.push_back((void*)*p);
   c->dev_bytes += (int64_t)(count * sizeof(T));
@@ -1333,6 +1365,7 @@ void dg_destroy(dg_ctx* ctx) {
   destroy_mixed(ctx);
   if (ctx->cap_stream) cudaStreamDestroy(ctx->cap_stream);
   for (void* p : ctx->allocs) cudaFree(p);
+  if (ctx->d_adig) cudaFree(ctx->d_adig);
   cudaSetDevice(cur);
   delete ctx;
 }
@@ -1377,6 +1410,8 @@ int dg_create(const dg_mesh_desc* m, const dg_config* cfg, dg_ctx** out) {
   CK(c.get(), cudaGetDeviceProperties(&prop, c->dev));
   c->nsm = prop.multiProcessorCount;
   {
+    const char* ml = std::getenv("DG_MEM_LIMIT");
+    if (ml && ml[0]) c->mem_limit = std::max<long long>(std::atoll(ml), 0);
     const char* t64 = std::getenv("DG_TAIL_MAX64");
     const char* t32 = std::getenv("DG_TAIL_MAX32");
     if (t64 && t64[0]) c->tail_max64 = std::min(std::max(std::atoi(t64), 1), kTailRows);

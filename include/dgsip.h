@@ -129,8 +129,10 @@ int dg_set_build_mode(dg_ctx* ctx, int32_t mode);
  * (z06/get_bdiag_diag.py:30-62) and _get_RAR_and_sfc_data_Um()
  * (z06/volume_mf_diff.py:1642-1693, multigrid_linearelastic.py:175-283).
  * On tetrahedra a mode 0 build also keeps the blocks' 8-bit digits for the FP64
- * products, another 16.4 KB an element (dg_gmres and the batched solve form them
- * after a mode 1 build); without that memory the FP64 blocks are used. */
+ * products, another 16.1 KB an element (dg_gmres and the batched solve form them
+ * after a mode 1 build).  They are left out where less than three times that
+ * is free, and given back when another buffer of the context does not fit; the
+ * FP64 blocks are used then, as by calls that the caller captures. */
 int dg_build_operator(dg_ctx* ctx, void* stream);
 /* Copy bdiagK (nele, nloc, nloc) and diagK (nele, nloc) out. */
 int dg_get_bdiag(dg_ctx* ctx, double* bdiag /* [device] */, double* diag /* [device] or NULL */, void* stream);
