@@ -406,7 +406,7 @@ def batched_leg(args, s, m, dofs, dev, stream, ws, R64=None, RMX=None):
         sc_us = a0.elapsed_time(a1) * 1e3 / 10
         del xs, cs, xo
     return {
-        "smoothing_kernel": kern, "smoothing_kernel_us": tune_us,
+        "smoothing_kernel": "scaled_faces_warp" if scaled else kern, "smoothing_kernel_us": tune_us,
         "scaled_face_steps": scaled, "scaled_step_us": sc_us,
         "workload": "c4: the %s mesh with %d Fourier right-hand sides (8 modes each, wavenumbers 1..4, "
                     "N(0,1) amplitudes, seed %d), solved together" % (

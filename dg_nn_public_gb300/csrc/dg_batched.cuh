@@ -1513,9 +1513,14 @@ int bsmooth_scaled(dg_ctx* c, Mixed& M, const float* xx, const float* cv, float*
 // Smoothing-kernel autotuner of the batched solve: times every variant of
 // the full smoothing step (x and b given) on zeroed scratch vectors with
 // CUDA events (one warm launch, then 3 timed) once per mixed build, before
-// any graph capture, and keeps the fastest; DG_BATCHED_KERNEL pins one.
+// any graph capture, and keeps the fastest; DG_BATCHED_KERNEL pins one.  With
+// scaled faces the solve runs bwarp_kernel whatever is fastest, so nothing is
+// timed (and no layout of the other forms made) unless dg_set_batched_kernel(-1)
+// asked for it: 9 of 65 ms of a first batch after a rebuild at 24,576 tetrahedra.
 int autotune_batched(dg_ctx* c, Mixed& M, BatchState& S, cudaStream_t st) {
   if (c->batched_pinned || S.tune_version == c->mixed_version) return DG_OK;
+  if (batched_scaled(c, M) && !c->batched_tune_asked) return DG_OK;
+  c->batched_tune_asked = false;
   const size_t nv = (size_t)c->nonods * kNR;
   CK(c, cudaMemsetAsync(S.t1, 0, sizeof(float) * nv, st));
   CK(c, cudaMemsetAsync(S.t2, 0, sizeof(float) * nv, st));
@@ -1778,7 +1783,7 @@ int run_bstep(dg_ctx* c, int j, int m, cudaStream_t st) {
   auto tag = [](int64_t v) { return reinterpret_cast<const void*>(static_cast<intptr_t>(v)); };
   const std::vector<const void*> key = {
       tag(m),
-      tag(c->batched_kernel),
+      tag(batched_scaled(c, M) ? -1 : c->batched_kernel),
       tag(c->mixed_version),
       tag(c->precond_bf16),
       tag(c->batched_gs2),
@@ -2151,7 +2156,7 @@ extern "C" int dg_smooth_scaled_batched(dg_ctx* c, const float* x, const float* 
 }
 
 // Batched smoothing kernel variant: -1 = timed choice at the next batched
-// solve (default), 0 CUDA cores, 1 / 2 mma.sync per element (4 / 8 warps),
+// solve, 0 CUDA cores, 1 / 2 mma.sync per element (4 / 8 warps),
 // 3 mma.sync persistent bulk-copy, 4 tcgen05 persistent bulk-copy.
 // tune_us (may be NULL) receives the last timing per variant (us, -1 = not
 // timed) and *chosen the variant in use.
@@ -2161,6 +2166,7 @@ extern "C" int dg_set_batched_kernel(dg_ctx* c, int32_t variant) {
     return fail(c, DG_ERR_ARG, "dg_set_batched_kernel: variant must be -1 .. 6");
   if (variant < 0) {
     c->batched_pinned = false;
+    c->batched_tune_asked = true;
     batch_of(mixed_of(c)).tune_version = -1;
   } else {
     c->batched_kernel = variant;

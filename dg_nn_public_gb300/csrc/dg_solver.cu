@@ -275,14 +275,16 @@ struct dg_ctx {
   // batched BF16 smoothing kernel variant (bsmooth): 0 CUDA cores, 1 / 2
   // mma.sync per element (4 / 8 warps), 3 mma.sync persistent bulk-copy, 4
   // tcgen05 persistent bulk-copy, 5 tcgen05 on split x, 6 the same
-  // warp-specialized; chosen by timing at the first batched
-  // solve of each mixed build unless pinned (DG_BATCHED_KERNEL or the older
-  // DG_BATCHED_MMA / _TMA / _WARPS switches)
+  // warp-specialized.  The solve takes it where the scaled faces are not in
+  // use (bwarp_kernel runs there) or where it is pinned (DG_BATCHED_KERNEL or
+  // the older DG_BATCHED_MMA / _TMA / _WARPS switches); unpinned it is then
+  // timed at the first batched solve of each mixed build
   int batched_kernel = 1;
   // batched Gram-Schmidt with one thread per (row lane, RHS) (bmdot2 /
   // baxpy2); DG_BATCHED_GS2=0 keeps the float4 forms
   bool batched_gs2 = true;
   bool batched_pinned = false;
+  bool batched_tune_asked = false;   // dg_set_batched_kernel(-1): time the variants at the next batched solve
   int tma_variant = 0;   // elements per group / stages / CTAs per SM of that kernel
   bool autotune = true;  // pick tma_variant by timing at the first mixed solve after a build
   // mixed preconditioner (3D, BF16 bulk-copy path): smoothing steps after

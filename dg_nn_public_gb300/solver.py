@@ -360,8 +360,8 @@ class DGSolver:
         return x_out
 
     def set_batched_kernel(self, kernel):
-        """Batched smoothing kernel: None / "auto" (timed choice at the next
-        batched solve) or one of BATCHED_KERNELS."""
+        """Batched smoothing kernel on the unscaled blocks: None / "auto"
+        (timed choice at the next batched solve) or one of BATCHED_KERNELS."""
         v = -1 if kernel in (None, "auto") else self.BATCHED_KERNELS.index(kernel)
         self._chk(self._lib.dg_set_batched_kernel(self._ctx, v))
 

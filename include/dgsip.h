@@ -209,11 +209,14 @@ int dg_solve_mixed_batched(dg_ctx* ctx, double* x, const double* b, int32_t nrhs
  * x_out must not alias x. */
 int dg_apply_batched(dg_ctx* ctx, const float* x, float* y, void* stream);
 int dg_smooth_pc_batched(dg_ctx* ctx, const float* x, const float* b, float* x_out, void* stream);
-/* Kernel of the batched BF16 smoothing step (no counterpart in the
- * reference): -1 = chosen by timing every variant at the next batched solve
- * (the default, once per operator build), 0 = CUDA cores, 1 / 2 = mma.sync
- * tensor-core tiles, one element per CTA (4 / 8 warps), 3 = mma.sync in a
- * persistent bulk-copy pipeline, 4 = tcgen05.mma with tensor-memory
+/* Kernel of the batched BF16 smoothing step on the unscaled blocks (no
+ * counterpart in the reference): dg_smooth_pc_batched runs it, and the batched
+ * solve where it is pinned to 0, 5 or 6 or the scaled faces are off; else the
+ * solve's steps are those of dg_smooth_scaled_batched.  -1 = chosen by timing
+ * every variant at the next batched solve (without scaled faces the default,
+ * once per operator build), 0 = CUDA cores, 1 / 2 = mma.sync tensor-core tiles,
+ * one element per CTA (4 / 8 warps; 1 until something else is chosen), 3 =
+ * mma.sync in a persistent bulk-copy pipeline, 4 = tcgen05.mma with tensor-memory
  * accumulators in a persistent bulk-copy pipeline, 5 = the same on an
  * iterate kept in the tensor-core operand layout (BF16 high + low parts,
  * bulk-copied straight into the MMA operand; the batched preconditioner
