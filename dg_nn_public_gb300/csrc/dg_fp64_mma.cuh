@@ -704,7 +704,7 @@ __global__ void __launch_bounds__(32 * kR64Warps, 2) res64_mma_kernel(
         double c = 0.0;
 #pragma unroll
         for (int n = 0; n < N; ++n) c = fma(We[n * N], rs[n], c);
-        x_out[e * N + lane] = x_own + c;
+        x_out[e * N + lane] = dead ? __longlong_as_double(0x7ff8000000000000ll) : x_own + c;
       }
       done();
     }
