@@ -414,6 +414,7 @@ __global__ void lev_jacobi_kernel(const int* __restrict__ rowptr, const int* __r
   const int i = t / LPR, lane = t % LPR;
   // the level matrix is fixed data: the first four entries of this lane are
   // read before the programmatic-launch wait, overlapping the previous kernel
+  // in the FP32 chain (the FP64 chain is launched plainly)
   constexpr int PRE = 4;
   int k0 = 0, k1 = 0;
   int cpre[PRE];
@@ -1201,8 +1202,8 @@ __global__ void __launch_bounds__(512) tail_columns_kernel(TailParams<double> p,
 // doubles).  With fine > 0, r and e0 are formed there as the pair sums of the
 // finer level's residual and error (fine rows; lev_restrict_kernel), so the
 // restriction needs no launch; e0 is not read when ncol == n (no finer
-// level: the error starts at zero).  The first entries of the fixed row are
-// read before the programmatic-launch wait.
+// level: the error starts at zero).  The first entries of the row are read
+// ahead of the vectors.
 __global__ void __launch_bounds__(256) dense_tail64_kernel(const double* __restrict__ T, int ld,
                                                            const double* __restrict__ r,
                                                            const double* __restrict__ e0, int fine,

@@ -985,9 +985,6 @@ int ensure_tail64(dg_ctx* c, cudaStream_t st) {
   tail_columns_kernel<<<ncol, 512, words * sizeof(double), st>>>(tp, c->d_tail, c->tail_ld);
   bump();
   CKL(c);
-  // not a kernel: the next one starts only when the matrix is in memory, also
-  // if it reads it before its programmatic-launch wait
-  CK(c, cudaMemsetAsync(c->d_part, 0, sizeof(double), st));
   c->t64_version = c->build_version;
   return DG_OK;
 }
