@@ -95,18 +95,18 @@ __device__ __forceinline__ void mma_f16_16816(float (&c)[4], uint32_t a0, uint32
 // 2^e as a double, -1022 <= e <= 1023
 __device__ __forceinline__ double exp2_int(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
 
-// b - 2^e v for |v| < 2^49, 0 or at least 2^-32: one rounding.  2^e need not
-// be a number where 2^e v is one, so it goes in as two factors; beyond the
-// clamp the product is below half of the smallest subnormal, or infinite.
-__device__ __forceinline__ double sub_scaled(double b, int e, double v) {
+// b - 2^e (H + 2^-32 L), H and L 48-bit signed integers: one rounding of the sum
+// and one of the difference.  2^e need not be a number where the product is
+// one, so half of it goes into the exponents of H and L as they become
+// doubles (exactly, one FP64 addition each) and the rest is a factor; beyond
+// the clamp the product is below half of the smallest subnormal, or infinite.
+__device__ __forceinline__ double sub_scaled(double b, int e, long long H, long long L) {
   e = min(max(e, -1200), 1100);
   const int h = e >> 1;
-  return fma(-exp2_int(e - h), v * exp2_int(h), b);
-}
-
-// a 48-bit signed integer as a double, exactly (one FP64 addition)
-__device__ __forceinline__ double int48_to_double(long long v) {
-  return __longlong_as_double(0x4330000000000000ll + (v + (1ll << 51))) - (4503599627370496.0 + 2251799813685248.0);
+  const long long k = ((long long)(1075 + h) << 52) + (1ll << 51);   // 2^h (2^52 + 2^51)
+  const double k_d = __longlong_as_double(k);
+  const double Hd = __longlong_as_double(k + H) - k_d, Ld = __longlong_as_double(k + L) - k_d;
+  return fma(-exp2_int(e - h), fma(Ld, 0x1p-32, Hd), b);
 }
 
 // sum of four accumulators, 8 bits apart
@@ -127,18 +127,20 @@ __device__ __forceinline__ long long join4(float a, float b, float c, float d) {
 //   - fewer than kDigNear of its own 20 values reach 2^-kDigDropX (2^-kDigDropXB
 //     in the batched product, which also drops the digit pairs beyond 2^-58) of
 //     the largest at the element and its neighbours, or
-//   - in some row all but kDigNear - 1 of the own block's entries do not reach
+//   - in some row all but kDigLow - 1 of the own block's entries do not reach
 //     2^-kDigDropA of the row's largest (arithmetic means over a jump), or
 //   - a value is not finite.
-// Otherwise at least one own term of every row is within 2^-(kDigDropA +
-// kDigDropX) of the row's scale, and mostly 2^-(8 .. 12).  Emulated row by row on
-// the operator (kappa 1, log-normal to sigma 3, jumps of 10 .. 1e8; x the
-// solution, the source, a Jacobi iterate, N(0, 1), 12 decades): largest error of a
-// row over 2^-53 sum |a||x| 1 for the single and 4 for the batched product,
-// against 4 .. 12 of the FP64 loop's 100-term chain.  With kappa from 1 to
-// log-normal sigma 1 the first rule takes 0 .. 3% of the elements (those at
-// edges of the Dirichlet boundary), the others none.
-constexpr int kDigNear = 6, kDigDropX = 6, kDigDropXB = 4, kDigDropA = 10;
+// Emulated row by row on the operator (kappa 1, log-normal to sigma 3, jumps of
+// 10 .. 1e8; x the solution, the source, a Jacobi iterate, N(0, 1), 4 and 12
+// decades): largest error of a row over 2^-53 sum |a||x| 3 for the single and 6.5
+// for the batched product, against 4 .. 13 of the FP64 loop's 100-term chain.
+// The first rule takes 0 .. 1% of the elements (batched 0 .. 4%) with kappa from 1
+// to log-normal sigma 1, mostly at edges of the Dirichlet boundary, the second
+// none.  It is one vote, taken in the lanes that hold the rows: with three the
+// apply took 123.8 us instead of 121.9, with a second, wider one for x 5 us more
+// on a preconditioned vector.
+constexpr int kDigNear = 4, kDigDropX = 6, kDigDropXB = 4;
+constexpr int kDigLow = 6, kDigDropA = 10;
 constexpr int kEaFp64 = 0x7fff;   // row exponent of an element that is always taken in FP64
 
 // Digits and row exponents of all blocks; one CTA of 128 threads per element.
@@ -166,7 +168,7 @@ __global__ void __launch_bounds__(128) block_digits_kernel(const double* __restr
     er[threadIdx.x] = mx;
     int low = 0;   // own entries below 2^-kDigDropA of the row's largest
     for (int n = 0; n < 20; ++n) low += max((int)((v[n * 20 + threadIdx.x] >> 52) & 2047), 1) < mx - kDigDropA;
-    const bool bad = mx == 2047 || low >= kDigNear;
+    const bool bad = mx == 2047 || low >= kDigLow;
     const unsigned any = __ballot_sync(0xfffffu, bad);
     ea[e * 20 + threadIdx.x] = any ? kEaFp64 : mx - 1022;
     if (any && threadIdx.x == 0) atomicAdd(nfp64, 1);
@@ -367,9 +369,9 @@ __global__ void __launch_bounds__(128, 2) bres64_mma_kernel(
 #pragma unroll
       for (int d = 0; d < 2; ++d) {
         const int c = 2 * q + d;
-        const double H = int48_to_double(join4(acc[0][nt][c], acc[1][nt][c], acc[2][nt][c], acc[3][nt][c]));
-        const double L = int48_to_double(join4(acc[4][nt][c], acc[5][nt][c], acc[6][nt][c], acc[7][nt][c]));
-        out[d] = sub_scaled(b[o + d], ea[e * N + m + d] + ex - 36, fma(L, 0x1p-32, H));
+        out[d] = sub_scaled(b[o + d], ea[e * N + m + d] + ex - 36,
+                            join4(acc[0][nt][c], acc[1][nt][c], acc[2][nt][c], acc[3][nt][c]),
+                            join4(acc[4][nt][c], acc[5][nt][c], acc[6][nt][c], acc[7][nt][c]));
       }
       *reinterpret_cast<double2*>(r + o) = make_double2(out[0], out[1]);
     }
@@ -510,10 +512,12 @@ __global__ void __launch_bounds__(32 * kR64Warps, 2) res64_mma_kernel(
   unsigned long long v[4];
   double bv;
   int ee;
+  // values of x that a lane holds: its own row's or one of 20 .. 31, then 32 q + lane
+  const int k0 = mine ? m : (t == 3 ? N + g : N + 4 + g);
   auto gather = [&](int64_t e) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const int k = lane + 32 * q, bb = k / N;
+      const int k = q == 0 ? k0 : lane + 32 * q, bb = k / N;
       v[q] = 0;
       if (k < NB * N) {
         const int64_t src = bb == 0 ? e : (bb == 1 ? nb.x : (bb == 2 ? nb.y : (bb == 3 ? nb.z : nb.w)));
@@ -547,12 +551,12 @@ __global__ void __launch_bounds__(32 * kR64Warps, 2) res64_mma_kernel(
 #pragma unroll
     for (int q = 0; q < 4; ++q) mx = max(mx, (int)((v[q] >> 52) & 2047));
     const int em = max(__reduce_max_sync(0xffffffffu, mx), 1);
-    const int near = max((int)((v[0] >> 52) & 2047), 1);   // lanes < N: the own values
-    const bool fp64 = em == 2047 || __any_sync(0xffffffffu, ee == kEaFp64) ||
-                      __popc(__ballot_sync(0xffffffffu, lane < N && near >= em - kDigDropX)) < kDigNear;
+    const int need = em == 2047 ? 2048 : em - kDigDropX;
+    const bool near = mine && ee != kEaFp64 && max((int)((v[0] >> 52) & 2047), 1) >= need;
+    const bool fp64 = __popc(__ballot_sync(0xffffffffu, near)) < kDigNear;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const int k = lane + 32 * q;
+      const int k = q == 0 ? k0 : lane + 32 * q;
       if (k < NB * N) {
         if (fp64) {
           reinterpret_cast<unsigned long long*>(xw)[k] = v[q];
@@ -564,7 +568,7 @@ __global__ void __launch_bounds__(32 * kR64Warps, 2) res64_mma_kernel(
       }
     }
     __syncwarp();
-    const double x_own = __longlong_as_double((long long)v[0]), b_e = bv;   // x_own: lane < N
+    const double x_own = __longlong_as_double((long long)v[0]), b_e = bv;   // of row m, where mine
     const int ee_e = ee;
     if (e + stride < B) {   // in flight during the products
       gather(e + stride);
@@ -680,8 +684,7 @@ __global__ void __launch_bounds__(32 * kR64Warps, 2) res64_mma_kernel(
         Lt += __shfl_xor_sync(0xffffffffu, Lt, o);
       }
       const long long H = (t & 1) ? Ht : Hs, L = (long long)((t & 1) ? Lt : Ls);
-      if (mine)
-        res = sub_scaled(b_e, ee_e + em - 1022 - 36, fma(int48_to_double(L), 0x1p-32, int48_to_double(H)));
+      if (mine) res = sub_scaled(b_e, ee_e + em - 1022 - 36, H, L);
     }
     if (dead) res = __longlong_as_double(0x7ff8000000000000ll);
     if (mine) {
@@ -699,12 +702,12 @@ __global__ void __launch_bounds__(32 * kR64Warps, 2) res64_mma_kernel(
     }
     if (smooth) {
       wait();
-      if (lane < N) {
-        const double* We = reinterpret_cast<const double*>(stage + (cc & 1) * kR64Stage) + lane;
+      if (mine) {
+        const double* We = reinterpret_cast<const double*>(stage + (cc & 1) * kR64Stage) + m;
         double c = 0.0;
 #pragma unroll
         for (int n = 0; n < N; ++n) c = fma(We[n * N], rs[n], c);
-        x_out[e * N + lane] = dead ? __longlong_as_double(0x7ff8000000000000ll) : x_own + c;
+        x_out[e * N + m] = dead ? __longlong_as_double(0x7ff8000000000000ll) : x_own + c;
       }
       done();
     }
