@@ -365,8 +365,9 @@ cudaError_t dev_malloc(dg_ctx* c, void** p, size_t bytes) {
 
 // The digit copy of the blocks is the one buffer that every caller has another
 // way for; it is outside allocs and given back when another one does not fit.
+// cudaFree waits for the device, so no product is reading them; a
+// cudaDeviceSynchronize would break a capture in another thread's context.
 void release_digits(dg_ctx* c) {
-  cudaDeviceSynchronize();   // no product is reading them
   if (c->d_adig) {
     cudaFree(c->d_adig);
     c->dev_bytes -= digit_bytes(c);
