@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(160) bprolong_lane_kernel(float* __restrict__ 
 // is staged per warp (no CTA barrier) with the next one already in registers;
 // x rows are read by the lanes that use them.  A 16-byte word of the block
 // (four columns of a row, the same for all lanes) feeds 4 CP FMAs, so the
-// FMA pipe bounds it (123 MFMA per element and 64 columns: 150 us at 48,000
+// FMA pipe bounds it (125,000 FMA per element and 64 columns: 150 us at 48,000
 // tetrahedra).  Same sums in the same order as bres_kernel (one CTA per
 // element, x slabs in shared memory: 471 us there, 313 us here; 32 columns of 7,722 elements
 // 82 -> 41 us).

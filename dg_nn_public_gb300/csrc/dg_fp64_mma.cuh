@@ -132,7 +132,7 @@ __device__ __forceinline__ long long join4(float a, float b, float c, float d) {
 //   - a value is not finite.
 // Emulated row by row on the operator (kappa 1, log-normal to sigma 3, jumps of
 // 10 .. 1e8; x the solution, the source, a Jacobi iterate, N(0, 1), 4 and 12
-// decades): largest error of a row over 2^-53 sum |a||x| 3 for the single and 6.5
+// decades): largest error of a row over 2^-53 sum |a||x| 3.3 for the single and 6.5
 // for the batched product, against 4 .. 13 of the FP64 loop's 100-term chain.
 // The first rule takes 0 .. 1% of the elements (batched 0 .. 4%) with kappa from 1
 // to log-normal sigma 1, mostly at edges of the Dirichlet boundary, the second
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(256) x_exponents_kernel(const double* __restri
 // the columns that they would not hold (kDigDropXB) are formed in FP64 as
 // well, four at a time, and a row takes what is closer.  Bound by the mma.sync rate (36 digit pairs x 3 mma x 8 k-tiles per
 // warp: 1.1 ms at 48,000 tetrahedra x 64 against 10.9 ms for 64 products on
-// the FP64 pipe) and the instructions that feed it.
+// the FP64 pipe) and the instructions that feed it; 2.47 ms.
 __global__ void __launch_bounds__(128, 2) bres64_mma_kernel(
     const unsigned char* __restrict__ adig, const int* __restrict__ ea, const double* __restrict__ blk,
     const int* __restrict__ nbe, const double* __restrict__ x, const unsigned* __restrict__ xe,
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(128, 2) bres64_mma_kernel(
 // with the smoother).  Every warp streams its own elements' chunks by bulk
 // copies into two shared-memory stages and gathers the next element's x
 // while it works, so no round trip is waited for: 48,000 tetrahedra
-// apply 122 us, smoothing step 147 us (113 / 136 us at HBM rate; FP64 pipe
+// apply 122 us, smoothing step 150 us (113 / 136 us at HBM rate; FP64 pipe
 // 171 / 206 us); 3,072 tetrahedra 17.0 -> 12.8 us.
 // Waits are bounded: on time-out the warp's remaining rows become NaN.
 constexpr int kR64Warps = 8, kR64Stage = 5760;
